@@ -918,16 +918,31 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
         });
     }
     // Device pin order for the per-net pass (kernels.cu): nets above
-    // kWarpPins pins first, largest first (a warp each), then degree
-    // kWarpPins down to 1, floor(kWarpPins / degree) nets per warp; original
-    // order inside a degree.  Nets without pins take no task.
+    // kWarpPins pins first, largest first (a block or a warp each), then
+    // degree kWarpPins down to 1, floor(kWarpPins / degree) nets per warp, 32
+    // Nets without pins take no task.
     std::vector<int4> net_tasks;
+    int n_block_nets = 0;
     std::vector<int32_t> dev_owner(np), dev_of_pin(np);
     std::vector<float2> dev_off(np);
+    std::vector<int32_t> order;  // nets in device order
     {
         std::vector<std::vector<int>> by_deg(kWarpPins + 1);
         std::vector<int> big_list;
-        for (int n = 0; n < nnet; n++) {
+        // by lowest owner (a counting sort), so that neighbouring nets of a
+        // degree read neighbouring centres
+        std::vector<int32_t> low(nnet), at(no + nt + 1, 0), by_low(nnet);
+        parallel_ranges(nnet, nth, [&](int, int n0, int n1) {
+            for (int n = n0; n < n1; n++) {
+                int32_t m = no + nt - 1;
+                for (int p = net_start[n]; p < net_start[n + 1]; p++) m = std::min(m, owner[p]);
+                low[n] = m;
+            }
+        });
+        for (int n = 0; n < nnet; n++) at[low[n] + 1]++;
+        for (int o = 0; o < no + nt; o++) at[o + 1] += at[o];
+        for (int n = 0; n < nnet; n++) by_low[at[low[n]]++] = n;
+        for (int n : by_low) {
             int deg = net_start[n + 1] - net_start[n];
             (deg > kWarpPins ? big_list : by_deg[deg]).push_back(n);
         }
@@ -935,7 +950,6 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
             return net_start[a + 1] - net_start[a] > net_start[b + 1] - net_start[b];
         });
         // nets in device order with their first device pin, then the copy
-        std::vector<int> order;
         std::vector<int32_t> first;
         order.reserve(nnet);
         first.reserve(nnet);
@@ -951,9 +965,10 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
         for (int n : big_list) {
             int at = put_net(n);
             net_tasks.push_back(make_int4(net_start[n + 1] - net_start[n], at, 1, 0));
+            n_block_nets += net_start[n + 1] - net_start[n] > kBlockPins;
         }
         for (int d = kWarpPins; d >= 1; d--) {
-            const size_t per = kWarpPins / d;
+            const size_t per = d > 1 && d <= kThreadPins ? 32 : kWarpPins / d;
             for (size_t i = 0; i < by_deg[d].size(); i += per) {
                 int at = q, count = (int)std::min(per, by_deg[d].size() - i);
                 for (int j = 0; j < count; j++) put_net(by_deg[d][i + j]);
@@ -1054,10 +1069,6 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
     for (int v = 0; v < 3; v++)
         if ((s = dupload(e, e->view_idx[v], e->h_view[v]))) return s;
     {
-        std::vector<int32_t> order;
-        order.reserve(nnet);
-        for (int p = 0; p < np; p++)
-            if (p == 0 || e->h_pin_net[p] != e->h_pin_net[p - 1]) order.push_back(e->h_pin_net[p]);
         for (int n = 0; n < nnet; n++)  // nets without pins last, so the order holds every net
             if (e->h_net_deg[n] == 0) order.push_back(n);
         if ((s = dupload(e, e->net_first, e->h_net_first)) || (s = dupload(e, e->net_deg, e->h_net_deg)) ||
@@ -1110,6 +1121,7 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
     d.pin_obj_slot = e->pin_obj_slot;
     d.net_tasks = e->net_tasks;
     d.n_net_tasks = (int)net_tasks.size();
+    d.n_block_nets = n_block_nets;
     d.big_objs = e->big_objs;
     d.big_slot = e->big_slot;
     d.n_big_objs = (int)big.size();

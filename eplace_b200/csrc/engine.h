@@ -55,11 +55,16 @@ inline void launch_kp(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// Per-net pass: one warp per task.  Nets of up to kWarpPins pins share a warp
-// (floor(kWarpPins / degree) nets of one degree, a pin per lane); larger nets
-// take a warp each, their first kStagedPins pins staged in shared memory.
+// Per-net pass: a unit of work per task, by the nets' degree (kernels.cu): a
+// thread per net of 2 to kThreadPins pins, a lane per pin up to kWarpPins, a
+// warp per net up to kBlockPins, a block per net above.  Measured (1M cells,
+// FP32 / 200k cells, FP64, us): kThreadPins 1 118 / 38, 3 106 / 30 and 4 97 /
+// 30 at the registers the compiler takes, 4 79 / 27, 5 75 / 26 and 6 73 / 26
+// held to six (FP32) and four (FP64) blocks an SM; 5 is the fastest at 200k
+// (17.7 against 18.5 with 6).
+constexpr int kThreadPins = 5;
 constexpr int kWarpPins = 32;
-constexpr int kStagedPins = 128;
+constexpr int kBlockPins = 96;
 constexpr int kNetWarps = 8;  // warps per block of the per-net pass
 // Objects whose bin footprint may exceed this many bins take the
 // block-per-object scatter / gather path.
@@ -114,9 +119,10 @@ struct DeviceNetlist {
                                    // order (-1 for terminal pins): where the per-net pass
                                    // writes the pin's gradient, so each object's pin
                                    // gradients lie contiguous for the combine
-    const int4 *net_tasks;         // per warp of the per-net pass: degree, first pin, nets,
-                                   // ceil(2^16 / degree) (0 for nets above kWarpPins pins)
+    const int4 *net_tasks;         // tasks of the per-net pass: degree, first pin, nets,
+                                   // ceil(2^16 / degree) (0 where a net is the whole task)
     int n_net_tasks;
+    int n_block_nets;              // tasks of a whole block (nets above kBlockPins pins): the first ones
     const int32_t *big_objs;  // indices of kBig objects
     const int32_t *big_slot;  // object -> index in big_objs (or -1)
     int n_big_objs;

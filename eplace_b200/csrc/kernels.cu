@@ -252,26 +252,18 @@ __device__ __forceinline__ void add_terms(R (&s)[8], const PinExp<R> &e, vec2<R>
     s[7] = add_rn(s[7], e.eny);
 }
 
-// Per-net factors of the gradient: 1 / (sum of exponentials) and the
-// exponentially weighted mean coordinate of each of the four terms.  Every
-// denominator holds the bound pin's exp(0) = 1, so it is >= 1.
+// Per-net factors of the gradient: 1 / (sum of exponentials) of each of the
+// four terms, and the weighted sums whose quotients are the weighted mean
+// coordinates.  Every denominator holds the bound pin's exp(0) = 1, so it is
+// >= 1.
 template <typename R>
 struct NetCoef {
-    R rmx, mmx, rnx, mnx, rmy, mmy, rny, mny;
+    R rmx, nmx, rnx, nnx, rmy, nmy, rny, nny;
 };
 
 template <typename R>
 __device__ __forceinline__ NetCoef<R> net_coef(const NetSums<R> &s) {
-    NetCoef<R> c;
-    c.rmx = rcp_rn(s.dmx);
-    c.rnx = rcp_rn(s.dnx);
-    c.rmy = rcp_rn(s.dmy);
-    c.rny = rcp_rn(s.dny);
-    c.mmx = s.nmx * c.rmx;
-    c.mnx = s.nnx * c.rnx;
-    c.mmy = s.nmy * c.rmy;
-    c.mny = s.nny * c.rny;
-    return c;
+    return NetCoef<R>{rcp_rn(s.dmx), s.nmx, rcp_rn(s.dnx), s.nnx, rcp_rn(s.dmy), s.nmy, rcp_rn(s.dny), s.nny};
 }
 
 // Per-pin gradient of the WA model (objects.cpp:359-415).  The reference's
@@ -280,15 +272,19 @@ __device__ __forceinline__ NetCoef<R> net_coef(const NetSums<R> &s) {
 // subtracts the weighted mean from the coordinate before scaling, which
 // avoids the cancellation of the expanded quotient (the two agree to the
 // reference's own rounding).  A zero exponential (argument <= -300) gives a
-// zero term as in the reference.  LSE (:423-437): e / d per term.
+// zero term as in the reference.  LSE (:423-437): e / d per term.  Every
+// contraction is written out, so that each form of the pass rounds alike.
+template <bool LSE, typename R>
+__device__ __forceinline__ R axis_gradient(R em, R en, R x, R ig, R rm, R nm, R rn, R nn) {
+    const R am = mul_rn(em, rm), an = mul_rn(en, rn);
+    if (LSE) return fma_r(em, rm, -an);
+    const R fm = fma_r(ig, fma_r(-nm, rm, x), (R)1), fn = fma_r(-ig, fma_r(-nn, rn, x), (R)1);
+    return fma_r(am, fm, -mul_rn(an, fn));
+}
 template <bool LSE, typename R>
 __device__ __forceinline__ vec2<R> pin_gradient(const PinExp<R> &e, vec2<R> xy, R igx, R igy, const NetCoef<R> &c) {
-    if (LSE) return mk2<R>(e.emx * c.rmx - e.enx * c.rnx, e.emy * c.rmy - e.eny * c.rny);
-    const R gmx = e.emx * c.rmx * fma_r(igx, xy.x - c.mmx, (R)1);
-    const R gnx = e.enx * c.rnx * fma_r(-igx, xy.x - c.mnx, (R)1);
-    const R gmy = e.emy * c.rmy * fma_r(igy, xy.y - c.mmy, (R)1);
-    const R gny = e.eny * c.rny * fma_r(-igy, xy.y - c.mny, (R)1);
-    return mk2<R>(gmx - gnx, gmy - gny);
+    return mk2<R>(axis_gradient<LSE, R>(e.emx, e.enx, xy.x, igx, c.rmx, c.nmx, c.rnx, c.nnx),
+                  axis_gradient<LSE, R>(e.emy, e.eny, xy.y, igy, c.rmy, c.nmy, c.rny, c.nny));
 }
 
 template <typename R>
@@ -332,21 +328,30 @@ __device__ void finish_hpwl(DevScalars *S, double hp, int mode) {
 }
 
 // ---- the per-net pass ---------------------------------------------------------
-// On the device the nets are ordered by degree and each warp runs one task
-// (tasks[w] = degree D, first pin, nets, m):
-//   D <= kWarpPins: the task's nets (up to floor(32 / D), all of degree D)
-//       sit on lanes s*D .. s*D+D-1, one pin per lane (s = lane * m >> 16,
-//       m = ceil(2^16 / D), exact for lanes < 32), and the bound pins and
-//       exponential sums are segmented shuffle reductions over those lanes;
-//   D >  kWarpPins: one net; the warp strides over its pins, keeping the
-//       first kStagedPins of them in shared memory between the passes.
-// Nets above kWarpPins pins come first (largest first), then degree 32 down
-// to 1, so the long tasks start early.  The sums are in the working precision
-// as in Net::calcWirelengthWA_2D (float there), added in a fixed tree order
-// instead of pin order (a few ulps apart).  Pin gradients are written in
-// device pin order (coalesced); the combine kernel gathers them back in each
-// object's reference pin order.  WL = false computes only the HPWL with the
-// same layout and reduction tree, so both passes give bitwise the same HPWL.
+// On the device the nets are ordered by degree, largest first, and cut into
+// tasks (degree D, first pin, nets, m), each run by one unit:
+//   D >  kBlockPins: one net, a whole block (net_in_block);
+//   D >  kWarpPins:  one net, a warp striding over its pins (net_in_warp);
+//   D >  kThreadPins: floor(32 / D) nets on the lanes of a warp, one pin per
+//       lane (nets_in_warp; s = lane * m >> 16, m = ceil(2^16 / D), exact for
+//       lanes < 32), segmented shuffle reductions over the lanes;
+//   D <= kThreadPins: 32 nets, a thread each (nets_by_thread): no shuffles, and
+//       D position loads of a lane in flight at once.
+// The long tasks start first.  The pass is bound by the latency of its
+// dependent loads (pin -> owner -> centre), so the split follows the loads in
+// flight: a 500-pin net on one warp was a chain of 16 rounds in each of three
+// sweeps that the whole pass waited for, and one pin per lane left a warp with
+// one load in flight and 450 instructions of shuffle trees.
+// The sums are in the working precision as in Net::calcWirelengthWA_2D (float
+// there), added in one fixed order per degree, the same in every form: the
+// lane form's trees below, and for D > kWarpPins lane l adds pins l, l + 32,
+// ... and an xor tree adds the lanes.  Pin gradients go to their object-major
+// slots.  Within a degree the nets follow their lowest owner, so that a warp's
+// centres and slots share sectors (1M cells: 84 -> 79 us).  The split of the
+// work and six blocks an SM (40 registers; four in FP64) took the pass from
+// 26.1 to 17.7 us at 200k cells, 112 to 75 at 1M, 17.4 to 8.6 at 30k (FP32),
+// 36.9 to 26.2 at 200k (FP64), with bitwise the same gradients.  WL = false computes only the HPWL with the same layout and reduction
+// tree, so both passes give bitwise the same HPWL.
 struct NetOut {
     double hpwl, value;
 };
@@ -422,7 +427,96 @@ __device__ __forceinline__ NetOut nets_in_warp(const int4 t, int lane, const Pin
     return r;
 }
 
-// One net of D > 32 pins on one warp; `stage` holds kStagedPins pin positions.
+// Sum of v[0..D-1] in the order of seg_sums: halves for a power of two, else
+// pairs of neighbours, level by level.
+template <int D, typename R>
+__device__ __forceinline__ R tree_sum(const R (&v)[D]) {
+    R t[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) t[k] = v[k];
+    if constexpr ((D & (D - 1)) == 0) {
+#pragma unroll
+        for (int o = D >> 1; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < o; k++) t[k] = add_rn(t[k], t[k + o]);
+    } else {
+#pragma unroll
+        for (int o = 1; o < D; o <<= 1)
+#pragma unroll
+            for (int k = 0; k + o < D; k += 2 * o) t[k] = add_rn(t[k], t[k + o]);
+    }
+    return t[0];
+}
+
+// One axis of a net held by a thread: coordinates x, bounds x1 and x0; the
+// gradient of each pin along the axis.
+template <int D, bool EXACT, bool LSE, typename R>
+__device__ __forceinline__ void net_axis(const R (&x)[D], R x1, R x0, R ig, R (&grad)[D], R &nm, R &dm, R &nn, R &dn) {
+    R em[D], en[D], v[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+        em[k] = term_exp<EXACT, R>(mul_rn(sub_rn(x[k], x1), ig));
+        en[k] = term_exp<EXACT, R>(mul_rn(sub_rn(x0, x[k]), ig));
+        v[k] = mul_rn(x[k], em[k]);
+    }
+    nm = tree_sum<D, R>(v);
+    dm = tree_sum<D, R>(em);
+#pragma unroll
+    for (int k = 0; k < D; k++) v[k] = mul_rn(x[k], en[k]);
+    nn = tree_sum<D, R>(v);
+    dn = tree_sum<D, R>(en);
+    const R rm = rcp_rn(dm), rn = rcp_rn(dn);
+#pragma unroll
+    for (int k = 0; k < D; k++) grad[k] = axis_gradient<LSE, R>(em[k], en[k], x[k], ig, rm, nm, rn, nn);
+}
+
+// 32 nets of D <= kThreadPins pins, a thread each; one axis after the other,
+// so that only one axis's exponentials are held.
+template <int D, bool WL, bool EXACT, bool LSE, typename R>
+__device__ __forceinline__ NetOut nets_by_thread(const int4 t, int lane, const PinCtx<R> &pc,
+                                                 vec2<R> *__restrict__ out, R igx, R igy, int want_value) {
+    NetOut r{0.0, 0.0};
+    if (lane >= t.z) return r;
+    const int p = t.y + lane * D;
+    int owner[D], sl[D];
+    float2 off[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+        owner[k] = pc.owner[p + k];
+        off[k] = pc.off[p + k];
+        if (WL) sl[k] = pc.slot[p + k];
+    }
+    R x[D], y[D];
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+        const vec2<R> c = pc.pos[owner[k]];
+        x[k] = add_rn(c.x, (R)off[k].x);
+        y[k] = add_rn(c.y, (R)off[k].y);
+    }
+    R x1 = x[0], x0 = x[0], y1 = y[0], y0 = y[0];
+#pragma unroll
+    for (int k = 1; k < D; k++) {
+        x1 = max_r(x1, x[k]);
+        x0 = min_r(x0, x[k]);
+        y1 = max_r(y1, y[k]);
+        y0 = min_r(y0, y[k]);
+    }
+    r.hpwl = ((double)x1 - (double)x0) + ((double)y1 - (double)y0);
+    if (WL) {
+        NetSums<R> ns;
+        R gx[D], gy[D];
+        net_axis<D, EXACT, LSE, R>(x, x1, x0, igx, gx, ns.nmx, ns.dmx, ns.nnx, ns.dnx);
+        net_axis<D, EXACT, LSE, R>(y, y1, y0, igy, gy, ns.nmy, ns.dmy, ns.nny, ns.dny);
+#pragma unroll
+        for (int k = 0; k < D; k++)
+            if (sl[k] >= 0) out[sl[k]] = mk2<R>(gx[k], gy[k]);
+        if (want_value) r.value = net_value<R>(ns, x1, x0, y1, y0, igx, igy, LSE);
+    }
+    return r;
+}
+
+// One net of kWarpPins < D <= kBlockPins pins on one warp, its pin positions
+// staged in shared memory (each read back by the lane that wrote it).
 template <bool WL, bool EXACT, bool LSE, typename R>
 __device__ __forceinline__ NetOut net_in_warp(const int4 t, int lane, const PinCtx<R> &pc, vec2<R> *__restrict__ out,
                                               R igx, R igy, int want_value, vec2<R> *__restrict__ stage) {
@@ -431,7 +525,7 @@ __device__ __forceinline__ NetOut net_in_warp(const int4 t, int lane, const PinC
 #pragma unroll 4
     for (int k = lane; k < D; k += 32) {
         const vec2<R> xy = pin_xy<R>(pc, p0 + k);
-        if (k < kStagedPins) stage[k] = xy;  // read back by this lane only
+        if (WL) stage[k] = xy;
         x1 = max_r(x1, xy.x);
         x0 = min_r(x0, xy.x);
         y1 = max_r(y1, xy.y);
@@ -448,7 +542,7 @@ __device__ __forceinline__ NetOut net_in_warp(const int4 t, int lane, const PinC
     if (WL) {
         R s[8] = {(R)0, (R)0, (R)0, (R)0, (R)0, (R)0, (R)0, (R)0};
         for (int k = lane; k < D; k += 32) {
-            const vec2<R> xy = k < kStagedPins ? stage[k] : pin_xy<R>(pc, p0 + k);
+            const vec2<R> xy = stage[k];
             add_terms<R>(s, pin_exps<EXACT, R>(xy, x1, x0, y1, y0, igx, igy), xy);
         }
 #pragma unroll
@@ -458,7 +552,7 @@ __device__ __forceinline__ NetOut net_in_warp(const int4 t, int lane, const PinC
         const NetSums<R> ns = net_sums<R>(s);
         const NetCoef<R> c = net_coef<R>(ns);
         for (int k = lane; k < D; k += 32) {
-            const vec2<R> xy = k < kStagedPins ? stage[k] : pin_xy<R>(pc, p0 + k);
+            const vec2<R> xy = stage[k];
             const int sl = pc.slot[p0 + k];
             if (sl >= 0)
                 out[sl] = pin_gradient<LSE, R>(pin_exps<EXACT, R>(xy, x1, x0, y1, y0, igx, igy), xy, igx, igy, c);
@@ -468,23 +562,145 @@ __device__ __forceinline__ NetOut net_in_warp(const int4 t, int lane, const PinC
     return r;
 }
 
+// One net of more than kBlockPins pins on a whole block.  Its pins are taken
+// kChunkPins at a time: every thread computes its pins' exponentials into
+// shared memory, then warp i adds the i-th of the eight sums, lane l the pins
+// l, l + 32, ... in order across the chunks, and an xor tree adds the lanes --
+// net_in_warp's order.  kChunkPins keeps the staging at 6 KB in both
+// precisions: at 12 KB four blocks an SM were left under the loop's 64 KB split
+// and the whole pass slowed by a fifth.  A net of more pins gathers its
+// positions anew in each sweep.
+template <typename R>
+struct BlockStage {
+    static constexpr int kChunkPins = 1024 / (int)sizeof(R);
+    vec2<R> xy[kChunkPins];
+    R e[4][kChunkPins];
+};
+
 template <bool WL, bool EXACT, bool LSE, typename R>
-__global__ void __launch_bounds__(kNetWarps * 32)
-k_wl(const int4 *__restrict__ tasks, int n_tasks, PinCtx<R> pc, vec2<R> *__restrict__ out, int want_value,
-     double *__restrict__ partials, int mode, DevScalars *__restrict__ S) {
+__device__ __forceinline__ NetOut net_in_block(const int4 t, const PinCtx<R> &pc, vec2<R> *__restrict__ out, R igx,
+                                               R igy, int want_value, BlockStage<R> &sm, R *__restrict__ red) {
+    constexpr int C = BlockStage<R>::kChunkPins, NT = kNetWarps * 32;
+    static_assert(kNetWarps == 8, "a warp for each of the eight sums");
+    static_assert(C % 32 == 0, "a lane's pins keep their order across the chunks");
+    const int D = t.x, p0 = t.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    R x1 = (R)-3.4e38f, x0 = (R)3.4e38f, y1 = (R)-3.4e38f, y0 = (R)3.4e38f;
+#pragma unroll 2
+    for (int k = tid; k < D; k += NT) {
+        const vec2<R> xy = pin_xy<R>(pc, p0 + k);
+        if (WL && k < C) sm.xy[k] = xy;
+        x1 = max_r(x1, xy.x);
+        x0 = min_r(x0, xy.x);
+        y1 = max_r(y1, xy.y);
+        y0 = min_r(y0, xy.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        x1 = max_r(x1, __shfl_xor_sync(kFull, x1, o));
+        x0 = min_r(x0, __shfl_xor_sync(kFull, x0, o));
+        y1 = max_r(y1, __shfl_xor_sync(kFull, y1, o));
+        y0 = min_r(y0, __shfl_xor_sync(kFull, y0, o));
+    }
+    if (lane == 0) {
+        red[wid] = x1;
+        red[kNetWarps + wid] = x0;
+        red[2 * kNetWarps + wid] = y1;
+        red[3 * kNetWarps + wid] = y0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kNetWarps; w++) {
+        x1 = max_r(x1, red[w]);
+        x0 = min_r(x0, red[kNetWarps + w]);
+        y1 = max_r(y1, red[2 * kNetWarps + w]);
+        y0 = min_r(y0, red[3 * kNetWarps + w]);
+    }
+    NetOut r{tid == 0 ? ((double)x1 - (double)x0) + ((double)y1 - (double)y0) : 0.0, 0.0};
+    if (WL) {
+        R s = (R)0;
+        const R *es = sm.e[wid >> 1];
+        for (int c0 = 0; c0 < D; c0 += C) {  // block-uniform
+            const int n = min(C, D - c0);
+            if (c0 > 0) __syncthreads();  // the sums of the chunk before have read its staging
+            for (int k = tid; k < n; k += NT) {
+                if (c0 > 0) sm.xy[k] = pin_xy<R>(pc, p0 + c0 + k);
+                const PinExp<R> e = pin_exps<EXACT, R>(sm.xy[k], x1, x0, y1, y0, igx, igy);
+                sm.e[0][k] = e.emx;
+                sm.e[1][k] = e.enx;
+                sm.e[2][k] = e.emy;
+                sm.e[3][k] = e.eny;
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (int k = lane; k < n; k += 32) {
+                const R e = es[k];
+                s = add_rn(s, (wid & 1) ? e : mul_rn(wid < 4 ? sm.xy[k].x : sm.xy[k].y, e));
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = add_rn(s, __shfl_xor_sync(kFull, s, o));
+        if (lane == 0) red[4 * kNetWarps + wid] = s;
+        __syncthreads();
+        const R *tot = red + 4 * kNetWarps;
+        const NetSums<R> ns{tot[0], tot[1], tot[2], tot[3], tot[4], tot[5], tot[6], tot[7]};
+        const NetCoef<R> c = net_coef<R>(ns);
+        for (int k = tid; k < D; k += NT) {
+            const int sl = pc.slot[p0 + k];
+            if (sl < 0) continue;
+            const vec2<R> xy = D <= C ? sm.xy[k] : pin_xy<R>(pc, p0 + k);
+            const PinExp<R> e = D <= C ? PinExp<R>{sm.e[0][k], sm.e[1][k], sm.e[2][k], sm.e[3][k]}
+                                       : pin_exps<EXACT, R>(xy, x1, x0, y1, y0, igx, igy);
+            out[sl] = pin_gradient<LSE, R>(e, xy, igx, igy, c);
+        }
+        if (want_value && tid == 0) r.value = net_value<R>(ns, x1, x0, y1, y0, igx, igy, LSE);
+    }
+    return r;
+}
+
+// Shared memory of the per-net pass: a block runs either one net or the tasks
+// of its warps.
+template <typename R>
+union NetStage {
+    BlockStage<R> block;
+    vec2<R> warp[kNetWarps][kBlockPins];
+    __device__ NetStage() {}
+};
+
+// Blocks [0, n_block): one net of more than kBlockPins pins each; the warps of
+// the blocks after them: a task each.
+template <bool WL, bool EXACT, bool LSE, typename R>
+__global__ void __launch_bounds__(kNetWarps * 32, sizeof(R) == 8 ? 4 : 6)
+k_wl(const int4 *__restrict__ tasks, int n_block, int n_tasks, PinCtx<R> pc, vec2<R> *__restrict__ out,
+     int want_value, double *__restrict__ partials, int mode, DevScalars *__restrict__ S) {
     pdl_begin();
     __shared__ double sh[64];
-    __shared__ vec2<R> stage[WL ? kNetWarps : 1][WL ? kStagedPins : 1];
+    __shared__ R red[5 * kNetWarps];
+    __shared__ unsigned char stage_mem[WL ? sizeof(NetStage<R>) : 16] __attribute__((aligned(16)));
+    NetStage<R> &stage = *reinterpret_cast<NetStage<R> *>(stage_mem);
     if (WL && S->done) return;
     const R igx = (R)S->inv_gamma_x, igy = (R)S->inv_gamma_y;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int w = blockIdx.x * kNetWarps + wid;
     NetOut r{0.0, 0.0};
-    if (w < n_tasks) {  // warp-uniform
-        const int4 t = tasks[w];
-        r = t.x <= kWarpPins ? nets_in_warp<WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value)
-                             : net_in_warp<WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value,
-                                                              stage[WL ? wid : 0]);
+    if ((int)blockIdx.x < n_block) {
+        r = net_in_block<WL, EXACT, LSE, R>(tasks[blockIdx.x], pc, out, igx, igy, want_value, stage.block, red);
+    } else {
+        const int w = n_block + ((int)blockIdx.x - n_block) * kNetWarps + wid;
+        if (w < n_tasks) {  // warp-uniform
+            const int4 t = tasks[w];
+            static_assert(kThreadPins == 5, "the degrees below");
+            if (t.x == 2)
+                r = nets_by_thread<2, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+            else if (t.x == 3)
+                r = nets_by_thread<3, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+            else if (t.x == 4)
+                r = nets_by_thread<4, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+            else if (t.x == 5)
+                r = nets_by_thread<5, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+            else if (t.x <= kWarpPins)
+                r = nets_in_warp<WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+            else
+                r = net_in_warp<WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value, stage.warp[wid]);
+        }
     }
     // the smooth wirelength value rides along only when asked for
     bool last;
@@ -937,7 +1153,7 @@ int prep_blocks(const Grid &g) { return std::min(blocks_for(g.nx * g.ny, kThread
 
 int reduction_blocks(const DeviceNetlist &d, int which) {
     switch (which) {
-        case 0: return blocks_for(d.n_net_tasks, kNetWarps);
+        case 0: return d.n_block_nets + blocks_for(d.n_net_tasks - d.n_block_nets, kNetWarps);
         default: return blocks_for(d.n_obj, kThreads);
     }
 }
@@ -1002,7 +1218,7 @@ static void launch_nets(const KernelCtx &c, const DeviceNetlist &d, void *pin_gr
     PinCtx<R> pc{d.pin_owner, d.pin_off, V<R>(d.pos), d.pin_obj_slot};
     if (d.n_net_tasks == 0) return;
     launch_kp(k_wl<WL, EXACT, LSE, R>, reduction_blocks(d, 0), kNetWarps * 32, 0, st, launch_priority(false),
-              d.net_tasks, d.n_net_tasks, pc, V<R>(pin_grad), c.want_wl_value, partials, mode, S);
+              d.net_tasks, d.n_block_nets, d.n_net_tasks, pc, V<R>(pin_grad), c.want_wl_value, partials, mode, S);
 }
 
 template <typename R>
