@@ -107,20 +107,11 @@ struct Grid {
     float isx, isy;            // 1 / bin step (gather only)
 };
 
-// getOverlap/getOverlapArea (PlaceCommon/global.h:477-518), FP64.
+// getOverlap (PlaceCommon/global.h:477-518), FP64: 0, or the negative length.
 __device__ __forceinline__ double overlap_len(double a0, double a1, double b0, double b1) {
     double s = fmax(a0, b0);
     double e = fmin(a1, b1);
     return s >= e ? 0.0 : __dsub_rn(s, e);
-}
-
-__device__ __forceinline__ double overlap_area(double l1, double b1, double r1, double t1,
-                                               double l2, double b2, double r2, double t2) {
-    double h = overlap_len(l1, r1, l2, r2);
-    if (h == 0.0) return 0.0;
-    double v = overlap_len(b1, t1, b2, t2);
-    if (v == 0.0) return 0.0;
-    return __dmul_rn(h, v);
 }
 
 // float_less (global.h:350-353)
@@ -198,22 +189,6 @@ __device__ __forceinline__ void bin_range(const Grid &g, const RectT<R> &r, int 
     j0 = max(j0, 0);
     i1 = min(i1, g.nx - 1);
     j1 = min(j1, g.ny - 1);
-}
-
-// Bin corners as binInitialization stores them (EPlace/eplace.cpp:300-307).
-template <typename R>
-__device__ __forceinline__ void bin_box(const Grid &g, int i, int j, R &l, R &b, R &r, R &t) {
-    l = add_rn(mul_rn((R)i, (R)g.sx), (R)g.llx);
-    b = add_rn(mul_rn((R)j, (R)g.sy), (R)g.lly);
-    r = add_rn(l, (R)g.sx);
-    t = add_rn(b, (R)g.sy);
-}
-
-template <typename R>
-__device__ __forceinline__ double rect_bin_overlap(const Grid &g, const RectT<R> &r, int i, int j) {
-    R l, b, rr, t;
-    bin_box<R>(g, i, j, l, b, rr, t);
-    return overlap_area(l, b, rr, t, r.llx, r.lly, r.urx, r.ury);
 }
 
 // PlaceDB::setModuleCenter_2D clamp (PlaceDB/placedb.cpp:257-281), double

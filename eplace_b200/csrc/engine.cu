@@ -58,7 +58,7 @@ struct ep_engine {
     size_t v2 = sizeof(float2), r = sizeof(float);
     // device buffers
     void *pos = nullptr, *x = nullptr, *g = nullptr, *y_prev = nullptr, *g_prev = nullptr;
-    void *pin_grad = nullptr, *gd_big = nullptr, *field = nullptr;
+    void *pin_grad = nullptr, *field = nullptr;
     float2 *size = nullptr, *pin_off = nullptr;
     void *dump_gd = nullptr, *dump_gwl = nullptr;  // component gradients (vec2<R>), keep_maps only
     float2 *static_map = nullptr;
@@ -71,7 +71,7 @@ struct ep_engine {
     void *rho = nullptr, *phi = nullptr;
     float *sxy = nullptr;
     int32_t *pin_owner = nullptr, *obj_pin_start = nullptr, *obj_pin_dev = nullptr, *pin_obj_slot = nullptr;
-    int32_t *big_objs = nullptr, *big_slot = nullptr;
+    int32_t *big_objs = nullptr;
     int4 *net_tasks = nullptr;
     int32_t *view_idx[3] = {nullptr, nullptr, nullptr};
     unsigned long long *node_q = nullptr, *filler_q = nullptr;
@@ -330,7 +330,7 @@ ep_status device_status(ep_engine *e) {
 // Kernels one enqueue_eval launches (the DCT is four GEMMs).
 int kernels_per_eval(const ep_engine *e) {
     const DeviceNetlist &d = e->dn;
-    return 1 + 1 + dct_launches(e->dct) + (d.n_net_tasks > 0) + (d.n_big_objs > 0) + 1;
+    return 1 + 1 + dct_launches(e->dct) + (d.n_net_tasks > 0) + 1;
 }
 
 int kernels_per_hpwl(const ep_engine *e) { return e->dn.n_net_tasks > 0; }
@@ -347,7 +347,7 @@ void enqueue_eval_to(ep_engine *e, int stepping, void *gout, const void *g_ref, 
         cudaMemsetAsync(e->node_q, 0, sizeof(unsigned long long) * e->grid.nx * e->grid.ny, st);
         cudaMemsetAsync(e->filler_q, 0, sizeof(unsigned long long) * e->grid.nx * e->grid.ny, st);
     }
-    if (scatter) launch_scatter(e->kc, e->dn, e->node_q, e->filler_q, e->S, st);
+    if (scatter) launch_scatter(e->kc, e->dn, e->node_q, e->S, st);
     void *bf = e->dct.mode == EP_DCT_BF16X3 ? dct_tc_rho_planes(e->dct) : nullptr;
     launch_prep(e->kc, e->node_q, e->filler_q, e->static_map, bf ? nullptr : e->rho, bf,
                 keep ? e->node_f : nullptr, keep ? e->filler_f : nullptr, keep ? 0 : 1, e->S, st);
@@ -359,8 +359,7 @@ void enqueue_eval_to(ep_engine *e, int stepping, void *gout, const void *g_ref, 
     cudaEventRecord(e->ev_join, e->st_wl);
     dct_run(e->dct, e->rho, e->field, keep ? e->phi : nullptr, e->S, st);
     cudaStreamWaitEvent(st, e->ev_join, 0);
-    launch_gather_big(e->kc, e->dn, e->field, e->gd_big, e->S, st);
-    launch_combine(e->kc, e->dn, e->field, e->gd_big, e->pin_grad, gout, g_ref, y_ref,
+    launch_combine(e->kc, e->dn, e->field, e->pin_grad, gout, g_ref, y_ref,
                    keep ? e->dump_gd : nullptr, keep ? e->dump_gwl : nullptr, stepping, e->S, st);
 }
 
@@ -379,8 +378,8 @@ void enqueue_loop_step(ep_engine *e) {
         return;
     }
     enqueue_eval_to(e, 1, e->g, e->g_prev, e->y_prev, false);
-    launch_update_scatter(e->kc, e->dn, e->pos, e->x, e->g, e->y_prev, e->g_prev, e->node_q, e->filler_q,
-                          e->S, e->st);
+    launch_update_scatter(e->kc, e->dn, e->pos, e->x, e->g, e->y_prev, e->g_prev, e->node_q, e->S,
+                          e->st);
     e->launches += 1;
 }
 
@@ -852,7 +851,7 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
     // big objects: may cover more bins than the thread-per-object path loops over.
     // Local smoothing depends on the size only, so its flags and sx*sy scale
     // are fixed here (EPlace/eplace.cpp:1061-1072, float division and product).
-    std::vector<int32_t> big, big_slot(no, -1);
+    std::vector<int32_t> big, huge;
     std::vector<float> h_sxy(no);
     for (int o = 0; o < no; o++) {
         float w = e->h_size[o].x, h = e->h_size[o].y;
@@ -870,10 +869,11 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
         long sy = f_less_h(h, g.sy) ? 2 : (long)(h / g.sy) + 2;
         if (sx * sy > kSmallObjectBins) {
             e->h_flags[o] |= kBig;
-            big_slot[o] = (int32_t)big.size();
-            big.push_back(o);
+            (sx * sy > kWarpObjectBins ? huge : big).push_back(o);
         }
     }
+    const int n_huge = (int)huge.size();
+    big.insert(big.begin(), huge.begin(), huge.end());
 
     // ---- pins: net CSR and the object -> pin CSR (pins in id order) ----
     lap(1);
@@ -1046,7 +1046,6 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
         (s = dalloc_bytes(e, e->g, v2 * no)) || (s = dalloc_bytes(e, e->y_prev, v2 * no)) ||
         (s = dalloc_bytes(e, e->g_prev, v2 * no)) || (s = dupload(e, e->size, e->h_size)) ||
         (s = dupload(e, e->pin_off, dev_off)) || (s = dalloc_bytes(e, e->pin_grad, v2 * std::max(np, 1))) ||
-        (s = dalloc_bytes(e, e->gd_big, v2 * std::max<size_t>(big.size(), 1))) ||
         (s = dalloc_bytes(e, e->field, v2 * nb)) || (s = dupload(e, e->static_map, stat)) ||
         (s = dalloc(e, e->staging, no + nt)) || (s = dalloc(e, e->flags, no)) ||
         (s = dupload(e, e->npins, h_npins)) || (s = dupload(e, e->area, h_area)) ||
@@ -1055,9 +1054,9 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
         (s = dupload(e, e->obj_pin_dev, obj_pin_dev)) || (s = dupload(e, e->net_tasks, net_tasks)) ||
         (s = dupload(e, e->pin_obj_slot, pin_obj_slot)) ||
         (s = dupload(e, e->big_objs, big)) ||
-        (s = dupload(e, e->big_slot, big_slot)) || (s = dalloc(e, e->node_q, nb)) ||
-        (s = dalloc(e, e->filler_q, nb)) || (s = dalloc(e, e->S, 1)))
+        (s = dalloc(e, e->node_q, 2 * (size_t)nb)) || (s = dalloc(e, e->S, 1)))
         return s;
+    e->filler_q = e->node_q + nb;
     // centres: through the float2 staging buffer into the working precision
     // (exact for FP64)
     CK(cudaMemcpy(e->staging, pos.data(), sizeof(float2) * (no + nt), cudaMemcpyHostToDevice));
@@ -1123,8 +1122,8 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
     d.n_net_tasks = (int)net_tasks.size();
     d.n_block_nets = n_block_nets;
     d.big_objs = e->big_objs;
-    d.big_slot = e->big_slot;
     d.n_big_objs = (int)big.size();
+    d.n_huge_objs = n_huge;
     if ((s = dalloc(e, kc.part_prep, (size_t)prep_blocks(g))) ||
         (s = dalloc(e, kc.part_wl, (size_t)2 * std::max(1, reduction_blocks(d, 0)))) ||
         (s = dalloc(e, kc.part_comb, (size_t)5 * std::max(1, reduction_blocks(d, 1)))) ||
@@ -1709,7 +1708,7 @@ ep_status run_start(ep_engine *e, int32_t max_steps, RunState &r) {
     r.launched = 0;
     if (!r.bktrk && fused_loop(e)) {
         // the first step's maps (the graph's steps start at prep)
-        launch_scatter(e->kc, e->dn, e->node_q, e->filler_q, e->S, e->st);
+        launch_scatter(e->kc, e->dn, e->node_q, e->S, e->st);
         e->launches += 1;
     }
     return EP_OK;
@@ -2023,7 +2022,7 @@ ep_status ep_time_kernels(ep_engine *e, int32_t reps, ep_kernel_times *out) try 
     const double nx = e->grid.nx, ny = e->grid.ny;
     // algorithmic bytes: compulsory reads + writes of each group, per launch
     s = timed("scatter", 1 + (d.n_big_objs > 0), (9.0 + 8.0 * q) * nobj + 16.0 * nbin, 0.0,
-              [&] { launch_scatter(e->kc, d, e->node_q, e->filler_q, e->S, e->st); }, zero_maps);
+              [&] { launch_scatter(e->kc, d, e->node_q, e->S, e->st); }, zero_maps);
     if (s) return s;
     s = timed("prep", 1, 24.0 * nbin + 4.0 * q * nbin + (keep_maps ? 0.0 : 16.0 * nbin), 0.0,
               [&] {
@@ -2042,15 +2041,9 @@ ep_status ep_time_kernels(ep_engine *e, int32_t reps, ep_kernel_times *out) try 
     s = timed("wirelength", d.n_net_tasks > 0, (16.0 + 16.0 * q) * npin + 16.0 * d.n_net_tasks, 0.0,
               [&] { launch_wirelength(e->kc, d, e->pin_grad, e->S, e->st); }, nothing);
     if (s) return s;
-    if (d.n_big_objs > 0) {
-        s = timed("gather_big", 1, 0.0, 0.0,
-                  [&] { launch_gather_big(e->kc, d, e->field, e->gd_big, e->S, e->st); }, nothing);
-        if (s) return s;
-    }
     s = timed("combine", 1, (29.0 + 56.0 * q) * nobj + 8.0 * q * npin, 0.0,
               [&] {
-                  launch_combine(e->kc, d, e->field, e->gd_big, e->pin_grad, e->g, e->g_prev,
-                                 e->y_prev, nullptr, nullptr, 1, e->S, e->st);
+                  launch_combine(e->kc, d, e->field, e->pin_grad, e->g, e->g_prev, e->y_prev, nullptr, nullptr, 1, e->S, e->st);
               }, nothing);
     if (s) return s;
     s = timed("update", 1, (9.0 + 56.0 * q) * nobj, 0.0,

@@ -66,9 +66,11 @@ constexpr int kThreadPins = 5;
 constexpr int kWarpPins = 32;
 constexpr int kBlockPins = 96;
 constexpr int kNetWarps = 8;  // warps per block of the per-net pass
-// Objects whose bin footprint may exceed this many bins take the
-// block-per-object scatter / gather path.
+// Objects whose bin footprint may exceed this many bins are kBig: a unit of
+// several threads scatters and gathers each.
 constexpr int kSmallObjectBins = 16;
+// A kBig object of at most this many bins takes a warp, a larger one a block.
+constexpr int kWarpObjectBins = 512;
 
 // ---- DCT / Poisson plan (dct.cu, dct_tc.cu) ---------------------------------
 struct DctPlan {
@@ -123,9 +125,8 @@ struct DeviceNetlist {
                                    // ceil(2^16 / degree) (0 where a net is the whole task)
     int n_net_tasks;
     int n_block_nets;              // tasks of a whole block (nets above kBlockPins pins): the first ones
-    const int32_t *big_objs;  // indices of kBig objects
-    const int32_t *big_slot;  // object -> index in big_objs (or -1)
-    int n_big_objs;
+    const int32_t *big_objs;  // indices of kBig objects, those above kWarpObjectBins bins first
+    int n_big_objs, n_huge_objs;
 };
 
 struct KernelCtx {
@@ -152,25 +153,23 @@ int reduction_blocks(const DeviceNetlist &d, int which);
 
 // Vectors typed void * hold vec2<R> (float2 / double2, KernelCtx::fp64) and
 // rho holds R.
-void launch_scatter(const KernelCtx &c, const DeviceNetlist &d, unsigned long long *node_q,
-                    unsigned long long *filler_q, const DevScalars *S, cudaStream_t st);
+// maps: the node map, the filler map behind it.
+void launch_scatter(const KernelCtx &c, const DeviceNetlist &d, unsigned long long *maps, const DevScalars *S,
+                    cudaStream_t st);
 void launch_prep(const KernelCtx &c, unsigned long long *node_q, unsigned long long *filler_q,
                  const float2 *static_map, void *rho, void *rho_bf16, float *node_f,
                  float *filler_f, int zero_maps, DevScalars *S, cudaStream_t st);
 void launch_wirelength(const KernelCtx &c, const DeviceNetlist &d, void *pin_grad, DevScalars *S,
                        cudaStream_t st);
-void launch_gather_big(const KernelCtx &c, const DeviceNetlist &d, const void *field, void *gd_big,
-                       const DevScalars *S, cudaStream_t st);
-void launch_combine(const KernelCtx &c, const DeviceNetlist &d, const void *field, const void *gd_big,
-                    const void *pin_grad, void *g, const void *g_prev, const void *y_prev, void *dump_gd,
-                    void *dump_gwl, int stepping, DevScalars *S, cudaStream_t st);
+void launch_combine(const KernelCtx &c, const DeviceNetlist &d, const void *field, const void *pin_grad, void *g,
+                    const void *g_prev, const void *y_prev, void *dump_gd, void *dump_gwl, int stepping, DevScalars *S,
+                    cudaStream_t st);
 void launch_update(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g, void *y_prev,
                    void *g_prev, DevScalars *S, cudaStream_t st);
 // The update of the captured loop: also scatters the new positions into the
 // (clear) density maps for the next evaluation, unless the step ends the stage.
 void launch_update_scatter(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
-                           void *y_prev, void *g_prev, unsigned long long *node_q, unsigned long long *filler_q,
-                           DevScalars *S, cudaStream_t st);
+                           void *y_prev, void *g_prev, unsigned long long *maps, DevScalars *S, cudaStream_t st);
 // Backtracking step rule: one trial move from y_k (ysave) along g_k, and the
 // scalar commit of an accepted trial (combine in stepping mode 2 decides).
 void launch_bktrk_move(const KernelCtx &c, const DeviceNetlist &d, const void *ysave, const void *g, const void *x,

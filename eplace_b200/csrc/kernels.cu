@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "scatter.cuh"
 
 namespace ep {
 
@@ -39,6 +40,12 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kPinChunk = 128;  // pin gradients a warp of the combine kernel stages per round
 
+constexpr int kSms = 148;
+// Grids of the kernels that loop over their work and end in a grid sum: one
+// block for each that an SM holds, so that a block's reduction and the wait for
+// its slowest warp are paid once.  Fixed numbers, so that the sums do not
+// depend on anything else.
+constexpr int kCombineBlocks = kSms * 3;
 inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
 
 using ull = unsigned long long;
@@ -49,71 +56,78 @@ __device__ __forceinline__ float warp_sum_r(float v) { return warp_sum_f(v); }
 __device__ __forceinline__ double warp_sum_r(double v) { return warp_sum(v); }
 
 // ---------------------------------------------------------------- scatter --
+// Rectangle and contribution scale of an object: sx*sy, times the target
+// density for macros (EPlace/eplace.cpp:1114-1128, evaluated left to right).
+// In FP32 sx*sy is the static table's value, the same float operations.
 template <typename R>
-__device__ __forceinline__ void scatter_one(const Grid &g, const RectT<R> &r, R scale, int i, int j, double qscale,
-                                            ull *__restrict__ map) {
-    R ovl = (R)rect_bin_overlap<R>(g, r, i, j);
-    if (ovl == (R)0) return;
-    R c = mul_rn(scale, ovl);
-    long long q = __double2ll_rn(__dmul_rn((double)c, qscale));
-    atomicAdd(&map[(size_t)i * g.ny + j], (ull)q);
+__device__ __forceinline__ RectT<R> scatter_rect(const Grid &g, vec2<R> p, float2 s, float sxy_table, uint8_t f,
+                                                 R &scale) {
+    const RectT<R> r = object_rect(g, p.x, p.y, (R)s.x, (R)s.y);
+    if constexpr (sizeof(R) == 4)
+        scale = sxy_table;
+    else
+        scale = mul_rn(r.sx, r.sy);
+    if (f & kMacro) scale = mul_rn(scale, (R)g.td);
+    return r;
 }
 
-// Contribution scale: sx*sy, times the target density for macros
-// (EPlace/eplace.cpp:1114-1128, evaluated left to right).
+// The objects of a warp, one a lane (valid false: none); every lane calls it.
+// The filler map lies behind the node map.
 template <typename R>
-__device__ __forceinline__ R contrib_scale(const RectT<R> &r, uint8_t f, float td) {
-    R s = mul_rn(r.sx, r.sy);
-    return (f & kMacro) ? mul_rn(s, (R)td) : s;
-}
-
-// One object of the thread-per-object path (kBig objects excluded).
-template <typename R>
-__device__ __forceinline__ void scatter_small_object(const Grid &g, vec2<R> p, float2 s, uint8_t f, double qscale,
-                                                     ull *__restrict__ node_q, ull *__restrict__ filler_q) {
-    RectT<R> r = object_rect(g, p.x, p.y, (R)s.x, (R)s.y);
+__device__ __forceinline__ void scatter_objects(const Grid &g, bool valid, vec2<R> p, float2 s, float sxy_table,
+                                                uint8_t f, double qscale, ull *__restrict__ maps) {
+    R scale;
+    const RectT<R> r = scatter_rect<R>(g, p, s, sxy_table, f, scale);
     int i0, i1, j0, j1;
     bin_range<R>(g, r, i0, i1, j0, j1);
-    R scale = contrib_scale<R>(r, f, g.td);
-    ull *map = (f & kFiller) ? filler_q : node_q;
-    for (int i = i0; i <= i1; i++)
-        for (int j = j0; j <= j1; j++) scatter_one<R>(g, r, scale, i, j, qscale, map);
+    if (!valid) i1 = i0 - 1;
+    const unsigned bin = (unsigned)(i0 * g.ny + j0) + ((f & kFiller) ? (unsigned)(g.nx * g.ny) : 0u);
+    scatter_by_lane<R>(g, r, scale, i0, i1, j0, j1, qscale, bin, maps);
 }
 
-// One kBig object by a whole block, its bins strided over the threads.
+// One kBig object by `count` threads of which this is the rank-th.
 template <typename R>
-__device__ __forceinline__ void scatter_big_object(const Grid &g, vec2<R> p, float2 s, uint8_t f, double qscale,
-                                                   ull *__restrict__ node_q, ull *__restrict__ filler_q) {
-    RectT<R> r = object_rect(g, p.x, p.y, (R)s.x, (R)s.y);
+__device__ __forceinline__ void scatter_big(const Grid &g, vec2<R> p, float2 s, float sxy_table, uint8_t f,
+                                            double qscale, int rank, int count, ull *__restrict__ maps) {
+    R scale;
+    const RectT<R> r = scatter_rect<R>(g, p, s, sxy_table, f, scale);
     int i0, i1, j0, j1;
     bin_range<R>(g, r, i0, i1, j0, j1);
-    if (i1 < i0 || j1 < j0) return;
-    R scale = contrib_scale<R>(r, f, g.td);
-    ull *map = (f & kFiller) ? filler_q : node_q;
-    const int wy = j1 - j0 + 1, nb = (i1 - i0 + 1) * wy;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x)
-        scatter_one<R>(g, r, scale, i0 + t / wy, j0 + t % wy, qscale, map);
+    scatter_by_group<R>(g, r, scale, i0, i1, j0, j1, qscale, rank, count,
+                        maps + ((f & kFiller) ? (size_t)g.nx * g.ny : 0));
 }
 
-// Blocks [0, small_blocks): thread per object; the blocks after them: one
-// kBig object each.
+// Work of the object kernels: blocks [0, big_blocks) take the kBig objects (a
+// block each for the first n_huge, then a warp each; they start first), the
+// blocks after them a thread per object.  o = n_obj: nothing.
+struct ObjectUnit {
+    int o;
+    int rank, count;  // this thread among the threads of the object
+};
+__device__ __forceinline__ ObjectUnit object_unit(const DeviceNetlist &d, int big_blocks) {
+    const int b = blockIdx.x, t = threadIdx.x;
+    if (b >= big_blocks) return ObjectUnit{min((int)((b - big_blocks) * blockDim.x + t), d.n_obj), 0, 1};
+    if (b < d.n_huge_objs) return ObjectUnit{d.big_objs[b], t, kThreads};
+    const int slot = d.n_huge_objs + (b - d.n_huge_objs) * (kThreads / 32) + (t >> 5);
+    return ObjectUnit{slot < d.n_big_objs ? d.big_objs[slot] : d.n_obj, t & 31, 32};
+}
+
 template <typename R>
 __global__ void __launch_bounds__(kThreads)
-k_scatter(Grid g, const vec2<R> *__restrict__ pos, const float2 *__restrict__ size,
-          const uint8_t *__restrict__ flags, int n, int small_blocks, const int32_t *__restrict__ big,
-          double qscale, ull *__restrict__ node_q, ull *__restrict__ filler_q, const DevScalars *__restrict__ S) {
+k_scatter(Grid g, DeviceNetlist d, int big_blocks, double qscale, ull *__restrict__ maps,
+          const DevScalars *__restrict__ S) {
+    const ObjectUnit u = object_unit(d, big_blocks);
+    bool valid = u.o < d.n_obj;
+    const uint8_t f = valid ? d.flags[u.o] : 0;
+    const float2 s = valid ? d.size[u.o] : make_float2(1.f, 1.f);
+    const float sxy = valid ? d.sxy[u.o] : 0.f;
     pdl_begin();
     if (S->done) return;
-    if ((int)blockIdx.x >= small_blocks) {
-        const int o = big[blockIdx.x - small_blocks];
-        scatter_big_object<R>(g, pos[o], size[o], flags[o], qscale, node_q, filler_q);
-        return;
-    }
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= n) return;
-    const uint8_t f = flags[o];
-    if (f & kBig) return;
-    scatter_small_object<R>(g, pos[o], size[o], f, qscale, node_q, filler_q);
+    const vec2<R> p = valid ? ((const vec2<R> *)d.pos)[u.o] : mk2<R>((R)g.llx, (R)g.lly);
+    if (u.count == 1)
+        scatter_objects<R>(g, valid && !(f & kBig), p, s, sxy, f, qscale, maps);
+    else if (valid)
+        scatter_big<R>(g, p, s, sxy, f, qscale, u.rank, u.count, maps);
 }
 
 // ------------------------------------------------------------------- prep --
@@ -687,19 +701,22 @@ k_wl(const int4 *__restrict__ tasks, int n_block, int n_tasks, PinCtx<R> pc, vec
         const int w = n_block + ((int)blockIdx.x - n_block) * kNetWarps + wid;
         if (w < n_tasks) {  // warp-uniform
             const int4 t = tasks[w];
+            NetOut q{0.0, 0.0};
             static_assert(kThreadPins == 5, "the degrees below");
             if (t.x == 2)
-                r = nets_by_thread<2, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+                q = nets_by_thread<2, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
             else if (t.x == 3)
-                r = nets_by_thread<3, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+                q = nets_by_thread<3, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
             else if (t.x == 4)
-                r = nets_by_thread<4, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+                q = nets_by_thread<4, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
             else if (t.x == 5)
-                r = nets_by_thread<5, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+                q = nets_by_thread<5, WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
             else if (t.x <= kWarpPins)
-                r = nets_in_warp<WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
-            else
-                r = net_in_warp<WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value, stage.warp[wid]);
+                q = nets_in_warp<WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value);
+            else {
+                q = net_in_warp<WL, EXACT, LSE, R>(t, lane, pc, out, igx, igy, want_value, stage.warp[wid]);
+            }
+            r = q;
         }
     }
     // the smooth wirelength value rides along only when asked for
@@ -766,56 +783,113 @@ __device__ __forceinline__ R smoothing_scale(const Grid &g, float table, float2 
     }
 }
 
+// Overlap length of [lo, hi] with bin k of an axis, 0 where they do not meet.
 template <typename R>
-__device__ __forceinline__ vec2<R> gather_bin(const Grid &g, const FRect<R> &r, R sxy, int i, int j,
-                                              const vec2<R> *__restrict__ field) {
-    const R bl = fma_r((R)i, (R)g.sx, (R)g.llx), bb = fma_r((R)j, (R)g.sy, (R)g.lly);
-    const R ox = min_r(r.r, bl + (R)g.sx) - max_r(r.l, bl);
-    const R oy = min_r(r.t, bb + (R)g.sy) - max_r(r.b, bb);
-    if (ox <= (R)0 || oy <= (R)0) return mk2<R>((R)0, (R)0);
-    const R ov = sxy * ox * oy;
-    const vec2<R> e = field[(size_t)i * g.ny + j];
-    return mk2<R>(ov * e.x, ov * e.y);
+__device__ __forceinline__ R gather_len(R base, R step, int k, R lo, R hi) {
+    const R b = fma_r((R)k, step, base);
+    const R len = min_r(hi, b + step) - max_r(lo, b);
+    return len <= (R)0 ? (R)0 : len;
 }
 
+// acc += overlap * field; a bin that the rectangle does not meet adds nothing,
+// whatever its field holds.
 template <typename R>
-__global__ void __launch_bounds__(128)
-k_gather_big(Grid g, const vec2<R> *__restrict__ pos, const float2 *__restrict__ size,
-             const uint8_t *__restrict__ flags, const float *__restrict__ sxy_of, const int32_t *__restrict__ big,
-             const vec2<R> *__restrict__ field, vec2<R> *__restrict__ out, const DevScalars *__restrict__ S) {
-    pdl_begin();
-    __shared__ R shx[4], shy[4];
-    if (S->done) return;
-    const int o = big[blockIdx.x];
-    const uint8_t f = flags[o];
-    const FRect<R> r = gather_rect<R>(g, pos[o], size[o], f);
-    const R sxy = smoothing_scale<R>(g, sxy_of[o], size[o], f);
+__device__ __forceinline__ void gather_add(R &gx, R &gy, R ov, vec2<R> e) {
+    if (ov == (R)0) return;
+    gx = add_rn(gx, mul_rn(ov, e.x));
+    gy = add_rn(gy, mul_rn(ov, e.y));
+}
+
+// Field sum of an object of at most kSmallObjectBins bins by one thread, bins
+// in order (x, then y).  Rows are two at most but for objects higher than a
+// bin: their overlap lengths are formed once, and the loads of two columns are
+// in flight at once.
+template <typename R>
+__device__ __forceinline__ vec2<R> gather_small(const Grid &g, const FRect<R> &r, R sxy,
+                                                const vec2<R> *__restrict__ field) {
+    int i0, i1, j0, j1;
+    gather_range<R>(g, r, i0, i1, j0, j1);
+    R gx = (R)0, gy = (R)0;
+    if (j1 < j0) return mk2<R>(gx, gy);
+    if (j1 - j0 <= 1) {
+        const bool two = j1 > j0;
+        const R v0 = gather_len<R>((R)g.lly, (R)g.sy, j0, r.b, r.t);
+        const R v1 = two ? gather_len<R>((R)g.lly, (R)g.sy, j1, r.b, r.t) : (R)0;
+        const vec2<R> *row = field + (size_t)i0 * g.ny + j0;
+        const vec2<R> zero = mk2<R>((R)0, (R)0);
+        for (int i = i0; i <= i1; i += 2, row += 2 * g.ny) {
+            const bool more = i < i1;
+            const vec2<R> a0 = row[0], a1 = two ? row[1] : zero;
+            const vec2<R> b0 = more ? row[g.ny] : zero, b1 = more && two ? row[g.ny + 1] : zero;
+            const R ha = mul_rn(sxy, gather_len<R>((R)g.llx, (R)g.sx, i, r.l, r.r));
+            const R hb = more ? mul_rn(sxy, gather_len<R>((R)g.llx, (R)g.sx, i + 1, r.l, r.r)) : (R)0;
+            gather_add<R>(gx, gy, mul_rn(ha, v0), a0);
+            gather_add<R>(gx, gy, mul_rn(ha, v1), a1);
+            gather_add<R>(gx, gy, mul_rn(hb, v0), b0);
+            gather_add<R>(gx, gy, mul_rn(hb, v1), b1);
+        }
+        return mk2<R>(gx, gy);
+    }
+    for (int i = i0; i <= i1; i++) {
+        const R h = mul_rn(sxy, gather_len<R>((R)g.llx, (R)g.sx, i, r.l, r.r));
+        for (int j = j0; j <= j1; j++)
+            gather_add<R>(gx, gy, mul_rn(h, gather_len<R>((R)g.lly, (R)g.sy, j, r.b, r.t)),
+                          field[(size_t)i * g.ny + j]);
+    }
+    return mk2<R>(gx, gy);
+}
+
+// Field sum of a kBig object: kBigLanes partial sums, sum v over the bins v, v +
+// kBigLanes, ... in order, a tree over each 32 of them, then these in order.
+// By a warp (a lane holds four of the sums) up to kWarpObjectBins bins, by the
+// first kBigLanes threads of a block above.
+constexpr int kBigLanes = 128;
+template <typename R>
+__device__ __forceinline__ void gather_strided(const Grid &g, const FRect<R> &r, R sxy, int i0, int j0, int wy, int nb,
+                                               int v, const vec2<R> *__restrict__ field, R &gx, R &gy) {
+#pragma unroll 4
+    for (int t = v; t < nb; t += kBigLanes) {
+        const int i = i0 + t / wy, j = j0 + t % wy;
+        const R h = mul_rn(sxy, gather_len<R>((R)g.llx, (R)g.sx, i, r.l, r.r));
+        gather_add<R>(gx, gy, mul_rn(h, gather_len<R>((R)g.lly, (R)g.sy, j, r.b, r.t)), field[(size_t)i * g.ny + j]);
+    }
+}
+
+// One kBig object by a warp (block_wide false) or by a whole block; the sum in
+// lane 0 of the warp, or in thread 0.
+template <typename R>
+__device__ __forceinline__ vec2<R> gather_big(const Grid &g, vec2<R> p, float2 size, uint8_t f, float sxy_table,
+                                              const vec2<R> *__restrict__ field, bool block_wide, vec2<R> *sm) {
+    const FRect<R> r = gather_rect<R>(g, p, size, f);
+    const R sxy = smoothing_scale<R>(g, sxy_table, size, f);
     int i0, i1, j0, j1;
     gather_range<R>(g, r, i0, i1, j0, j1);
     const int wy = j1 - j0 + 1;
     const int nb = (i1 >= i0 && j1 >= j0) ? (i1 - i0 + 1) * wy : 0;
-    R gx = (R)0, gy = (R)0;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-        vec2<R> v = gather_bin<R>(g, r, sxy, i0 + t / wy, j0 + t % wy, field);
-        gx += v.x;
-        gy += v.y;
-    }
-    gx = warp_sum_r(gx);
-    gy = warp_sum_r(gy);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        shx[wid] = gx;
-        shy[wid] = gy;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        R ax = (R)0, ay = (R)0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) {
-            ax += shx[k];
-            ay += shy[k];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    R ax = (R)0, ay = (R)0;
+    if (block_wide) {
+        R gx = (R)0, gy = (R)0;
+        if (threadIdx.x < kBigLanes) gather_strided<R>(g, r, sxy, i0, j0, wy, nb, threadIdx.x, field, gx, gy);
+        gx = warp_sum_r(gx);
+        gy = warp_sum_r(gy);
+        if (lane == 0) sm[wid] = mk2<R>(gx, gy);
+        __syncthreads();
+        for (int k = 0; k < kBigLanes / 32; k++) {
+            ax += sm[k].x;
+            ay += sm[k].y;
         }
-        out[blockIdx.x] = mk2<R>(ax, ay);
+        __syncthreads();  // sm is used again
+    } else {
+#pragma unroll
+        for (int k = 0; k < kBigLanes / 32; k++) {
+            R gx = (R)0, gy = (R)0;
+            gather_strided<R>(g, r, sxy, i0, j0, wy, nb, 32 * k + lane, field, gx, gy);
+            ax += warp_sum_r(gx);
+            ay += warp_sum_r(gy);
+        }
     }
+    return mk2<R>(ax, ay);
 }
 
 // --------------------------------------------------------------- combine --
@@ -834,106 +908,152 @@ __device__ int stop_after_step(const DevScalars *S, double tau, int it) {
     return stop;
 }
 
-template <typename R>
-__global__ void __launch_bounds__(kThreads)
-k_combine(Grid g, DeviceNetlist d, const vec2<R> *__restrict__ field, const vec2<R> *__restrict__ gd_big,
-          const vec2<R> *__restrict__ pin_grad, vec2<R> *__restrict__ gout, const vec2<R> *__restrict__ g_prev,
-          const vec2<R> *__restrict__ y_prev, vec2<R> *__restrict__ dump_gd, vec2<R> *__restrict__ dump_gwl,
-          int stepping, double *__restrict__ partials, DevScalars *__restrict__ S) {
-    pdl_begin();
-    __shared__ double sh[32 * 5];
-    if (S->done) return;
-    const vec2<R> *__restrict__ pos = (const vec2<R> *)d.pos;
-    int o = blockIdx.x * blockDim.x + threadIdx.x;
-    R lam = S->lambda0_mode ? (R)0 : (R)S->lambda;
-    int iter = S->iter;
-    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // dg2, dy2, s.y, |gwl|, |gd|
+// What the combine reads of an object that no kernel writes.
+struct ObjStatic {
+    int o, ps, pe;
+    float2 size;
+    float sxy, npins, area;
+    uint8_t f;
+};
+__device__ __forceinline__ ObjStatic load_static(const DeviceNetlist &d, int o) {
+    ObjStatic s{o, 0, 0, make_float2(0.f, 0.f), 0.f, 0.f, 0.f, 0};
+    if (o < d.n_obj) {
+        s.f = d.flags[o];
+        s.size = d.size[o];
+        s.sxy = d.sxy[o];
+        s.npins = d.npins[o];
+        s.area = d.area[o];
+        s.ps = d.obj_pin_start[o];
+        s.pe = d.obj_pin_start[o + 1];
+    }
+    return s;
+}
 
-    // Wirelength gradient of the object: its pins' gradients added in pin
-    // order (EPlace/eplace.cpp:539-547).  The per-net pass wrote them in
-    // object-major order, so the objects of a warp own one contiguous run of
-    // gradient slots: the warp stages that run in shared memory with
-    // coalesced loads all in flight at once (kPinChunk per round), then
-    // every lane adds its own pins from there in order.  Fillers own no pins.
+// The objects' field and wirelength gradients, the direction, and the sums of
+// the step: a thread per object, the kBig objects in blocks of their own before
+// them (object_unit).  Bound by the latency of an object's loads (netlist arrays
+// -> pin gradients and field bins -> the previous step's vectors) at about half
+// the warps an SM can hold.  So: the blocks loop, and load the next object's
+// static arrays during this one's gather (the first one's before the wait for
+// the previous grid); pin gradients and previous vectors are in flight during
+// the gather; and the registers are left room, as spilling cost more than the
+// warps it bought (1M cells, blocks an SM: 2 69 us, 3 59, 4 64, 5 73; one object
+// a thread at 4 blocks 96).  With the kBig objects' gather, a launch of its own
+// before, us: 200k cells 18.3 + 3.1 -> 16.8, FP64 29.9 + 3.4 -> 25.5, 1M
+// 88.7 + 9.1 -> 59.5.
+template <typename R>
+__global__ void __launch_bounds__(kThreads, 3)
+k_combine(Grid g, DeviceNetlist d, const vec2<R> *__restrict__ field, const vec2<R> *__restrict__ pin_grad,
+          vec2<R> *__restrict__ gout, const vec2<R> *__restrict__ g_prev, const vec2<R> *__restrict__ y_prev,
+          vec2<R> *__restrict__ dump_gd, vec2<R> *__restrict__ dump_gwl, int big_blocks, int stepping,
+          double *__restrict__ partials, DevScalars *__restrict__ S) {
+    __shared__ double sh[32 * 5];
     __shared__ vec2<R> pin_sm[kThreads / 32][kPinChunk];
-    R wx = (R)0, wy = (R)0;
-    {
-        const int lane = threadIdx.x & 31;
-        vec2<R> *sm = pin_sm[threadIdx.x >> 5];
-        const bool valid = o < d.n_obj;
-        const int ps = valid ? d.obj_pin_start[o] : 0, pe = valid ? d.obj_pin_start[o + 1] : 0;
-        const int wbeg = __shfl_sync(0xffffffffu, ps, 0);
-        const int wend = __reduce_max_sync(0xffffffffu, (unsigned)pe);
+    const vec2<R> *__restrict__ pos = (const vec2<R> *)d.pos;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const ObjectUnit unit = object_unit(d, big_blocks);
+    const bool big = unit.count > 1, huge = unit.count == kThreads;
+    const int stride = big ? d.n_obj : ((int)gridDim.x - big_blocks) * kThreads;
+    ObjStatic next = load_static(d, unit.o);
+    pdl_begin();
+    if (S->done) return;
+    const R lam = S->lambda0_mode ? (R)0 : (R)S->lambda;
+    const int iter = S->iter;
+    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // dg2, dy2, s.y, |gwl|, |gd|
+    do {
+        const ObjStatic c = next;
+        const int o = c.o;
+        const uint8_t f = c.f;
+        const bool valid = o < d.n_obj && (big ? unit.rank == 0 : !(f & kBig));
+        // Lipschitz sums against the previous reference point: from the second
+        // step on, and for every backtracking trial (stepping == 2)
+        const bool lip = valid && (stepping == 2 || (stepping && iter > 0)) && (f & kInView);
+
+        // Wirelength gradient of the object: its pins' gradients added in pin
+        // order (EPlace/eplace.cpp:539-547).  The per-net pass wrote them in
+        // object-major order, so the objects of a warp own one contiguous run
+        // of gradient slots: the warp stages that run in shared memory with
+        // coalesced loads all in flight at once (kPinChunk per round), then
+        // every lane adds its own pins from there in order.  Fillers own none.
+        const int wend = (int)__reduce_max_sync(kFull, valid ? (unsigned)c.pe : 0u);
+        const int wbeg = min((int)__reduce_min_sync(kFull, valid ? (unsigned)c.ps : 0x7fffffffu), wend);
+        vec2<R> pv[kPinChunk / 32];
+#pragma unroll
+        for (int u = 0; u < kPinChunk / 32; u++)
+            if (wbeg + lane + 32 * u < wend) pv[u] = pin_grad[wbeg + lane + 32 * u];
+        vec2<R> p = mk2<R>((R)0, (R)0), gp = p, yp = p;
+        if (o < d.n_obj) p = pos[o];
+        if (lip) {
+            gp = g_prev[o];
+            yp = y_prev[o];
+        }
+        next = load_static(d, o < d.n_obj - stride ? o + stride : d.n_obj);
+        vec2<R> gd = mk2<R>((R)0, (R)0);
+        if (big) {
+            if (o < d.n_obj) gd = gather_big<R>(g, p, c.size, f, c.sxy, field, huge, pin_sm[0]);  // uniform per unit
+        } else if (valid) {
+            gd = gather_small<R>(g, gather_rect<R>(g, p, c.size, f), smoothing_scale<R>(g, c.sxy, c.size, f), field);
+        }
+        R wx = (R)0, wy = (R)0;
+        vec2<R> *sm = pin_sm[wid];
         for (int base = wbeg; base < wend; base += kPinChunk) {  // warp-uniform
             const int n = min(kPinChunk, wend - base);
 #pragma unroll
             for (int u = 0; u < kPinChunk / 32; u++) {
                 const int t = lane + 32 * u;
-                if (t < n) sm[t] = pin_grad[base + t];
+                if (t < n) sm[t] = base == wbeg ? pv[u] : pin_grad[base + t];
             }
             __syncwarp();
-            const int k1 = min(pe, base + n);
-            for (int k = max(ps, base); k < k1; k++) {
-                const vec2<R> v = sm[k - base];
-                wx = add_rn(wx, v.x);
-                wy = add_rn(wy, v.y);
-            }
-            __syncwarp();
-        }
-    }
-    if (o < d.n_obj) {
-        uint8_t f = d.flags[o];
-        vec2<R> p = pos[o];
-        R gdx = (R)0, gdy = (R)0;
-        if (f & kBig) {
-            vec2<R> v = gd_big[d.big_slot[o]];
-            gdx = v.x;
-            gdy = v.y;
-        } else {
-            const float2 sz = d.size[o];
-            const FRect<R> r = gather_rect<R>(g, p, sz, f);
-            const R sxy = smoothing_scale<R>(g, d.sxy[o], sz, f);
-            int i0, i1, j0, j1;
-            gather_range<R>(g, r, i0, i1, j0, j1);
-            for (int i = i0; i <= i1; i++)
-                for (int j = j0; j <= j1; j++) {
-                    vec2<R> v = gather_bin<R>(g, r, sxy, i, j, field);
-                    gdx += v.x;
-                    gdy += v.y;
+            if (valid) {
+                const int k1 = min(c.pe, base + n);
+                for (int k = max(c.ps, base); k < k1; k++) {
+                    const vec2<R> v = sm[k - base];
+                    wx = add_rn(wx, v.x);
+                    wy = add_rn(wy, v.y);
                 }
+            }
+            __syncwarp();
         }
-        // preconditioner 1/max(1, #pins + lambda*area) and direction
-        R den = max_r((R)1, add_rn((R)d.npins[o], mul_rn(lam, (R)d.area[o])));
-        R pre = div_rn((R)1, den);
-        vec2<R> gg;
-        if (f & kFiller) {
-            gg.x = mul_rn(mul_rn(pre, lam), gdx);
-            gg.y = mul_rn(mul_rn(pre, lam), gdy);
-        } else {
-            gg.x = mul_rn(pre, sub_rn(mul_rn(lam, gdx), wx));
-            gg.y = mul_rn(pre, sub_rn(mul_rn(lam, gdy), wy));
+        if (valid) {
+            // preconditioner 1/max(1, #pins + lambda*area) and direction
+            R den = max_r((R)1, add_rn((R)c.npins, mul_rn(lam, (R)c.area)));
+            R pre = div_rn((R)1, den);
+            vec2<R> gg;
+            if (f & kFiller) {
+                gg.x = mul_rn(mul_rn(pre, lam), gd.x);
+                gg.y = mul_rn(mul_rn(pre, lam), gd.y);
+            } else {
+                gg.x = mul_rn(pre, sub_rn(mul_rn(lam, gd.x), wx));
+                gg.y = mul_rn(pre, sub_rn(mul_rn(lam, gd.y), wy));
+            }
+            gout[o] = gg;
+            if (dump_gd) {
+                dump_gd[o] = gd;
+                dump_gwl[o] = mk2<R>(wx, wy);
+            }
+            if (lip) {
+                double dgx = sub_rn(gg.x, gp.x), dgy = sub_rn(gg.y, gp.y);
+                double dyx = sub_rn(p.x, yp.x), dyy = sub_rn(p.y, yp.y);
+                acc[0] += dgx * dgx + dgy * dgy;
+                acc[1] += dyx * dyx + dyy * dyy;
+                acc[2] += dyx * dgx + dyy * dgy;
+            }
+            if (S->lambda0_mode) {
+                if (!(f & kFiller)) acc[3] += fabs((double)wx) + fabs((double)wy);
+                acc[4] += fabs((double)gd.x) + fabs((double)gd.y);
+            }
         }
-        gout[o] = gg;
-        if (dump_gd) {
-            dump_gd[o] = mk2<R>(gdx, gdy);
-            dump_gwl[o] = mk2<R>(wx, wy);
-        }
-        // Lipschitz sums against the previous reference point: from the
-        // second step on, and for every backtracking trial (stepping == 2)
-        if ((stepping == 2 || (stepping && iter > 0)) && (f & kInView)) {
-            vec2<R> gp = g_prev[o], yp = y_prev[o];
-            double dgx = sub_rn(gg.x, gp.x), dgy = sub_rn(gg.y, gp.y);
-            double dyx = sub_rn(p.x, yp.x), dyy = sub_rn(p.y, yp.y);
-            acc[0] = dgx * dgx + dgy * dgy;
-            acc[1] = dyx * dyx + dyy * dyy;
-            acc[2] = dyx * dgx + dyy * dgy;
-        }
-        if (S->lambda0_mode) {
-            if (!(f & kFiller)) acc[3] = fabs((double)wx) + fabs((double)wy);
-            acc[4] = fabs((double)gdx) + fabs((double)gdy);
-        }
+    } while (!big && __shfl_sync(kFull, next.o, 0) < d.n_obj);
+    // only the sums that this call reads: the step's three, or lambda_0's two
+    bool last = false;
+    if (stepping && !S->lambda0_mode) {
+        double a3[3] = {acc[0], acc[1], acc[2]};
+        last = grid_sum<3>(a3, sh, partials, &S->cnt_comb, gridDim.x, blockIdx.x);
+        for (int k = 0; k < 3; k++) acc[k] = a3[k];
+    } else if (stepping || S->lambda0_mode) {
+        last = grid_sum<5>(acc, sh, partials, &S->cnt_comb, gridDim.x, blockIdx.x);
     }
-    if (grid_sum<5>(acc, sh, partials, &S->cnt_comb, gridDim.x, blockIdx.x) && threadIdx.x == 0) {
+    if (last && threadIdx.x == 0) {
         {
             double dg2 = acc[0], dy2 = acc[1], sy = acc[2];
             double l1w = acc[3], l1d = acc[4];
@@ -988,7 +1108,7 @@ k_combine(Grid g, DeviceNetlist d, const vec2<R> *__restrict__ field, const vec2
 // (opt_step_vanilla, Optimization/nesterov.hpp:391-404); returns the clamped
 // new position, which becomes the object's position.
 template <typename R>
-__device__ __forceinline__ vec2<R> nesterov_move(const Grid &g, int o, R s, R c, const float2 *__restrict__ size,
+__device__ __forceinline__ vec2<R> nesterov_move(const Grid &g, int o, R s, R c, float2 size,
                                                  vec2<R> *__restrict__ pos, vec2<R> *__restrict__ x,
                                                  const vec2<R> *__restrict__ gin, vec2<R> *__restrict__ y_prev,
                                                  vec2<R> *__restrict__ g_prev) {
@@ -998,7 +1118,7 @@ __device__ __forceinline__ vec2<R> nesterov_move(const Grid &g, int o, R s, R c,
     y_prev[o] = y;
     g_prev[o] = gg;
     x[o] = xn;
-    const vec2<R> p = clamp_center<R>(g, yn, size[o]);
+    const vec2<R> p = clamp_center<R>(g, yn, size);
     pos[o] = p;
     return p;
 }
@@ -1022,44 +1142,45 @@ k_update(Grid g, int n, const uint8_t *__restrict__ flags, const float2 *__restr
     if (S->done) return;
     int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o < n && (flags[o] & kInView))
-        nesterov_move<R>(g, o, (R)S->step, (R)S->coef, size, pos, x, gin, y_prev, g_prev);
+        nesterov_move<R>(g, o, (R)S->step, (R)S->coef, size[o], pos, x, gin, y_prev, g_prev);
     if (threadIdx.x == 0 && last_block(&S->cnt_upd, gridDim.x)) end_step(S);
 }
 
 // The update of the captured loop, with the next evaluation's scatter fused
 // in: every object is scattered at its new position right after its move
-// (objects outside the stage view at their unchanged one).  kBig objects are
-// moved and scattered by a block of their own (the blocks after
-// small_blocks).  The step that ends the stage scatters nothing, so the maps
-// stay clear (prep clears them after each read).
-template <typename R>
-__global__ void __launch_bounds__(kThreads)
-k_update_scatter(Grid g, int n, int small_blocks, const int32_t *__restrict__ big, const uint8_t *__restrict__ flags,
-                 const float2 *__restrict__ size, vec2<R> *__restrict__ pos, vec2<R> *__restrict__ x,
+// (objects outside the stage view at their unchanged one); of a kBig object's
+// threads the first moves it.  The step that ends the stage scatters nothing,
+// so the maps stay clear (prep clears them after each read).
+// MINB: blocks an SM that the registers have to allow.  Six hide the latency of
+// a large design's atomics, though they spill a few registers; a design whose
+// blocks are all resident anyway takes the instance without.
+template <int MINB, typename R>
+__global__ void __launch_bounds__(kThreads, MINB)
+k_update_scatter(Grid g, DeviceNetlist d, int big_blocks, vec2<R> *__restrict__ pos, vec2<R> *__restrict__ x,
                  const vec2<R> *__restrict__ gin, vec2<R> *__restrict__ y_prev, vec2<R> *__restrict__ g_prev,
-                 double qscale, ull *__restrict__ node_q, ull *__restrict__ filler_q, DevScalars *__restrict__ S) {
+                 double qscale, ull *__restrict__ maps, DevScalars *__restrict__ S) {
+    __shared__ vec2<R> big_pos[kThreads / 32];
+    const ObjectUnit u = object_unit(d, big_blocks);
+    const bool valid = u.o < d.n_obj;
+    const uint8_t f = valid ? d.flags[u.o] : 0;
+    const float2 sz = valid ? d.size[u.o] : make_float2(1.f, 1.f);
+    const float sxy = valid ? d.sxy[u.o] : 0.f;
     pdl_begin();
-    __shared__ vec2<R> big_pos;
     if (S->done) return;
     const R s = (R)S->step, c = (R)S->coef;
     const bool scatter = !S->stop_pending;
-    if ((int)blockIdx.x >= small_blocks) {
-        const int o = big[blockIdx.x - small_blocks];
-        const uint8_t f = flags[o];
-        if (threadIdx.x == 0)
-            big_pos = (f & kInView) ? nesterov_move<R>(g, o, s, c, size, pos, x, gin, y_prev, g_prev) : pos[o];
-        __syncthreads();
-        if (scatter) scatter_big_object<R>(g, big_pos, size[o], f, qscale, node_q, filler_q);
+    auto move = [&] {
+        return (f & kInView) ? nesterov_move<R>(g, u.o, s, c, sz, pos, x, gin, y_prev, g_prev) : pos[u.o];
+    };
+    if (u.count == 1) {
+        const bool mine = valid && !(f & kBig);
+        const vec2<R> p = mine ? move() : mk2<R>((R)g.llx, (R)g.lly);
+        if (scatter) scatter_objects<R>(g, mine, p, sz, sxy, f, qscale, maps);
     } else {
-        const int o = blockIdx.x * blockDim.x + threadIdx.x;
-        if (o < n) {
-            const uint8_t f = flags[o];
-            if (!(f & kBig)) {
-                const vec2<R> p =
-                    (f & kInView) ? nesterov_move<R>(g, o, s, c, size, pos, x, gin, y_prev, g_prev) : pos[o];
-                if (scatter) scatter_small_object<R>(g, p, size[o], f, qscale, node_q, filler_q);
-            }
-        }
+        const int slot = u.count == kThreads ? 0 : threadIdx.x >> 5;
+        if (valid && u.rank == 0) big_pos[slot] = move();
+        __syncthreads();  // block-uniform: every unit of this block has several threads
+        if (valid && scatter) scatter_big<R>(g, big_pos[slot], sz, sxy, f, qscale, u.rank, u.count, maps);
     }
     if (threadIdx.x == 0 && last_block(&S->cnt_upd, gridDim.x)) end_step(S);
 }
@@ -1149,12 +1270,17 @@ int launch_priority(bool high) {
     return high ? range.y : range.x;
 }
 
-int prep_blocks(const Grid &g) { return std::min(blocks_for(g.nx * g.ny, kThreads), 148 * 8); }
+int prep_blocks(const Grid &g) { return std::min(blocks_for(g.nx * g.ny, kThreads), kSms * 8); }
+
+// Blocks of the object kernels that take the kBig objects (object_unit).
+static int big_blocks(const DeviceNetlist &d) {
+    return d.n_huge_objs + blocks_for(d.n_big_objs - d.n_huge_objs, kThreads / 32);
+}
 
 int reduction_blocks(const DeviceNetlist &d, int which) {
     switch (which) {
         case 0: return d.n_block_nets + blocks_for(d.n_net_tasks - d.n_block_nets, kNetWarps);
-        default: return blocks_for(d.n_obj, kThreads);
+        default: return big_blocks(d) + std::min(blocks_for(d.n_obj, kThreads), kCombineBlocks);
     }
 }
 
@@ -1170,30 +1296,29 @@ inline const vec2<R> *V(const void *p) {
 }  // namespace
 
 template <typename R>
-static void scatter_t(const KernelCtx &c, const DeviceNetlist &d, ull *node_q, ull *filler_q, const DevScalars *S,
-                      cudaStream_t st) {
-    const int sb = blocks_for(d.n_obj, kThreads);
-    launch_k(k_scatter<R>, sb + d.n_big_objs, kThreads, 0, st, c.grid, V<R>(d.pos), d.size, d.flags, d.n_obj, sb,
-             d.big_objs, c.qscale, node_q, filler_q, S);
+static void scatter_t(const KernelCtx &c, const DeviceNetlist &d, ull *maps, const DevScalars *S, cudaStream_t st) {
+    const int bb = big_blocks(d);
+    launch_k(k_scatter<R>, bb + blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d, bb, c.qscale, maps, S);
 }
 
-void launch_scatter(const KernelCtx &c, const DeviceNetlist &d, ull *node_q, ull *filler_q, const DevScalars *S,
-                    cudaStream_t st) {
-    c.fp64 ? scatter_t<double>(c, d, node_q, filler_q, S, st) : scatter_t<float>(c, d, node_q, filler_q, S, st);
+void launch_scatter(const KernelCtx &c, const DeviceNetlist &d, ull *maps, const DevScalars *S, cudaStream_t st) {
+    c.fp64 ? scatter_t<double>(c, d, maps, S, st) : scatter_t<float>(c, d, maps, S, st);
 }
 
 template <typename R>
 static void update_scatter_t(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
-                             void *y_prev, void *g_prev, ull *node_q, ull *filler_q, DevScalars *S, cudaStream_t st) {
-    const int sb = blocks_for(d.n_obj, kThreads);
-    launch_k(k_update_scatter<R>, sb + d.n_big_objs, kThreads, 0, st, c.grid, d.n_obj, sb, d.big_objs, d.flags,
-             d.size, V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), c.qscale, node_q, filler_q, S);
+                             void *y_prev, void *g_prev, ull *maps, DevScalars *S, cudaStream_t st) {
+    const int bb = big_blocks(d);
+    const int blocks = bb + blocks_for(d.n_obj, kThreads);
+    constexpr int kMany = sizeof(R) == 8 ? 5 : 6;
+    launch_k(blocks <= kSms * 4 ? k_update_scatter<1, R> : k_update_scatter<kMany, R>, blocks, kThreads, 0, st, c.grid,
+             d, bb, V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), c.qscale, maps, S);
 }
 
 void launch_update_scatter(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
-                           void *y_prev, void *g_prev, ull *node_q, ull *filler_q, DevScalars *S, cudaStream_t st) {
-    c.fp64 ? update_scatter_t<double>(c, d, pos, x, g, y_prev, g_prev, node_q, filler_q, S, st)
-           : update_scatter_t<float>(c, d, pos, x, g, y_prev, g_prev, node_q, filler_q, S, st);
+                           void *y_prev, void *g_prev, ull *maps, DevScalars *S, cudaStream_t st) {
+    c.fp64 ? update_scatter_t<double>(c, d, pos, x, g, y_prev, g_prev, maps, S, st)
+           : update_scatter_t<float>(c, d, pos, x, g, y_prev, g_prev, maps, S, st);
 }
 
 void launch_prep(const KernelCtx &c, ull *node_q, ull *filler_q, const float2 *static_map, void *rho,
@@ -1235,28 +1360,21 @@ void launch_wirelength(const KernelCtx &c, const DeviceNetlist &d, void *pin_gra
     c.fp64 ? wirelength_t<double>(c, d, pin_grad, S, st) : wirelength_t<float>(c, d, pin_grad, S, st);
 }
 
-void launch_gather_big(const KernelCtx &c, const DeviceNetlist &d, const void *field, void *gd_big,
-                       const DevScalars *S, cudaStream_t st) {
-    if (d.n_big_objs == 0) return;
-    if (c.fp64)
-        launch_k(k_gather_big<double>, d.n_big_objs, 128, 0, st, c.grid, V<double>(d.pos), d.size, d.flags, d.sxy,
-                 d.big_objs, V<double>(field), V<double>(gd_big), S);
-    else
-        launch_k(k_gather_big<float>, d.n_big_objs, 128, 0, st, c.grid, V<float>(d.pos), d.size, d.flags, d.sxy,
-                 d.big_objs, V<float>(field), V<float>(gd_big), S);
+template <typename R>
+static void combine_t(const KernelCtx &c, const DeviceNetlist &d, const void *field, const void *pin_grad, void *g,
+                      const void *g_prev, const void *y_prev, void *dump_gd, void *dump_gwl, int stepping,
+                      DevScalars *S, cudaStream_t st) {
+    const int bb = big_blocks(d);
+    launch_k(k_combine<R>, reduction_blocks(d, 1), kThreads, 0, st, c.grid, d, V<R>(field),
+             V<R>(pin_grad), V<R>(g), V<R>(g_prev), V<R>(y_prev), V<R>(dump_gd), V<R>(dump_gwl), bb, stepping,
+             c.part_comb, S);
 }
 
-void launch_combine(const KernelCtx &c, const DeviceNetlist &d, const void *field, const void *gd_big,
-                    const void *pin_grad, void *g, const void *g_prev, const void *y_prev, void *dump_gd,
-                    void *dump_gwl, int stepping, DevScalars *S, cudaStream_t st) {
-    if (c.fp64)
-        launch_k(k_combine<double>, blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d, V<double>(field),
-                 V<double>(gd_big), V<double>(pin_grad), V<double>(g), V<double>(g_prev), V<double>(y_prev),
-                 V<double>(dump_gd), V<double>(dump_gwl), stepping, c.part_comb, S);
-    else
-        launch_k(k_combine<float>, blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d, V<float>(field),
-                 V<float>(gd_big), V<float>(pin_grad), V<float>(g), V<float>(g_prev), V<float>(y_prev),
-                 V<float>(dump_gd), V<float>(dump_gwl), stepping, c.part_comb, S);
+void launch_combine(const KernelCtx &c, const DeviceNetlist &d, const void *field, const void *pin_grad, void *g,
+                    const void *g_prev, const void *y_prev, void *dump_gd, void *dump_gwl, int stepping, DevScalars *S,
+                    cudaStream_t st) {
+    c.fp64 ? combine_t<double>(c, d, field, pin_grad, g, g_prev, y_prev, dump_gd, dump_gwl, stepping, S, st)
+           : combine_t<float>(c, d, field, pin_grad, g, g_prev, y_prev, dump_gd, dump_gwl, stepping, S, st);
 }
 
 template <typename R>
@@ -1326,8 +1444,9 @@ static void loop_kernels(std::vector<const void *> &fns) {
     const void *f[] = {(const void *)k_scatter<R>, (const void *)k_prep<R>, (const void *)k_wl<true, false, false, R>,
                        (const void *)k_wl<true, true, false, R>, (const void *)k_wl<true, false, true, R>,
                        (const void *)k_wl<true, true, true, R>, (const void *)k_wl<false, false, false, R>,
-                       (const void *)k_gather_big<R>, (const void *)k_combine<R>, (const void *)k_update<R>,
-                       (const void *)k_update_scatter<R>, (const void *)k_bktrk_move<R>,
+                       (const void *)k_combine<R>, (const void *)k_update<R>,
+                       (const void *)k_update_scatter<1, R>,
+                       (const void *)k_update_scatter<sizeof(R) == 8 ? 5 : 6, R>, (const void *)k_bktrk_move<R>,
                        (const void *)k_stage_begin<R>, (const void *)k_wrap_up<R>};
     fns.insert(fns.end(), std::begin(f), std::end(f));
 }

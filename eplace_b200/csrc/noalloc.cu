@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "engine.h"
+#include "scatter.cuh"
 
 namespace ep {
 namespace {
@@ -73,14 +74,6 @@ __global__ void k_noalloc_clear(unsigned long long *__restrict__ s, int n) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) s[k] = 0ull;
 }
 
-__device__ __forceinline__ void noalloc_add(const Grid &g, const Rect &r, float s, int i, int j, double qscale,
-                                            unsigned long long *__restrict__ map) {
-    float ovl = (float)rect_bin_overlap(g, r, i, j);
-    if (ovl == 0.0f) return;
-    long long q = __double2ll_rn(__dmul_rn((double)__fmul_rn(s, ovl), qscale));
-    atomicAdd(&map[(size_t)i * g.ny + j], (unsigned long long)q);
-}
-
 // Same contributions as the engine's scatter (EPlace/eplace.cpp:1029-1133).
 // A thread takes its object's bins when the footprint is small; objects that
 // may cover more than kNoallocSmallBins bins are queued in shared memory and
@@ -95,21 +88,19 @@ k_noalloc_scatter(Grid g, int n, const float *__restrict__ cx, const float *__re
     if (threadIdx.x == 0) n_big = 0;
     __syncthreads();
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o < n) {
-        const uint8_t f = flags ? flags[o] : 0;
-        const Rect r = object_rect(g, cx[o], cy[o], w[o], h[o]);
-        int i0, i1, j0, j1;
-        bin_range(g, r, i0, i1, j0, j1);
-        if ((long long)max(i1 - i0 + 1, 0) * max(j1 - j0 + 1, 0) > kNoallocSmallBins) {
-            big[atomicAdd(&n_big, 1)] = o;
-        } else {
-            float s = __fmul_rn(r.sx, r.sy);
-            if (f & kMacro) s = __fmul_rn(s, g.td);
-            unsigned long long *map = (f & kFiller) ? filler_q : node_q;
-            for (int i = i0; i <= i1; i++)
-                for (int j = j0; j <= j1; j++) noalloc_add(g, r, s, i, j, qscale, map);
-        }
+    const bool valid = o < n;
+    const uint8_t f = valid && flags ? flags[o] : 0;
+    const Rect r = valid ? object_rect(g, cx[o], cy[o], w[o], h[o]) : Rect{};
+    int i0 = 0, i1 = -1, j0 = 0, j1 = -1;
+    if (valid) bin_range(g, r, i0, i1, j0, j1);
+    if ((long long)max(i1 - i0 + 1, 0) * max(j1 - j0 + 1, 0) > kNoallocSmallBins) {
+        big[atomicAdd(&n_big, 1)] = o;
+        i1 = i0 - 1;
     }
+    float s = __fmul_rn(r.sx, r.sy);
+    if (f & kMacro) s = __fmul_rn(s, g.td);
+    const unsigned bin = (unsigned)(i0 * g.ny + j0) + ((f & kFiller) ? (unsigned)(g.nx * g.ny) : 0u);
+    scatter_by_lane<float>(g, r, s, i0, i1, j0, j1, qscale, bin, node_q);  // the filler map lies behind
     __syncthreads();
     for (int k = 0; k < n_big; k++) {
         const int b = big[k];
@@ -120,8 +111,7 @@ k_noalloc_scatter(Grid g, int n, const float *__restrict__ cx, const float *__re
         float s = __fmul_rn(r.sx, r.sy);
         if (f & kMacro) s = __fmul_rn(s, g.td);
         unsigned long long *map = (f & kFiller) ? filler_q : node_q;
-        const int wy = j1 - j0 + 1, nbins = (i1 - i0 + 1) * wy;
-        for (int t = threadIdx.x; t < nbins; t += blockDim.x) noalloc_add(g, r, s, i0 + t / wy, j0 + t % wy, qscale, map);
+        scatter_by_group<float>(g, r, s, i0, i1, j0, j1, qscale, threadIdx.x, blockDim.x, map);
     }
 }
 
