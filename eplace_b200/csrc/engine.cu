@@ -897,21 +897,25 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
     // previous ranges' pins of the same object end
     std::vector<int32_t> ops(no + 1, 0), pin_slot(np, -1);
     {
-        std::vector<std::vector<int32_t>> cnt(nth, std::vector<int32_t>(no, 0));
+        std::vector<std::vector<int32_t>> cnt(nth);
         parallel_ranges(np, nth, [&](int t, int p0, int p1) {
+            cnt[t].assign(no, 0);
             for (int p = p0; p < p1; p++)
                 if (owner[p] < no) cnt[t][owner[p]]++;
         });
-        for (int o = 0; o < no; o++) {
-            int32_t at = 0;
-            for (int t = 0; t < nth; t++) {
-                const int32_t c = cnt[t][o];
-                cnt[t][o] = at;  // this thread's first slot, relative to the object's start
-                at += c;
+        parallel_ranges(no, nth, [&](int, int o0, int o1) {
+            for (int o = o0; o < o1; o++) {
+                int32_t at = 0;
+                for (int t = 0; t < nth; t++) {
+                    const int32_t c = cnt[t][o];
+                    cnt[t][o] = at;  // this thread's first slot, relative to the object's start
+                    at += c;
+                }
+                ops[o + 1] = at;
+                if (o < nn) h_npins[o] = (float)at;
             }
-            ops[o + 1] = ops[o] + at;
-            if (o < nn) h_npins[o] = (float)at;
-        }
+        });
+        for (int o = 0; o < no; o++) ops[o + 1] += ops[o];
         parallel_ranges(np, nth, [&](int t, int p0, int p1) {
             for (int p = p0; p < p1; p++)
                 if (owner[p] < no) pin_slot[p] = ops[owner[p]] + cnt[t][owner[p]]++;
@@ -929,23 +933,33 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
     {
         std::vector<std::vector<int>> by_deg(kWarpPins + 1);
         std::vector<int> big_list;
-        // by lowest owner (a counting sort), so that neighbouring nets of a
-        // degree read neighbouring centres
-        std::vector<int32_t> low(nnet), at(no + nt + 1, 0), by_low(nnet);
+        for (int n = 0; n < nnet; n++) {
+            int deg = net_start[n + 1] - net_start[n];
+            (deg > kWarpPins ? big_list : by_deg[deg]).push_back(n);
+        }
+        // by lowest owner inside a degree, so that neighbouring nets read
+        // neighbouring centres: a counting sort over runs of 64 objects
+        std::vector<int32_t> low(nnet);
         parallel_ranges(nnet, nth, [&](int, int n0, int n1) {
             for (int n = n0; n < n1; n++) {
                 int32_t m = no + nt - 1;
                 for (int p = net_start[n]; p < net_start[n + 1]; p++) m = std::min(m, owner[p]);
-                low[n] = m;
+                low[n] = m >> 6;
             }
         });
-        for (int n = 0; n < nnet; n++) at[low[n] + 1]++;
-        for (int o = 0; o < no + nt; o++) at[o + 1] += at[o];
-        for (int n = 0; n < nnet; n++) by_low[at[low[n]]++] = n;
-        for (int n : by_low) {
-            int deg = net_start[n + 1] - net_start[n];
-            (deg > kWarpPins ? big_list : by_deg[deg]).push_back(n);
-        }
+        std::atomic<int> next_deg{1};
+        parallel_ranges(nth, nth, [&](int, int, int) {
+            std::vector<int32_t> at, sorted;
+            for (int d; (d = next_deg++) <= kWarpPins;) {
+                if (by_deg[d].size() < 2) continue;
+                at.assign(((no + nt - 1) >> 6) + 2, 0);
+                sorted.resize(by_deg[d].size());
+                for (int n : by_deg[d]) at[low[n] + 1]++;
+                for (size_t o = 1; o < at.size(); o++) at[o] += at[o - 1];
+                for (int n : by_deg[d]) sorted[at[low[n]]++] = n;
+                std::copy(sorted.begin(), sorted.end(), by_deg[d].begin());
+            }
+        });
         std::stable_sort(big_list.begin(), big_list.end(), [&](int a, int b) {
             return net_start[a + 1] - net_start[a] > net_start[b + 1] - net_start[b];
         });
@@ -1013,11 +1027,15 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
     });
 
     // stage views (EPlace/eplace.cpp:190-203)
-    for (int v = 0; v < 3; v++) e->h_view[v].reserve(no);
-    for (int o = 0; o < no; o++) {
-        e->h_view[EP_STAGE_MGP].push_back(o);
-        if (o >= nn) e->h_view[EP_STAGE_FILLERONLY].push_back(o);
-        if (o >= nn || !is_macro[o]) e->h_view[EP_STAGE_CGP].push_back(o);
+    e->h_view[EP_STAGE_MGP].resize(no);
+    for (int o = 0; o < no; o++) e->h_view[EP_STAGE_MGP][o] = o;
+    e->h_view[EP_STAGE_FILLERONLY].assign(e->h_view[EP_STAGE_MGP].begin() + nn, e->h_view[EP_STAGE_MGP].end());
+    if (e->n_macros == 0) {
+        e->h_view[EP_STAGE_CGP] = e->h_view[EP_STAGE_MGP];
+    } else {
+        e->h_view[EP_STAGE_CGP].reserve(no);
+        for (int o = 0; o < no; o++)
+            if (o >= nn || !is_macro[o]) e->h_view[EP_STAGE_CGP].push_back(o);
     }
     e->n_cgp = (int)e->h_view[EP_STAGE_CGP].size();
 
