@@ -2102,20 +2102,23 @@ ep_status qp_setup(ep_engine *e) {
 
     // at most 4 entries per pin and axis: every counted pair of a net involves
     // one of its two bound pins (< 2 d pairs, two entries each)
-    const size_t cap = 4 * (size_t)np + 16;
+    const size_t cap = qp_entry_cap(nn, np);
+    const size_t n2 = ((size_t)nn + 1) & ~(size_t)1;  // the vector kernels take rows in pairs
+    unsigned char *layout = nullptr;
     const int pb = qp_partial_blocks(nn, nnet);
     ep_status s;
     if ((s = dalloc(e, q.bound, std::max(nnet, 1))) || (s = dalloc(e, q.abspin, std::max(np, 1))) ||
-        (s = dalloc(e, q.count, 2 * (size_t)nn)) || (s = dalloc(e, q.row_x, (size_t)nn + 1)) ||
-        (s = dalloc(e, q.row_y, (size_t)nn + 1)) || (s = dalloc(e, q.col_x, cap)) || (s = dalloc(e, q.col_y, cap)) ||
-        (s = dalloc(e, q.val_x, cap)) || (s = dalloc(e, q.val_y, cap)) || (s = dalloc(e, q.diag, nn)) ||
-        (s = dalloc(e, q.rhs, nn)) || (s = dalloc(e, q.x, nn)) || (s = dalloc(e, q.r, nn)) ||
-        (s = dalloc(e, q.r0, nn)) || (s = dalloc(e, q.p, nn)) || (s = dalloc(e, q.v, nn)) ||
-        (s = dalloc(e, q.s, nn)) || (s = dalloc(e, q.t, nn)) || (s = dalloc(e, q.partials, 4 * (size_t)pb)) ||
+        (s = dalloc(e, q.count, 2 * (size_t)nn)) || (s = dalloc(e, layout, qp_layout_bytes(nn))) ||
+        (s = dalloc(e, q.ent_x, cap)) || (s = dalloc(e, q.ent_y, cap)) ||
+        (s = dalloc(e, q.diag, n2)) ||
+        (s = dalloc(e, q.rhs, n2)) || (s = dalloc(e, q.x, n2)) || (s = dalloc(e, q.r, n2)) ||
+        (s = dalloc(e, q.r0, n2)) || (s = dalloc(e, q.p, n2)) || (s = dalloc(e, q.v, n2)) ||
+        (s = dalloc(e, q.s, n2)) || (s = dalloc(e, q.t, n2)) || (s = dalloc(e, q.partials, 4 * (size_t)pb)) ||
         (s = dalloc(e, q.cnt, 1)) || (s = dalloc(e, q.out, 4)) || (s = dalloc(e, q.solve, 1)) ||
-        (s = dalloc(e, q.scan, (size_t)qp_scan_blocks(nn) + 2)) || (s = dalloc(e, q.y, nn)) ||
-        (s = dalloc(e, q.z, nn)) || (s = dalloc(e, q.dinv, nn)))
+        (s = dalloc(e, q.y, n2)) ||
+        (s = dalloc(e, q.z, n2)) || (s = dalloc(e, q.dinv, n2)))
         return s;
+    q.layout = layout;
     q.pin_net = e->pin_net;
     q.net_first = e->net_first;
     q.net_deg = e->net_deg;
@@ -2140,14 +2143,14 @@ ep_status qp_read(ep_engine *e, int n) {
 // Build both systems at the centres of the last bounds pass (its bound pins
 // and pin positions): count, prefix sum, fill.
 ep_status qp_build(ep_engine *e) {
-    // counts, the CSR offsets by a scan on the device, then the entries: no
+    // counts, the rows' places by a scan on the device, then the entries: no
     // host round trip (an allocation overflow is flagged in the solver state
     // and reported by qp_solve)
     QpDev &q = e->qp;
     qp_rows(q, 0, e->st);
-    qp_offsets(q, e->st);
+    qp_scan(q, e->st);
     qp_rows(q, 1, e->st);
-    e->qp_launches += 5;
+    e->qp_launches += 3;
     CK(cudaGetLastError());
     return EP_OK;
 }
@@ -2157,31 +2160,62 @@ ep_status qp_build(ep_engine *e) {
 // device (qp.cu): stop when |r|^2 <= (eps |b|)^2 with eps the float epsilon,
 // or after max_it iterations; the current centres are the initial guess.
 // The host enqueues iterations in chunks and reads the solver state once per
-// chunk.  err[c] = |r|/|b| at the end, the value QPPlacer reads as
+// chunk, some iterations before the chunk's end, so that the device has work
+// while the host reads it and enqueues more.  An iteration that finds a restart
+// owed leaves everything to the restart kernel, which the host launches when it
+// sees the flag (r0.r rarely vanishes: a launch in every iteration for it cost
+// 2.5 us).  err[c] = |r|/|b| at the end, the value QPPlacer reads as
 // solver.error().
 ep_status qp_solve(ep_engine *e, const float2 *qpos, int max_it, bool jacobi, double err[2], int &iters) {
     QpDev &q = e->qp;
     cudaStream_t st = e->st;
-    constexpr int kChunk = 10;
+    constexpr int kChunk = 10, kAhead = 4;
     qp_to_x(q, qpos, st);
     if (jacobi) qp_dinv(q, st);
     qp_init(q, max_it, st);
     e->qp_launches += 3 + (jacobi ? 1 : 0);
     QpSolve h{};
-    for (int done = 0; done < max_it;) {
-        const int n = std::min(kChunk, max_it - done);
-        qp_iterations(q, n, jacobi, st);
-        e->qp_launches += 6LL * n;
-        done += n;
-        CK(cudaMemcpyAsync(e->qp_state_h, q.solve, sizeof(QpSolve), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+    auto state = [&]() -> ep_status {
+        CK(cudaEventSynchronize(e->ev_poll));
         h = *e->qp_state_h;
         if (h.overflow) {
             e->err = "quadratic placement: more matrix entries than the bound allows";
             return EP_ERR_STATE;
         }
+        return EP_OK;
+    };
+    auto ask = [&]() -> ep_status {
+        CK(cudaMemcpyAsync(e->qp_state_h, q.solve, sizeof(QpSolve), cudaMemcpyDeviceToHost, st));
+        CK(cudaEventRecord(e->ev_poll, st));
+        return EP_OK;
+    };
+    auto run = [&](int n) {
+        qp_iterations(q, n, jacobi, st);
+        e->qp_launches += 5LL * n;
+    };
+    ep_status s;
+    // iterations the device may still take: max_it in all, those skipped while a
+    // restart was owed not counted
+    for (int left = max_it; left > 0;) {
+        const int n = std::min(kChunk, left), tail = n > kAhead ? kAhead : 0;
+        run(n - tail);
+        if ((s = ask())) return s;
+        run(tail);
+        left -= n;
+        if ((s = state())) return s;
         if (!h.active[0] && !h.active[1]) break;
+        if (h.restart_mask || left == 0) {
+            // a restart may be owed since any iteration up to the last enqueued
+            if ((s = ask()) || (s = state())) return s;
+            if (!h.active[0] && !h.active[1]) break;
+            if (h.restart_mask && h.iters < max_it) {
+                qp_restart(q, st);
+                e->qp_launches += 1;
+                left = max_it - h.iters;
+            }
+        }
     }
+    if ((s = ask()) || (s = state())) return s;
     CK(cudaGetLastError());
     iters = h.iters;
     for (int c = 0; c < 2; c++) err[c] = h.bb[c] > 0.0 ? std::sqrt(h.rr[c] / h.bb[c]) : 0.0;

@@ -217,6 +217,7 @@ struct QpSolve {
     int it[2], restarts[2], active[2];
     int restart_mask, zero_mask, iters, max_it;
     int overflow;  // the last matrix build needed more entries than allocated
+    int n_long;    // long rows of the last matrix build
 };
 // Device view of one engine's quadratic placement: the netlist in device pin
 // order (nets contiguous) plus the per-round systems and BiCGSTAB vectors,
@@ -233,9 +234,9 @@ struct QpDev {
     int4 *bound;                                 // per net: x-min, x-max, y-min, y-max pin (in net)
     float2 *abspin;                              // [np] pin positions (device order) at the last bounds pass
     int32_t *count;                              // [2 nn] entries per row (X then Y)
-    int32_t *row_x, *row_y;                      // [nn + 1] CSR offsets
-    int32_t *col_x, *col_y;
-    float *val_x, *val_y;
+    void *layout;                                // where the rows' entries lie (QpLayout, qp.cu)
+    int2 *ent_x, *ent_y;                         // (column, value bits)
+    // vectors of nn rows, allocated to an even number
     float2 *diag, *rhs;
     float2 *x, *r, *r0, *p, *v, *s, *t;
     float2 *y, *z, *dinv;  // Jacobi-preconditioned solves: M^-1 p, M^-1 s, 1 / diagonal
@@ -243,19 +244,21 @@ struct QpDev {
     unsigned *cnt;
     double *out;      // [4] sums of the last reduction (bounds: HPWL)
     QpSolve *solve;   // device BiCGSTAB state
-    int32_t *scan;    // [qp_scan_blocks + 2] chunk totals of the row counts, then the two totals
     int cap_x, cap_y; // entries allocated per system
 };
 void qp_bounds(const QpDev &q, const float2 *pos, double *hpwl, cudaStream_t st);
 // the rows read the pin positions the last qp_bounds stored
 void qp_rows(const QpDev &q, int fill, cudaStream_t st);
-// CSR row offsets of both systems from the counts, on the device
-void qp_offsets(const QpDev &q, cudaStream_t st);
-int qp_scan_blocks(int nn);
+// where the rows' entries of both systems go, from the counts, on the device
+void qp_scan(const QpDev &q, cudaStream_t st);
+size_t qp_layout_bytes(int nn);
+size_t qp_entry_cap(int nn, int np);
 // r = b - A x and the solver's initial state (zero right-hand sides give x = 0)
 void qp_init(const QpDev &q, int max_it, cudaStream_t st);
-// enqueue `count` BiCGSTAB iterations (no-ops once both axes have stopped)
+// enqueue `count` BiCGSTAB iterations (no-ops once both axes have stopped, and
+// while a restart is owed)
 void qp_iterations(const QpDev &q, int count, bool jacobi, cudaStream_t st);
+void qp_restart(const QpDev &q, cudaStream_t st);
 // 1 / diagonal of both systems (the Jacobi preconditioner), after a build
 void qp_dinv(const QpDev &q, cudaStream_t st);
 void qp_to_x(const QpDev &q, const float2 *pos, cudaStream_t st);

@@ -195,16 +195,17 @@ k_prep(Grid g, ull *__restrict__ node_q, ull *__restrict__ filler_q, const float
             filler_q[k] = 0ull;
         }
     }
-    if (grid_sum<1>(acc, sh, partials, &S->cnt_prep, gridDim.x, blockIdx.x) && threadIdx.x == 0) {
-        {
-            double tau = acc[0] / area_norm;
-            S->tau = tau;
-            if (!isfinite(tau)) S->status |= 1 << EP_ERR_NAN;
-            double gx, gy;
-            inv_gamma(tau, g.sx, g.sy, gx, gy);
-            S->inv_gamma_x = gx;
-            S->inv_gamma_y = gy;
-        }
+    if (!grid_arrive<1>(acc, sh, partials, &S->cnt_prep, gridDim.x, blockIdx.x)) return;
+    const int status = S->status;
+    grid_total<1>(acc, sh, partials, &S->cnt_prep, gridDim.x);
+    if (threadIdx.x == 0) {
+        const double tau = acc[0] / area_norm;
+        S->tau = tau;
+        if (!isfinite(tau)) S->status = status | 1 << EP_ERR_NAN;
+        double gx, gy;
+        inv_gamma(tau, g.sx, g.sy, gx, gy);
+        S->inv_gamma_x = gx;
+        S->inv_gamma_y = gy;
     }
 }
 
@@ -316,26 +317,35 @@ __device__ __forceinline__ double lambda_multiplier(double cur, double last) {
     return fmin(fmax(m, 0.95), 1.05);
 }
 
-// HPWL finaliser shared by the wirelength kernels.
-__device__ void finish_wirelength(DevScalars *S, double hp, double wl) {
+// The scalars that the HPWL finalisers read, loaded ahead of them.
+struct HpwlScalars {
+    double lambda, last_hpwl;
+    int lambda_pending, lambda0_mode;
+};
+__device__ __forceinline__ HpwlScalars load_hpwl_scalars(const DevScalars *S) {
+    return HpwlScalars{S->lambda, S->last_hpwl, S->lambda_pending, S->lambda0_mode};
+}
+
+// HPWL finaliser of the wirelength pass.
+__device__ __forceinline__ void finish_wirelength(DevScalars *S, const HpwlScalars &h, double hp, double wl) {
     S->wirelength = wl;
     S->hpwl = hp;
     // atomic: the Poisson solve, running beside this pass, may raise a bit too
     if (!isfinite(hp)) atomicOr(&S->status, 1 << EP_ERR_NAN);
-    if (S->lambda_pending) {
-        S->lambda *= lambda_multiplier(hp, S->last_hpwl);
-        S->last_hpwl = hp;
+    if (h.lambda_pending) {
+        S->lambda = h.lambda * lambda_multiplier(hp, h.last_hpwl);
         S->lambda_pending = 0;
     }
-    if (S->lambda0_mode) S->last_hpwl = hp;  // penaltyFactorInitilization: lastHPWL = calcHPWL()
+    // updatePenaltyFactor's, or penaltyFactorInitilization's lastHPWL = calcHPWL()
+    if (h.lambda_pending || h.lambda0_mode) S->last_hpwl = hp;
 }
 
 // Finaliser of the HPWL-only pass (PlaceDB::calcHPWL): mode 0 stores it,
 // mode 1 applies updatePenaltyFactor, mode 2 applies it only if one is owed.
-__device__ void finish_hpwl(DevScalars *S, double hp, int mode) {
+__device__ __forceinline__ void finish_hpwl(DevScalars *S, const HpwlScalars &h, double hp, int mode) {
     S->hpwl_query = hp;
-    if (mode == 1 || (mode == 2 && S->lambda_pending)) {
-        S->lambda *= lambda_multiplier(hp, S->last_hpwl);
+    if (mode == 1 || (mode == 2 && h.lambda_pending)) {
+        S->lambda = h.lambda * lambda_multiplier(hp, h.last_hpwl);
         S->last_hpwl = hp;
         S->lambda_pending = 0;
     }
@@ -723,21 +733,26 @@ k_wl(const int4 *__restrict__ tasks, int n_block, int n_tasks, PinCtx<R> pc, vec
         }
     }
     // the smooth wirelength value rides along only when asked for
-    bool last;
+    unsigned *cnt = WL ? &S->cnt_wl : &S->cnt_hp;
     double acc[2] = {r.hpwl, r.value};
+    HpwlScalars h;
     if (WL && want_value) {
-        last = grid_sum<2>(acc, sh, partials, &S->cnt_wl, gridDim.x, blockIdx.x);
+        if (!grid_arrive<2>(acc, sh, partials, cnt, gridDim.x, blockIdx.x)) return;
+        h = load_hpwl_scalars(S);
+        grid_total<2>(acc, sh, partials, cnt, gridDim.x);
     } else {
         double a1[1] = {r.hpwl};
-        last = grid_sum<1>(a1, sh, partials, WL ? &S->cnt_wl : &S->cnt_hp, gridDim.x, blockIdx.x);
+        if (!grid_arrive<1>(a1, sh, partials, cnt, gridDim.x, blockIdx.x)) return;
+        h = load_hpwl_scalars(S);
+        grid_total<1>(a1, sh, partials, cnt, gridDim.x);
         acc[0] = a1[0];
         acc[1] = 0.0;
     }
-    if (last && threadIdx.x == 0) {
+    if (threadIdx.x == 0) {
         if (WL)
-            finish_wirelength(S, acc[0], acc[1]);
+            finish_wirelength(S, h, acc[0], acc[1]);
         else
-            finish_hpwl(S, acc[0], mode);
+            finish_hpwl(S, h, acc[0], mode);
     }
 }
 
@@ -896,19 +911,80 @@ __device__ __forceinline__ vec2<R> gather_big(const Grid &g, vec2<R> p, float2 s
 }
 
 // --------------------------------------------------------------- combine --
+// The scalars that the combine's finaliser reads, loaded ahead of it.
+struct CombineScalars {
+    double tau, step, a, bk_ratio;
+    int iter, stage, max_iter, step_cap, status, step_rule, lambda0_mode;
+    float target_overflow;
+};
+__device__ __forceinline__ CombineScalars load_combine_scalars(const DevScalars *S) {
+    return CombineScalars{S->tau,      S->step,   S->a,         S->bk_ratio,     S->iter,           S->stage, S->max_iter,
+                          S->step_cap, S->status, S->step_rule, S->lambda0_mode, S->target_overflow};
+}
+
 // stop_condition after a step (Optimization/nesterov.hpp:86-122): `it` steps
 // taken in this stage, tau of the last gradient evaluation.
-__device__ int stop_after_step(const DevScalars *S, double tau, int it) {
+__device__ __forceinline__ int stop_after_step(const CombineScalars &c, int status, int it) {
     int stop;
-    if (S->stage == EP_STAGE_MGP)
-        stop = tau < (double)S->target_overflow || it > S->max_iter;
-    else if (S->stage == EP_STAGE_FILLERONLY)
+    if (c.stage == EP_STAGE_MGP)
+        stop = c.tau < (double)c.target_overflow || it > c.max_iter;
+    else if (c.stage == EP_STAGE_FILLERONLY)
         stop = it >= 20;
     else
-        stop = tau < (double)0.07f || it > S->max_iter;
-    if (S->step_cap > 0 && it >= S->step_cap) stop = 1;
-    if (S->status) stop = 1;
+        stop = c.tau < (double)0.07f || it > c.max_iter;
+    if (c.step_cap > 0 && it >= c.step_cap) stop = 1;
+    if (status) stop = 1;
     return stop;
+}
+
+// acc: dg2, dy2, s.y, |gwl|, |gd|
+__device__ __forceinline__ void finish_combine(DevScalars *S, const CombineScalars &c, const double (&acc)[5],
+                                               int stepping) {
+    const double dg2 = acc[0], dy2 = acc[1], sy = acc[2];
+    int status = c.status;
+    if (c.lambda0_mode) {
+        // penaltyFactorInitilization (EPlace/eplace.cpp:812-835)
+        const double lambda = acc[3] / acc[4];
+        S->lambda = lambda;
+        S->lambda0_mode = 0;
+        if (!isfinite(lambda)) status |= 1 << EP_ERR_NAN;
+    }
+    if (stepping == 2) {
+        // backtracking trial (opt_step_bktrk, Optimization/nesterov.hpp:351-364):
+        // 1/L between the trial point and y_k; accepted when it is at
+        // least BKTRK_EPS (0.95, nesterov.hpp:37; ep_limits) of the step tried
+        double ns = sqrt(dy2) / sqrt(dg2);
+        if (!isfinite(ns)) {
+            status |= 1 << EP_ERR_NAN;
+            ns = 0.0;
+        }
+        S->bk_accept = c.bk_ratio * c.step <= ns;
+        S->step = ns;
+        S->stop_pending = stop_after_step(c, status, c.iter + 1);
+    } else if (stepping) {
+        double step = 1.0;
+        if (c.iter > 0) {
+            const double lip = sqrt(dy2) / sqrt(dg2);  // 1/L
+            S->lip_step = lip;
+            step = lip;
+            if (c.step_rule == EP_STEP_BB) {
+                // BB short step s.y / y.y, else min(|s|/|y|, 1/L), which are the
+                // same number (nesterov.hpp:262-274)
+                const double bb = sy / dg2;
+                step = bb > 0.0 ? bb : lip;
+            }
+        }
+        if (!isfinite(step)) {
+            status |= 1 << EP_ERR_NAN;
+            step = 0.0;
+        }
+        const double an = (1.0 + sqrt(4.0 * c.a * c.a + 1.0)) / 2.0;
+        S->step = step;
+        S->coef = (c.a - 1.0) / an;
+        S->a = an;
+        S->stop_pending = stop_after_step(c, status, c.iter + 1);
+    }
+    if (status != c.status) S->status = status;
 }
 
 // What the combine reads of an object that no kernel writes.
@@ -1048,61 +1124,22 @@ k_combine(Grid g, DeviceNetlist d, const vec2<R> *__restrict__ field, const vec2
         }
     } while (!big && __shfl_sync(kFull, next.o, 0) < d.n_obj);
     // only the sums that this call reads: the step's three, or lambda_0's two
-    bool last = false;
-    if (stepping && !S->lambda0_mode) {
+    const bool lambda0 = S->lambda0_mode;
+    CombineScalars c;
+    if (stepping && !lambda0) {
         double a3[3] = {acc[0], acc[1], acc[2]};
-        last = grid_sum<3>(a3, sh, partials, &S->cnt_comb, gridDim.x, blockIdx.x);
+        if (!grid_arrive<3>(a3, sh, partials, &S->cnt_comb, gridDim.x, blockIdx.x)) return;
+        c = load_combine_scalars(S);
+        grid_total<3>(a3, sh, partials, &S->cnt_comb, gridDim.x);
         for (int k = 0; k < 3; k++) acc[k] = a3[k];
-    } else if (stepping || S->lambda0_mode) {
-        last = grid_sum<5>(acc, sh, partials, &S->cnt_comb, gridDim.x, blockIdx.x);
+    } else if (stepping || lambda0) {
+        if (!grid_arrive<5>(acc, sh, partials, &S->cnt_comb, gridDim.x, blockIdx.x)) return;
+        c = load_combine_scalars(S);
+        grid_total<5>(acc, sh, partials, &S->cnt_comb, gridDim.x);
+    } else {
+        return;
     }
-    if (last && threadIdx.x == 0) {
-        {
-            double dg2 = acc[0], dy2 = acc[1], sy = acc[2];
-            double l1w = acc[3], l1d = acc[4];
-            if (S->lambda0_mode) {
-                // penaltyFactorInitilization (EPlace/eplace.cpp:812-835)
-                S->lambda = l1w / l1d;
-                S->lambda0_mode = 0;
-                if (!isfinite(S->lambda)) S->status |= 1 << EP_ERR_NAN;
-            }
-            if (stepping == 2) {
-                // backtracking trial (opt_step_bktrk, Optimization/nesterov.hpp:351-364):
-                // 1/L between the trial point and y_k; accepted when it is at
-                // least BKTRK_EPS (0.95, nesterov.hpp:37; ep_limits) of the step tried
-                double ns = sqrt(dy2) / sqrt(dg2);
-                if (!isfinite(ns)) {
-                    S->status |= 1 << EP_ERR_NAN;
-                    ns = 0.0;
-                }
-                S->bk_accept = S->bk_ratio * S->step <= ns;
-                S->step = ns;
-                S->stop_pending = stop_after_step(S, S->tau, S->iter + 1);
-            } else if (stepping) {
-                double step = 1.0;
-                if (S->iter > 0) {
-                    double lip = sqrt(dy2) / sqrt(dg2);  // 1/L
-                    S->lip_step = lip;
-                    step = lip;
-                    if (S->step_rule == EP_STEP_BB) {
-                        // BB short step s.y / y.y, else min(|s|/|y|, 1/L) (nesterov.hpp:262-274)
-                        double bb = sy / dg2;
-                        step = bb > 0.0 ? bb : fmin(sqrt(dy2) / sqrt(dg2), lip);
-                    }
-                }
-                if (!isfinite(step)) {
-                    S->status |= 1 << EP_ERR_NAN;
-                    step = 0.0;
-                }
-                double a = S->a;
-                double an = (1.0 + sqrt(4.0 * a * a + 1.0)) / 2.0;
-                S->step = step;
-                S->coef = (a - 1.0) / an;
-                S->a = an;
-                S->stop_pending = stop_after_step(S, S->tau, S->iter + 1);
-            }
-        }
-    }
+    if (threadIdx.x == 0) finish_combine(S, c, acc, stepping);
 }
 
 // ---------------------------------------------------------------- update --

@@ -37,10 +37,14 @@ constexpr int kQT = 256;
 constexpr float kMinDistance = 25.0f;  // MIN_DISTANCE, QPlace/qplace.h
 
 inline int qblocks(int n) { return (n + kQT - 1) / kQT; }
-// Kernels that end in a grid reduction run on at most 8 blocks per SM and
-// loop over their rows, so the finalising block adds few partials; the grid
-// depends only on the sizes, so the sums are the same on every run.
+// The bounds pass runs on at most 8 blocks per SM and loops over its nets, so the
+// finalising block adds few partials; the grid depends only on the sizes, so
+// the sum is the same on every run.
 constexpr int kQpMaxBlocks = 148 * 8;
+// The solver's kernels: at most what the SMs hold at once.  The SpMV's need 80
+// registers for that; with the 90 it would take, half of the blocks wait for a
+// second wave (24 against 17 us).
+constexpr int kSolveBlocks = 148 * 3;
 inline int qgrid(int n) { return std::min(qblocks(n), kQpMaxBlocks); }
 
 __device__ __forceinline__ float2 abs_pin(const float2 *__restrict__ pos, const float2 *__restrict__ off,
@@ -118,7 +122,9 @@ k_qp_bounds(int nnet, int n_big, const int32_t *__restrict__ order, const int32_
         bound[n] = b;
         if (d > 0) acc[0] += (mxx - mnx) + (mxy - mny);
     }
-    if (grid_sum<1>(acc, sh, partials, cnt, gridDim.x, blockIdx.x) && threadIdx.x == 0) *hpwl = acc[0];
+    if (!grid_arrive<1>(acc, sh, partials, cnt, gridDim.x, blockIdx.x)) return;
+    grid_total<1>(acc, sh, partials, cnt, gridDim.x);
+    if (threadIdx.x == 0) *hpwl = acc[0];
 }
 
 // Partners of pin a (index in its net of d pins) in the X model: every pin
@@ -214,97 +220,170 @@ __device__ __forceinline__ bool is_long(const PartnerRange &r) {
     return r.end - (r.skip >= 0) + (r.extra >= 0) > kLongPartners;
 }
 
-// ---- CSR row offsets on the device ------------------------------------------
-// The counts of both systems lie in one array c[0 .. 2 nn) (X rows, then Y
-// rows); with E the exclusive prefix sum of c over [0, 2 nn], row_x[i] =
-// E[i] (i <= nn) and row_y[i] = E[nn + i] - E[nn].  Three passes over
-// chunks of kScanChunk entries: chunk totals; one block scanning the totals
-// (and finding E[nn], E[2 nn]); each chunk's prefix sums.  Integer sums:
-// the same offsets the host loop gave.
-constexpr int kScanItems = 4, kScanChunk = kQT * kScanItems;
+// ---- matrix layout --------------------------------------------------------------
+// Entries (column, value) of one axis lie in one array.  The rows of at most
+// kLongRow entries on both axes go by slices of 32 rows (a warp): entry k of
+// the slice's row l is at base + 32 k + l, so a thread per row reads them with
+// one coalesced load per k.  A slice is as long as its longest row, so the rows
+// of each window of kQT rows (a block) are sorted by length first; the window
+// is small, so that a slice's rows still lie near one another in the vectors.
+// The longer rows (the bound pins of large nets) follow all slices, their
+// entries contiguous, and are listed in `longs`, so that warps of their own take
+// them first.  The count pass sorts its
+// window and leaves the rows' places in it; one block scans the windows.
+constexpr int kLongRow = 32;
+constexpr int kSlices = kQT / 32;  // of a window
 
-__device__ __forceinline__ int block_excl_scan(int v, int &total) {
-    __shared__ int warp_tot[kQT / 32];
+struct __align__(16) Window {  // totals of a window, then its first places
+    int x, y;                  // entries of its slices (32 x the longest row of each)
+    int n_long, long_x, long_y, pad[3];
+};
+
+struct QpLayout {
+    Window *win;
+    int2 *slice;  // a slice's first X and Y entry, from its window's
+    int2 *slot;   // the slices' rows: (row, X entries | Y entries << 8), row -1: none
+    int2 *rel;    // a row's first X and Y entry, from its window's
+    int4 *longs;  // two per long row: (row, first X entry, first Y entry, X entries), (Y entries, 0, 0, 0)
+};
+
+constexpr int kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads)
+k_qp_scan(int nw, Window *__restrict__ t, int cap_x, int cap_y, QpSolve *__restrict__ S) {
+    __shared__ int warp_tot[5][kScanThreads / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int x = v;
+    // a contiguous run of windows per thread
+    const int per = (nw + kScanThreads - 1) / kScanThreads, s0 = min(nw, (int)threadIdx.x * per), s1 = min(nw, s0 + per);
+    int v[5] = {0, 0, 0, 0, 0};
+    for (int k = s0; k < s1; k++) {
+        const Window c = t[k];
+        v[0] += c.x;
+        v[1] += c.y;
+        v[2] += c.n_long;
+        v[3] += c.long_x;
+        v[4] += c.long_y;
+    }
+    int run[5], total[5];
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+        int x = v[q];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_tot[q][w] = x;
+        run[q] = x - v[q];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+        total[q] = 0;
+        for (int k = 0; k < kScanThreads / 32; k++) {
+            if (k < w) run[q] += warp_tot[q][k];
+            total[q] += warp_tot[q][k];
+        }
+    }
+    for (int k = s0; k < s1; k++) {
+        const Window c = t[k];
+        t[k] = Window{run[0], run[1], run[2], total[0] + run[3], total[1] + run[4], {0, 0, 0}};
+        run[0] += c.x;
+        run[1] += c.y;
+        run[2] += c.n_long;
+        run[3] += c.long_x;
+        run[4] += c.long_y;
+    }
+    if (threadIdx.x == 0) {
+        S->n_long = total[2];
+        S->overflow = total[0] + total[3] > cap_x || total[1] + total[4] > cap_y;
+    }
+}
+
+// Sort the block's rows by their length (stable, the long rows last) and leave
+// their places: a counting sort over the keys 0 .. kLongRow + 1.  Every thread
+// of the block calls it; lx, ly: its row's entries (rows past the last: 0, 0,
+// which take slots of no row).
+__device__ __forceinline__ void place_window(int i, int nn, int lx, int ly, const QpLayout &q) {
+    constexpr int kKeys = kLongRow + 2;
+    __shared__ int warp_key[kSlices][kKeys], first[kKeys];
+    __shared__ int slice_len[2][kSlices], long_n, long_x, long_y;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const bool lg = max(lx, ly) > kLongRow;
+    const int key = lg ? kKeys - 1 : max(lx, ly);
+    for (int k = tid; k < kSlices * kKeys; k += kQT) (&warp_key[0][0])[k] = 0;
+    if (tid < kSlices) slice_len[0][tid] = slice_len[1][tid] = 0;
+    __syncthreads();
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const int rank = __popc(peers & ((1u << lane) - 1));
+    if (rank == 0) warp_key[w][key] = __popc(peers);
+    __syncthreads();
+    if (tid < kKeys) {  // rows of this key in the warps before each warp
+        int n = 0;
+        for (int k = 0; k < kSlices; k++) {
+            const int c = warp_key[k][tid];
+            warp_key[k][tid] = n;
+            n += c;
+        }
+        first[tid] = n;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int n = 0;
+        for (int k = 0; k < kKeys; k++) {
+            const int c = first[k];
+            first[k] = n;
+            n += c;
+        }
+        // the long rows' entries one after another, in row order
+        long_n = long_x = long_y = 0;
+    }
+    __syncthreads();
+    const int at = first[key] + warp_key[w][key] + rank, sl = at >> 5;
+    if (!lg) {
+        atomicMax(&slice_len[0][sl], lx);
+        atomicMax(&slice_len[1][sl], ly);
+    }
+    // exclusive sums over the long rows of the block, warp by warp
+    int px = lg ? lx : 0, py = lg ? ly : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[w] = x;
-    __syncthreads();
-    int before = 0;
-    total = 0;
-    for (int k = 0; k < kQT / 32; k++) {
-        if (k < w) before += warp_tot[k];
-        total += warp_tot[k];
-    }
-    __syncthreads();
-    return before + x - v;
-}
-
-__global__ void __launch_bounds__(kQT) k_qp_chunk_sums(const int32_t *__restrict__ c, int n2, int32_t *__restrict__ sums) {
-    const int base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
-    int v = 0;
-#pragma unroll
-    for (int u = 0; u < kScanItems; u++) v += base + u < n2 ? c[base + u] : 0;
-    int total;
-    block_excl_scan(v, total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-// one block: exclusive scan of the chunk totals in place, then E[nn] and
-// E[2 nn] into sums[nb], sums[nb + 1], and the overflow flag
-__global__ void __launch_bounds__(kQT) k_qp_chunk_scan(int32_t *__restrict__ sums, int nb, const int32_t *__restrict__ c,
-                                                      int nn, int cap_x, int cap_y, QpSolve *__restrict__ S) {
-    __shared__ int carry_s;
-    int carry = 0;
-    for (int t0 = 0; t0 < nb; t0 += kQT) {
-        const int i = t0 + threadIdx.x;
-        const int v = i < nb ? sums[i] : 0;
-        int total;
-        const int ex = block_excl_scan(v, total);
-        if (i < nb) sums[i] = carry + ex;
-        carry += total;
-    }
-    // E[nn]: the scanned total of nn's chunk plus that chunk's entries before nn
-    const int ch = nn / kScanChunk;
-    int part = 0;
-    for (int k = ch * kScanChunk + threadIdx.x; k < nn; k += kQT) part += c[k];
-    int total;
-    block_excl_scan(part, total);
-    if (threadIdx.x == 0) carry_s = carry;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int enn = sums[ch] + total;
-        sums[nb] = enn;
-        sums[nb + 1] = carry_s;
-        S->overflow = enn > cap_x || carry_s - enn > cap_y;
-    }
-}
-
-__global__ void __launch_bounds__(kQT) k_qp_offsets(const int32_t *__restrict__ c, int nn, const int32_t *__restrict__ sums,
-                                                   int nb, int32_t *__restrict__ row_x, int32_t *__restrict__ row_y) {
-    const int n2 = 2 * nn, base = blockIdx.x * kScanChunk + threadIdx.x * kScanItems;
-    int v[kScanItems], s = 0;
-#pragma unroll
-    for (int u = 0; u < kScanItems; u++) {
-        v[u] = base + u < n2 ? c[base + u] : 0;
-        s += v[u];
-    }
-    int total;
-    int e = sums[blockIdx.x] + block_excl_scan(s, total);
-    const int enn = sums[nb];
-#pragma unroll
-    for (int u = 0; u < kScanItems; u++) {
-        const int i = base + u;  // E[i] = e
-        if (i <= n2) {
-            if (i <= nn) row_x[i] = e;
-            if (i >= nn) row_y[i - nn] = e - enn;
+        const int a = __shfl_up_sync(0xffffffffu, px, o), b = __shfl_up_sync(0xffffffffu, py, o);
+        if (lane >= o) {
+            px += a;
+            py += b;
         }
-        e += v[u];
     }
+    const int nlong = __popc(__ballot_sync(0xffffffffu, lg));
+    int bx = 0, by = 0;
+    for (int k = 0; k < kSlices; k++) {
+        __syncthreads();
+        if (k == w) {
+            bx = long_x;
+            by = long_y;
+        }
+        __syncthreads();
+        if (k == w && lane == 31) {
+            long_x += px;
+            long_y += py;
+            long_n += nlong;
+        }
+    }
+    __syncthreads();
+    int ox = 0, oy = 0, tx = 0, ty = 0;
+    for (int k = 0; k < kSlices; k++) {
+        if (k == sl) {
+            ox = tx;
+            oy = ty;
+        }
+        tx += 32 * slice_len[0][k];
+        ty += 32 * slice_len[1][k];
+    }
+    const size_t slot0 = (size_t)blockIdx.x * kQT;
+    q.slot[slot0 + at] = make_int2(i < nn && !lg ? i : -1, lg ? 0 : lx | (ly << 8));
+    if ((at & 31) == 0) q.slice[blockIdx.x * kSlices + sl] = make_int2(ox, oy);
+    if (i < nn)
+        q.rel[i] = lg ? make_int2(bx + px - lx, by + py - ly) : make_int2(ox + (at & 31), oy + (at & 31));
+    if (tid == 0) q.win[blockIdx.x] = Window{tx, ty, long_n, long_x, long_y, {0, 0, 0}};
 }
 
 // One movable node's row of both systems: counts (FILL = false: the
@@ -319,9 +398,8 @@ __global__ void __launch_bounds__(kQT)
 k_qp_rows(int nn, const int32_t *__restrict__ obj_pin_start, const int32_t *__restrict__ obj_pin_dev,
           const int32_t *__restrict__ pin_net, const int32_t *__restrict__ first, const int32_t *__restrict__ deg,
           const int4 *__restrict__ bound, const int32_t *__restrict__ owner, const float2 *__restrict__ off,
-          const float2 *__restrict__ abspin, int32_t *__restrict__ count, const int32_t *__restrict__ row_x,
-          const int32_t *__restrict__ row_y, int32_t *__restrict__ col_x, float *__restrict__ val_x,
-          int32_t *__restrict__ col_y, float *__restrict__ val_y, float2 *__restrict__ diag,
+          const float2 *__restrict__ abspin, int32_t *__restrict__ count, QpLayout lay,
+          int2 *__restrict__ ent_x, int2 *__restrict__ ent_y, float2 *__restrict__ diag,
           float2 *__restrict__ rhs, const QpSolve *__restrict__ S) {
     constexpr bool fill = FILL;
     if (fill && S->overflow) return;  // uniform: the offsets exceed the allocation, the solve reports it
@@ -329,15 +407,30 @@ k_qp_rows(int nn, const int32_t *__restrict__ obj_pin_start, const int32_t *__re
     const bool valid = i < nn;  // every lane stays for the warp's long sets
     int cnt[2] = {0, 0};
     double dsum[2] = {0.0, 0.0}, bsum[2] = {0.0, 0.0};
-    const int row0[2] = {fill && valid ? row_x[i] : 0, fill && valid ? row_y[i] : 0};
-    int32_t *const col[2] = {col_x, col_y};
-    float *const val[2] = {val_x, val_y};
+    int row0[2] = {0, 0}, step = 1;
+    if (fill) {
+        const Window w = lay.win[blockIdx.x];
+        const bool lg = valid && max(count[i], count[nn + i]) > kLongRow;
+        const int2 rel = valid ? lay.rel[i] : make_int2(0, 0);
+        row0[0] = (lg ? w.long_x : w.x) + rel.x;
+        row0[1] = (lg ? w.long_y : w.y) + rel.y;
+        step = lg ? 1 : 32;
+        // the window's long rows in row order
+        __shared__ int warp_long[kSlices];
+        const unsigned m = __ballot_sync(0xffffffffu, lg);
+        if (lane == 0) warp_long[threadIdx.x >> 5] = __popc(m);
+        __syncthreads();
+        if (lg) {
+            int at = w.n_long + __popc(m & ((1u << lane) - 1));
+            for (int k = 0; k < (int)(threadIdx.x >> 5); k++) at += warp_long[k];
+            lay.longs[2 * at] = make_int4(i, row0[0], row0[1], count[i]);
+            lay.longs[2 * at + 1] = make_int4(count[nn + i], 0, 0, 0);
+        }
+    }
+    int2 *const ent[2] = {ent_x, ent_y};
     const int k0 = valid ? obj_pin_start[i] : 0, np_i = valid ? obj_pin_start[i + 1] - k0 : 0;
     auto entry = [&](int axis, int j, float w, int at) {
-        if (fill) {
-            col[axis][row0[axis] + at] = j;
-            val[axis][row0[axis] + at] = -w;
-        }
+        if (fill) ent[axis][row0[axis] + at * step] = make_int2(j, __float_as_int(-w));
     };
     for (int k = k0; k < k0 + np_i; k++) {
         const int q = obj_pin_dev[k], n = pin_net[q], f = first[n], d = deg[n], a = q - f;
@@ -396,7 +489,8 @@ k_qp_rows(int nn, const int32_t *__restrict__ obj_pin_start, const int32_t *__re
                 const float c = (float)(1.0 / ((double)sd - 1.0));
                 const float2 pa2 = abspin[sq], oa2 = off[sq];
                 const float pa = axis ? pa2.y : pa2.x, oa = axis ? oa2.y : oa2.x;
-                const int row = fill ? (axis ? row_y[si] : row_x[si]) : 0;
+                const int row = __shfl_sync(0xffffffffu, row0[axis], src);
+                const int rstep = __shfl_sync(0xffffffffu, step, src);
                 double ds = 0.0, bs = 0.0;
                 int added = 0;
                 for (int base = 0; base < end; base += 32) {
@@ -407,11 +501,9 @@ k_qp_rows(int nn, const int32_t *__restrict__ obj_pin_start, const int32_t *__re
                         j = FILL ? pair_terms(si, nn, sf + b, axis, owner, abspin, off, c, pa, oa, w, ds, bs)
                                  : pair_partner(si, nn, sf + b, owner);
                     const unsigned m = __ballot_sync(0xffffffffu, j >= 0);
-                    if (fill && j >= 0) {
-                        const int at = row + at0 + added + __popc(m & ((1u << lane) - 1));
-                        col[axis][at] = j;
-                        val[axis][at] = -w;
-                    }
+                    if (fill && j >= 0)
+                        ent[axis][row + (at0 + added + __popc(m & ((1u << lane) - 1))) * rstep] =
+                            make_int2(j, __float_as_int(-w));
                     added += __popc(m);
                 }
                 if (extra >= 0) {
@@ -420,10 +512,7 @@ k_qp_rows(int nn, const int32_t *__restrict__ obj_pin_start, const int32_t *__re
                     if (lane == 0)
                         j = FILL ? pair_terms(si, nn, sf + extra, axis, owner, abspin, off, c, pa, oa, w, ds, bs)
                                  : pair_partner(si, nn, sf + extra, owner);
-                    if (fill && j >= 0) {
-                        col[axis][row + at0 + added] = j;
-                        val[axis][row + at0 + added] = -w;
-                    }
+                    if (fill && j >= 0) ent[axis][row + (at0 + added) * rstep] = make_int2(j, __float_as_int(-w));
                     added += __shfl_sync(0xffffffffu, j >= 0 ? 1 : 0, 0);
                 }
 #pragma unroll
@@ -439,6 +528,7 @@ k_qp_rows(int nn, const int32_t *__restrict__ obj_pin_start, const int32_t *__re
             }
         }
     }
+    if (!fill) place_window(i, nn, cnt[0], cnt[1], lay);
     if (!valid) return;
     if (!fill) {
         count[i] = cnt[0];
@@ -450,83 +540,94 @@ k_qp_rows(int nn, const int32_t *__restrict__ obj_pin_start, const int32_t *__re
 }
 
 struct QpMat {
-    const int32_t *row_x, *col_x, *row_y, *col_y;
-    const float *val_x, *val_y;
+    const int2 *ent_x, *ent_y;
+    QpLayout lay;
+    const int32_t *count;  // [2 nn] entries of each row
     const float2 *diag;
+    int nn;
 };
 
-// (A_x v.x, A_y v.y) for row i.  A row takes the kRowLanes lanes of an
-// aligned lane group (lane sub of the group sums entries sub, sub + 8, ...
-// of both axes in order, a fixed xor tree adds the 8 partial sums); a row of
-// more than kLongRow entries on either axis (the bound pins of large nets)
-// takes the whole warp after the short rows are done (lane l sums entries
-// l, l + 32, ..., a fixed xor tree over the warp).  The diagonal term comes
-// last.  The split depends only on the row lengths, so the result is the
-// same on every run.  Every lane of the warp must call it (valid = false
-// for lanes past the last row); every lane of the row's group gets the
-// result.
-constexpr int kRowLanes = 8, kRowsPerWarp = 32 / kRowLanes, kLongRow = 4 * kRowLanes;
-
-__device__ __forceinline__ void row_partial(const QpMat &m, const float2 *__restrict__ v, int bx, int lx, int by,
-                                            int ly, int lane, int step, float &ax, float &ay) {
-    const int len = max(lx, ly);
-#pragma unroll 2
-    for (int k = lane; k < len; k += step) {
-        if (k < lx) ax = fmaf(m.val_x[bx + k], v[m.col_x[bx + k]].x, ax);
-        if (k < ly) ay = fmaf(m.val_y[by + k], v[m.col_y[by + k]].y, ay);
-    }
+// The partial sums of a row of eight lanes, in its tree's order.
+__device__ __forceinline__ float tree8(const float (&a)[8]) {
+    return ((a[0] + a[4]) + (a[2] + a[6])) + ((a[1] + a[5]) + (a[3] + a[7]));
 }
 
-__device__ __forceinline__ float2 spmv_row8(const QpMat &m, const float2 *__restrict__ v, int i, int sub, bool valid) {
-    const int lane = threadIdx.x & 31;
-    int bx = 0, lx = 0, by = 0, ly = 0;
-    if (valid) {
-        bx = m.row_x[i];
-        lx = m.row_x[i + 1] - bx;
-        by = m.row_y[i];
-        ly = m.row_y[i + 1] - by;
-    }
-    const bool is_long = max(lx, ly) > kLongRow;
-    float ax = 0.f, ay = 0.f;
-    if (!is_long) row_partial(m, v, bx, lx, by, ly, sub, kRowLanes, ax, ay);
+// (A_x v.x, A_y v.y) of every row i, and emit(i, result, pre), pre = before(i)
+// loaded ahead of the row: a thread per row of a slice, a warp per long row
+// (emit on its first lane).  The sums keep one order per row: eight partial
+// sums over the entries k, k + 8, ... in order, added by a tree (a long row: 32,
+// and a tree over the lanes), the diagonal last.  Bound by the latency of
+// entry -> vector element: a thread has eight of each on either axis in flight
+// where a lane of eight per row had one.  Three blocks an SM: 444 blocks sum
+// fewer partials than 1184.  200k rows, 1.9M entries an axis, warm, us: SpMV
+// 27 -> 17, an iteration (five kernels) 80 -> 47.
+template <class Before, class Emit>
+__device__ __forceinline__ void spmv_rows(const QpMat &m, const float2 *__restrict__ v, const QpSolve *__restrict__ S,
+                                          Before &&before, Emit &&emit) {
+    const int lane = threadIdx.x & 31, nn = m.nn;
+    const int windows = (nn + kQT - 1) / kQT;
+    const int n_long = S->n_long, units = S->overflow ? 0 : n_long + windows * kSlices;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < units; u += warps) {  // warp-uniform
+        if (u < n_long) {
+            const int4 r = m.lay.longs[2 * u];
+            const int lx = r.w, ly = m.lay.longs[2 * u + 1].x, len = max(lx, ly);
+            float2 pre, d, vi;
+            if (lane == 0) {
+                pre = before(r.x);
+                d = m.diag[r.x];
+                vi = v[r.x];
+            }
+            float ax = 0.f, ay = 0.f;
+#pragma unroll 4
+            for (int k = lane; k < len; k += 32) {
+                if (k < lx) {
+                    const int2 e = m.ent_x[r.y + k];
+                    ax = fmaf(__int_as_float(e.y), v[e.x].x, ax);
+                }
+                if (k < ly) {
+                    const int2 e = m.ent_y[r.z + k];
+                    ay = fmaf(__int_as_float(e.y), v[e.x].y, ay);
+                }
+            }
 #pragma unroll
-    for (int o = kRowLanes / 2; o > 0; o >>= 1) {
-        ax += __shfl_xor_sync(0xffffffffu, ax, o);
-        ay += __shfl_xor_sync(0xffffffffu, ay, o);
-    }
-    unsigned longs = __ballot_sync(0xffffffffu, is_long && sub == 0);
-    while (longs) {  // warp-uniform
-        const int src = __ffs(longs) - 1;
-        longs &= longs - 1;
-        const int lbx = __shfl_sync(0xffffffffu, bx, src), llx = __shfl_sync(0xffffffffu, lx, src);
-        const int lby = __shfl_sync(0xffffffffu, by, src), lly = __shfl_sync(0xffffffffu, ly, src);
-        float sx = 0.f, sy = 0.f;
-        row_partial(m, v, lbx, llx, lby, lly, lane, 32, sx, sy);
+            for (int o = 16; o > 0; o >>= 1) {
+                ax += __shfl_xor_sync(0xffffffffu, ax, o);
+                ay += __shfl_xor_sync(0xffffffffu, ay, o);
+            }
+            if (lane == 0) emit(r.x, make_float2(fmaf(d.x, vi.x, ax), fmaf(d.y, vi.y, ay)), pre);
+            continue;
+        }
+        // the longest slices of all windows first, so that a block's warps have
+        // slices of about one length
+        const int q = u - n_long, slice = q % windows * kSlices + kSlices - 1 - q / windows;
+        const int2 slot = m.lay.slot[(size_t)slice * 32 + lane], rel = m.lay.slice[slice];
+        const int2 first = *reinterpret_cast<const int2 *>(m.lay.win + slice / kSlices);  // x, y
+        const int i = slot.x, lx = slot.y & 255, ly = slot.y >> 8;
+        const bool mine = i >= 0;
+        const int len = __reduce_max_sync(0xffffffffu, max(lx, ly));
+        const float2 zero = make_float2(0.f, 0.f);
+        const float2 pre = mine ? before(i) : zero, d = mine ? m.diag[i] : zero, vi = mine ? v[i] : zero;
+        const int2 *ex = m.ent_x + first.x + rel.x + lane, *ey = m.ent_y + first.y + rel.y + lane;
+        float sx[8], sy[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            sx += __shfl_xor_sync(0xffffffffu, sx, o);
-            sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        for (int k = 0; k < 8; k++) sx[k] = sy[k] = 0.f;
+        for (int k0 = 0; k0 < len; k0 += 8) {
+            int2 a[8], b[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                a[k] = k0 + k < lx ? ex[(k0 + k) * 32] : make_int2(-1, 0);
+                b[k] = k0 + k < ly ? ey[(k0 + k) * 32] : make_int2(-1, 0);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                if (a[k].x >= 0) sx[k] = fmaf(__int_as_float(a[k].y), v[a[k].x].x, sx[k]);
+                if (b[k].x >= 0) sy[k] = fmaf(__int_as_float(b[k].y), v[b[k].x].y, sy[k]);
+            }
         }
-        if (lane / kRowLanes == src / kRowLanes) {
-            ax = sx;
-            ay = sy;
-        }
+        if (mine) emit(i, make_float2(fmaf(d.x, vi.x, tree8(sx)), fmaf(d.y, vi.y, tree8(sy))), pre);
     }
-    if (valid) {
-        const float2 d = m.diag[i], vi = v[i];
-        ax = fmaf(d.x, vi.x, ax);
-        ay = fmaf(d.y, vi.y, ay);
-    }
-    return make_float2(ax, ay);
 }
-
-__device__ __forceinline__ int row_group_first() {
-    return ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kRowsPerWarp;
-}
-__device__ __forceinline__ int row_group_stride() { return ((gridDim.x * blockDim.x) >> 5) * kRowsPerWarp; }
-#define ROW_GROUPS(nn)                                                                                        \
-    for (int base_ = row_group_first(), sub = threadIdx.x % kRowLanes, i = base_ + (threadIdx.x & 31) / kRowLanes; \
-         base_ < (nn); base_ += row_group_stride(), i = base_ + (threadIdx.x & 31) / kRowLanes)
 
 // ---- BiCGSTAB on the device -----------------------------------------------------
 // Eigen's BiCGSTAB (van der Vorst's method, restart when r0.r vanishes,
@@ -536,8 +637,9 @@ __device__ __forceinline__ int row_group_stride() { return ((gridDim.x * blockDi
 // alpha, beta and omega from there.  Per axis c:
 //   head     rho_old = rho; rho = r0.r; restart when |rho| < eps^2 r0sq
 //            (in the finaliser of the previous step, or of the set-up)
-//   restart  (only when flagged) r = b - A x, r0 = r; rho = r0sq = |r|^2,
-//            the iteration count reset at the first restart
+//   restart  (only when flagged, launched by the host when it sees the flag)
+//            r = b - A x, r0 = r; rho = r0sq = |r|^2, the iteration count reset
+//            at the first restart
 //   dir      p = r + beta (p - omega v), beta = (rho / rho_old)(alpha / omega)
 //   av       v = A p; alpha = rho / (r0.v)
 //   s        s = r - alpha v
@@ -548,11 +650,14 @@ __device__ __forceinline__ int row_group_stride() { return ((gridDim.x * blockDi
 // An inactive axis uses alpha = beta = omega = 0 (its x and r stay), and
 // every kernel returns at once when neither axis is active, so iterations
 // can be enqueued ahead of the convergence test.
+// Neither axis stopped, and no restart owed: the kernels of the iterations
+// already enqueued wait (return at once) until the host has launched it.
 __device__ __forceinline__ bool any_active(const QpSolve *S) { return S->active[0] || S->active[1]; }
+__device__ __forceinline__ bool running(const QpSolve *S) { return any_active(S) && !S->restart_mask; }
 
 // The head of an iteration (rho_old = rho; rho = r0.r; the restart test),
 // run by the finaliser that ends the previous iteration (or the set-up).
-__device__ void qp_pre(QpSolve *S) {
+__device__ __forceinline__ void qp_pre(QpSolve *S) {
     if (!any_active(S)) return;
     const double eps = 1.1920928955078125e-07, eps2 = eps * eps;
     int restart = 0;
@@ -567,28 +672,27 @@ __device__ void qp_pre(QpSolve *S) {
 
 // r = b - A x, r0 = r, p = v = 0; |r|^2 and |b|^2 per system, then the
 // solver's initial state.
-__global__ void __launch_bounds__(kQT)
+__global__ void __launch_bounds__(kQT, kSolveBlocks / 148)
 k_qp_init(int nn, QpMat m, const float2 *__restrict__ rhs, const float2 *__restrict__ x, float2 *__restrict__ r,
           float2 *__restrict__ r0, float2 *__restrict__ p, float2 *__restrict__ v, double *__restrict__ partials,
-          unsigned *__restrict__ cnt, int max_it, QpSolve *__restrict__ S) {
+          unsigned *__restrict__ cnt, int max_it, QpSolve *__restrict__ G) {
     __shared__ double sh[4 * 32];
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    ROW_GROUPS(nn) {
-        const float2 ax = spmv_row8(m, x, i, sub, i < nn);
-        if (i < nn && sub == 0) {
-            const float2 bi = rhs[i];
-            const float2 ri = make_float2(bi.x - ax.x, bi.y - ax.y);
-            r[i] = ri;
-            r0[i] = ri;
-            p[i] = make_float2(0.f, 0.f);
-            v[i] = make_float2(0.f, 0.f);
-            acc[0] += (double)ri.x * ri.x;
-            acc[1] += (double)ri.y * ri.y;
-            acc[2] += (double)bi.x * bi.x;
-            acc[3] += (double)bi.y * bi.y;
-        }
-    }
-    if (grid_sum<4>(acc, sh, partials, cnt, gridDim.x, blockIdx.x) && threadIdx.x == 0) {
+    spmv_rows(m, x, G, [&](int i) { return rhs[i]; }, [&](int i, float2 ax, float2 bi) {
+        const float2 ri = make_float2(bi.x - ax.x, bi.y - ax.y);
+        r[i] = ri;
+        r0[i] = ri;
+        p[i] = make_float2(0.f, 0.f);
+        v[i] = make_float2(0.f, 0.f);
+        acc[0] += (double)ri.x * ri.x;
+        acc[1] += (double)ri.y * ri.y;
+        acc[2] += (double)bi.x * bi.x;
+        acc[3] += (double)bi.y * bi.y;
+    });
+    if (!grid_arrive<4>(acc, sh, partials, cnt, gridDim.x, blockIdx.x)) return;
+    grid_total<4>(acc, sh, partials, cnt, gridDim.x);
+    if (threadIdx.x == 0) {
+        QpSolve s = *G, *S = &s;
         const double eps = 1.1920928955078125e-07, eps2 = eps * eps;
         S->zero_mask = 0;
         S->restart_mask = 0;
@@ -612,6 +716,7 @@ k_qp_init(int nn, QpMat m, const float2 *__restrict__ rhs, const float2 *__restr
         }
         S->max_it = max_it;
         qp_pre(S);
+        *G = s;
     }
 }
 
@@ -626,29 +731,26 @@ __global__ void k_qp_zero(int nn, const QpSolve *__restrict__ S, float2 *__restr
 
 
 // Restart of the flagged systems: r = b - A x, r0 = r; rho = r0sq = |r|^2.
-__global__ void __launch_bounds__(kQT)
+__global__ void __launch_bounds__(kQT, kSolveBlocks / 148)
 k_qp_restart(int nn, QpMat m, const float2 *__restrict__ rhs, const float2 *__restrict__ x, float2 *__restrict__ r,
              float2 *__restrict__ r0, double *__restrict__ partials, unsigned *__restrict__ cnt,
              QpSolve *__restrict__ S) {
     __shared__ double sh[2 * 32];
     pdl_begin();
     const int mask = S->restart_mask;
-    if (!mask || !any_active(S)) return;  // uniform over the grid
     double acc[2] = {0.0, 0.0};
-    ROW_GROUPS(nn) {
-        const float2 ax = spmv_row8(m, x, i, sub, i < nn);
-        if (i < nn && sub == 0) {
-            const float2 bi = rhs[i];
-            float2 ri = r[i], zi = r0[i];
-            if (mask & 1) ri.x = zi.x = bi.x - ax.x;
-            if (mask & 2) ri.y = zi.y = bi.y - ax.y;
-            r[i] = ri;
-            r0[i] = zi;
-            acc[0] += (double)ri.x * ri.x;
-            acc[1] += (double)ri.y * ri.y;
-        }
-    }
-    if (grid_sum<2>(acc, sh, partials, cnt, gridDim.x, blockIdx.x) && threadIdx.x == 0) {
+    spmv_rows(m, x, S, [&](int i) { return rhs[i]; }, [&](int i, float2 ax, float2 bi) {
+        float2 ri = r[i], zi = r0[i];
+        if (mask & 1) ri.x = zi.x = bi.x - ax.x;
+        if (mask & 2) ri.y = zi.y = bi.y - ax.y;
+        r[i] = ri;
+        r0[i] = zi;
+        acc[0] += (double)ri.x * ri.x;
+        acc[1] += (double)ri.y * ri.y;
+    });
+    if (!grid_arrive<2>(acc, sh, partials, cnt, gridDim.x, blockIdx.x)) return;
+    grid_total<2>(acc, sh, partials, cnt, gridDim.x);
+    if (threadIdx.x == 0) {
         for (int c = 0; c < 2; c++)
             if (mask & (1 << c)) {
                 S->rho[c] = S->r0sq[c] = acc[c];
@@ -658,48 +760,53 @@ k_qp_restart(int nn, QpMat m, const float2 *__restrict__ rhs, const float2 *__re
     }
 }
 
+// Rows 2 k and 2 k + 1 of a vector (allocated to an even number of rows).
+__device__ __forceinline__ float4 pair(const float2 *v, int k) { return reinterpret_cast<const float4 *>(v)[k]; }
+__device__ __forceinline__ void set_pair(float2 *v, int k, float4 a) { reinterpret_cast<float4 *>(v)[k] = a; }
+
 // p = r + beta (p - omega v); with a diagonal preconditioner (dinv, else
 // null) also y = M^-1 p, the vector the SpMV then takes
 __global__ void __launch_bounds__(kQT)
 k_qp_dir(int nn, const float2 *__restrict__ r, const float2 *__restrict__ v, float2 *__restrict__ p,
          const float2 *__restrict__ dinv, float2 *__restrict__ y, const QpSolve *__restrict__ S) {
     pdl_begin();
-    if (!any_active(S)) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nn) return;
+    if (!running(S)) return;
     float b[2], w[2];
     for (int c = 0; c < 2; c++) {
         b[c] = S->active[c] ? (float)((S->rho[c] / S->rho_old[c]) * (S->alpha[c] / S->w[c])) : 0.f;
         w[c] = S->active[c] ? (float)S->w[c] : 0.f;
     }
-    const float2 ri = r[i], vi = v[i], pi = p[i];
-    const float2 pn = make_float2(ri.x + b[0] * (pi.x - w[0] * vi.x), ri.y + b[1] * (pi.y - w[1] * vi.y));
-    p[i] = pn;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (nn + 1) / 2) return;
+    const float4 ri = pair(r, t), vi = pair(v, t), pi = pair(p, t);
+    const float4 pn = make_float4(ri.x + b[0] * (pi.x - w[0] * vi.x), ri.y + b[1] * (pi.y - w[1] * vi.y),
+                                  ri.z + b[0] * (pi.z - w[0] * vi.z), ri.w + b[1] * (pi.w - w[1] * vi.w));
+    set_pair(p, t, pn);
     if (dinv) {
-        const float2 d = dinv[i];
-        y[i] = make_float2(pn.x * d.x, pn.y * d.y);
+        const float4 d = pair(dinv, t);
+        set_pair(y, t, make_float4(pn.x * d.x, pn.y * d.y, pn.z * d.z, pn.w * d.w));
     }
 }
 
 // v = A p; alpha = rho / (r0.v)
-__global__ void __launch_bounds__(kQT)
+__global__ void __launch_bounds__(kQT, kSolveBlocks / 148)
 k_qp_av(int nn, QpMat m, const float2 *__restrict__ p, const float2 *__restrict__ r0, float2 *__restrict__ v,
         double *__restrict__ partials, unsigned *__restrict__ cnt, QpSolve *__restrict__ S) {
     __shared__ double sh[2 * 32];
     pdl_begin();
-    if (!any_active(S)) return;
+    if (!running(S)) return;
     double acc[2] = {0.0, 0.0};
-    ROW_GROUPS(nn) {
-        const float2 vi = spmv_row8(m, p, i, sub, i < nn);
-        if (i < nn && sub == 0) {
-            const float2 z = r0[i];
-            v[i] = vi;
-            acc[0] += (double)z.x * vi.x;
-            acc[1] += (double)z.y * vi.y;
-        }
-    }
-    if (grid_sum<2>(acc, sh, partials, cnt, gridDim.x, blockIdx.x) && threadIdx.x == 0)
-        for (int c = 0; c < 2; c++) S->alpha[c] = S->active[c] ? S->rho[c] / acc[c] : 0.0;
+    spmv_rows(m, p, S, [&](int i) { return r0[i]; }, [&](int i, float2 vi, float2 z) {
+        v[i] = vi;
+        acc[0] += (double)z.x * vi.x;
+        acc[1] += (double)z.y * vi.y;
+    });
+    if (!grid_arrive<2>(acc, sh, partials, cnt, gridDim.x, blockIdx.x)) return;
+    const double rho[2] = {S->rho[0], S->rho[1]};
+    const int active[2] = {S->active[0], S->active[1]};
+    grid_total<2>(acc, sh, partials, cnt, gridDim.x);
+    if (threadIdx.x == 0)
+        for (int c = 0; c < 2; c++) S->alpha[c] = active[c] ? rho[c] / acc[c] : 0.0;
 }
 
 // s = r - alpha v; with the preconditioner also z = M^-1 s
@@ -707,41 +814,40 @@ __global__ void __launch_bounds__(kQT)
 k_qp_s(int nn, const float2 *__restrict__ r, const float2 *__restrict__ v, float2 *__restrict__ s,
        const float2 *__restrict__ dinv, float2 *__restrict__ z, const QpSolve *__restrict__ S) {
     pdl_begin();
-    if (!any_active(S)) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nn) return;
+    if (!running(S)) return;
     const float ax = (float)S->alpha[0], ay = (float)S->alpha[1];
-    const float2 ri = r[i], vi = v[i];
-    const float2 si = make_float2(ri.x - ax * vi.x, ri.y - ay * vi.y);
-    s[i] = si;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (nn + 1) / 2) return;
+    const float4 ri = pair(r, t), vi = pair(v, t);
+    const float4 si = make_float4(ri.x - ax * vi.x, ri.y - ay * vi.y, ri.z - ax * vi.z, ri.w - ay * vi.w);
+    set_pair(s, t, si);
     if (dinv) {
-        const float2 d = dinv[i];
-        z[i] = make_float2(si.x * d.x, si.y * d.y);
+        const float4 d = pair(dinv, t);
+        set_pair(z, t, make_float4(si.x * d.x, si.y * d.y, si.z * d.z, si.w * d.w));
     }
 }
 
 // t = A z (z = s, or M^-1 s); omega = t.s / t.t
-__global__ void __launch_bounds__(kQT)
+__global__ void __launch_bounds__(kQT, kSolveBlocks / 148)
 k_qp_at(int nn, QpMat m, const float2 *__restrict__ z, const float2 *__restrict__ s, float2 *__restrict__ t,
         double *__restrict__ partials, unsigned *__restrict__ cnt, QpSolve *__restrict__ S) {
     __shared__ double sh[4 * 32];
     pdl_begin();
-    if (!any_active(S)) return;
+    if (!running(S)) return;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    ROW_GROUPS(nn) {
-        const float2 ti = spmv_row8(m, z, i, sub, i < nn);
-        if (i < nn && sub == 0) {
-            const float2 si = s[i];
-            t[i] = ti;
-            acc[0] += (double)ti.x * ti.x;
-            acc[1] += (double)ti.y * ti.y;
-            acc[2] += (double)ti.x * si.x;
-            acc[3] += (double)ti.y * si.y;
-        }
-    }
-    if (grid_sum<4>(acc, sh, partials, cnt, gridDim.x, blockIdx.x) && threadIdx.x == 0)
+    spmv_rows(m, z, S, [&](int i) { return s[i]; }, [&](int i, float2 ti, float2 si) {
+        t[i] = ti;
+        acc[0] += (double)ti.x * ti.x;
+        acc[1] += (double)ti.y * ti.y;
+        acc[2] += (double)ti.x * si.x;
+        acc[3] += (double)ti.y * si.y;
+    });
+    if (!grid_arrive<4>(acc, sh, partials, cnt, gridDim.x, blockIdx.x)) return;
+    const int active[2] = {S->active[0], S->active[1]};
+    grid_total<4>(acc, sh, partials, cnt, gridDim.x);
+    if (threadIdx.x == 0)
         for (int c = 0; c < 2; c++)
-            if (S->active[c]) S->w[c] = acc[c] > 0.0 ? acc[2 + c] / acc[c] : 0.0;
+            if (active[c]) S->w[c] = acc[c] > 0.0 ? acc[2 + c] / acc[c] : 0.0;
 }
 
 // x += alpha y + omega z (y, z = p, s, or their preconditioned forms);
@@ -752,33 +858,44 @@ k_qp_step(int nn, const float2 *__restrict__ p, const float2 *__restrict__ zs, c
           double *__restrict__ partials, unsigned *__restrict__ cnt, QpSolve *__restrict__ S) {
     __shared__ double sh[4 * 32];
     pdl_begin();
-    if (!any_active(S)) return;
+    if (!running(S)) return;
     float a[2], w[2];
     for (int c = 0; c < 2; c++) {
         a[c] = S->active[c] ? (float)S->alpha[c] : 0.f;
         w[c] = S->active[c] ? (float)S->w[c] : 0.f;
     }
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
-        const float2 pi = p[i], zi = zs[i], si = s[i], ti = t[i], xi = x[i], z = r0[i];
-        x[i] = make_float2(xi.x + a[0] * pi.x + w[0] * zi.x, xi.y + a[1] * pi.y + w[1] * zi.y);
-        const float2 ri = make_float2(si.x - w[0] * ti.x, si.y - w[1] * ti.y);
-        r[i] = ri;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < (nn + 1) / 2; k += gridDim.x * blockDim.x) {
+        const float4 pi = pair(p, k), zi = pair(zs, k), si = pair(s, k), ti = pair(t, k), xi = pair(x, k), z = pair(r0, k);
+        set_pair(x, k, make_float4(xi.x + a[0] * pi.x + w[0] * zi.x, xi.y + a[1] * pi.y + w[1] * zi.y,
+                                   xi.z + a[0] * pi.z + w[0] * zi.z, xi.w + a[1] * pi.w + w[1] * zi.w));
+        const float4 ri = make_float4(si.x - w[0] * ti.x, si.y - w[1] * ti.y, si.z - w[0] * ti.z, si.w - w[1] * ti.w);
+        set_pair(r, k, ri);
         acc[0] += (double)ri.x * ri.x;
         acc[1] += (double)ri.y * ri.y;
         acc[2] += (double)z.x * ri.x;
         acc[3] += (double)z.y * ri.y;
-    }
-    if (grid_sum<4>(acc, sh, partials, cnt, gridDim.x, blockIdx.x) && threadIdx.x == 0) {
-        S->iters++;
-        for (int c = 0; c < 2; c++) {
-            if (!S->active[c]) continue;
-            S->rr[c] = acc[c];
-            S->r0r[c] = acc[2 + c];
-            S->it[c]++;
-            S->active[c] = S->rr[c] > S->tol2[c] && S->it[c] < S->max_it;
+        if (2 * k + 1 < nn) {  // the last row's pair holds no row
+            acc[0] += (double)ri.z * ri.z;
+            acc[1] += (double)ri.w * ri.w;
+            acc[2] += (double)z.z * ri.z;
+            acc[3] += (double)z.w * ri.w;
         }
-        qp_pre(S);
+    }
+    if (!grid_arrive<4>(acc, sh, partials, cnt, gridDim.x, blockIdx.x)) return;
+    QpSolve h = *S;  // the finaliser works on a copy
+    grid_total<4>(acc, sh, partials, cnt, gridDim.x);
+    if (threadIdx.x == 0) {
+        h.iters++;
+        for (int c = 0; c < 2; c++) {
+            if (!h.active[c]) continue;
+            h.rr[c] = acc[c];
+            h.r0r[c] = acc[2 + c];
+            h.it[c]++;
+            h.active[c] = h.rr[c] > h.tol2[c] && h.it[c] < h.max_it;
+        }
+        qp_pre(&h);
+        *S = h;
     }
 }
 
@@ -812,25 +929,44 @@ void qp_bounds(const QpDev &q, const float2 *pos, double *hpwl, cudaStream_t st)
                                                                q.cnt, hpwl);
 }
 
+static int windows(int nn) { return qblocks(nn); }
+// The layout arrays in one block of memory.
+size_t qp_layout_bytes(int nn) {
+    const size_t w = windows(nn);
+    return w * (sizeof(Window) + kSlices * sizeof(int2) + kQT * (2 * sizeof(int2) + 2 * sizeof(int4)));
+}
+static QpLayout layout(const QpDev &q) {
+    const size_t w = windows(q.nn);
+    QpLayout l;
+    l.win = static_cast<Window *>(q.layout);
+    l.longs = reinterpret_cast<int4 *>(l.win + w);
+    l.slot = reinterpret_cast<int2 *>(l.longs + 2 * w * kQT);
+    l.rel = l.slot + w * kQT;
+    l.slice = l.rel + w * kQT;
+    return l;
+}
+// Entries an axis can need: every slice kLongRow long, and the long rows' own.
+size_t qp_entry_cap(int nn, int np) { return (size_t)windows(nn) * kQT * kLongRow + 4 * (size_t)np + 16; }
+
 void qp_rows(const QpDev &q, int fill, cudaStream_t st) {
-    (fill ? k_qp_rows<true> : k_qp_rows<false>)<<<qblocks(q.nn), kQT, 0, st>>>(q.nn, q.obj_pin_start, q.obj_pin_dev, q.pin_net, q.net_first,
-                                             q.net_deg, q.bound, q.owner, q.off, q.abspin, q.count, q.row_x, q.row_y,
-                                             q.col_x, q.val_x, q.col_y, q.val_y, q.diag, q.rhs, q.solve);
+    (fill ? k_qp_rows<true> : k_qp_rows<false>)<<<qblocks(q.nn), kQT, 0, st>>>(
+        q.nn, q.obj_pin_start, q.obj_pin_dev, q.pin_net, q.net_first, q.net_deg, q.bound, q.owner, q.off, q.abspin,
+        q.count, layout(q), q.ent_x, q.ent_y, q.diag, q.rhs, q.solve);
 }
 
-int qp_scan_blocks(int nn) { return (2 * nn + 1 + kScanChunk - 1) / kScanChunk; }
-
-void qp_offsets(const QpDev &q, cudaStream_t st) {
-    const int nb = qp_scan_blocks(q.nn);
-    k_qp_chunk_sums<<<nb, kQT, 0, st>>>(q.count, 2 * q.nn, q.scan);
-    k_qp_chunk_scan<<<1, kQT, 0, st>>>(q.scan, nb, q.count, q.nn, q.cap_x, q.cap_y, q.solve);
-    k_qp_offsets<<<nb, kQT, 0, st>>>(q.count, q.nn, q.scan, nb, q.row_x, q.row_y);
+void qp_scan(const QpDev &q, cudaStream_t st) {
+    k_qp_scan<<<1, kScanThreads, 0, st>>>(windows(q.nn), layout(q).win, q.cap_x, q.cap_y, q.solve);
 }
 
-static QpMat mat(const QpDev &q) { return QpMat{q.row_x, q.col_x, q.row_y, q.col_y, q.val_x, q.val_y, q.diag}; }
+static QpMat mat(const QpDev &q) { return QpMat{q.ent_x, q.ent_y, layout(q), q.count, q.diag, q.nn}; }
+
+// Grids that depend on the sizes alone, so that the dot products group alike on
+// every run: the SpMV kernels' with warps to spare for the long rows of a small
+// design.
+static int spmv_grid(int nn) { return std::min(2 * qblocks(nn), kSolveBlocks); }
 
 void qp_init(const QpDev &q, int max_it, cudaStream_t st) {
-    k_qp_init<<<qgrid(kRowLanes * q.nn), kQT, 0, st>>>(q.nn, mat(q), q.rhs, q.x, q.r, q.r0, q.p, q.v, q.partials,
+    k_qp_init<<<spmv_grid(q.nn), kQT, 0, st>>>(q.nn, mat(q), q.rhs, q.x, q.r, q.r0, q.p, q.v, q.partials,
                                                          q.cnt, max_it, q.solve);
     k_qp_zero<<<qblocks(q.nn), kQT, 0, st>>>(q.nn, q.solve, q.x);
 }
@@ -843,14 +979,18 @@ __global__ void k_qp_dinv(int nn, const float2 *__restrict__ diag, float2 *__res
     dinv[i] = make_float2(d.x != 0.f ? 1.f / d.x : 1.f, d.y != 0.f ? 1.f / d.y : 1.f);
 }
 
+void qp_restart(const QpDev &q, cudaStream_t st) {
+    launch_k(k_qp_restart, spmv_grid(q.nn), kQT, 0, st, q.nn, mat(q), q.rhs, q.x, q.r, q.r0, q.partials, q.cnt,
+             q.solve);
+}
+
 void qp_iterations(const QpDev &q, int count, bool jacobi, cudaStream_t st) {
-    const int b = qblocks(q.nn), bm = qgrid(kRowLanes * q.nn), br = qgrid(q.nn);
+    const int b = qblocks((q.nn + 1) / 2), bm = spmv_grid(q.nn), br = std::min(b, kSolveBlocks);
     for (int k = 0; k < count; k++) {
         // programmatic serialisation: each kernel's blocks are resident and
-        // waiting (pdl_begin) while the previous one drains
-        launch_k(k_qp_restart, bm, kQT, 0, st, q.nn, mat(q), q.rhs, q.x, q.r, q.r0, q.partials, q.cnt, q.solve);
-        // Eigen's preconditioned form: y = M^-1 p and z = M^-1 s go into the
-        // SpMVs and the update; without a preconditioner y = p and z = s
+        // waiting (pdl_begin) while the previous one drains.  Eigen's
+        // preconditioned form: y = M^-1 p and z = M^-1 s go into the SpMVs and
+        // the update; without a preconditioner y = p and z = s
         const float2 *dinv = jacobi ? q.dinv : nullptr;
         const float2 *y = jacobi ? q.y : q.p, *z = jacobi ? q.z : q.s;
         launch_k(k_qp_dir, b, kQT, 0, st, q.nn, q.r, q.v, q.p, dinv, q.y, q.solve);
