@@ -51,7 +51,7 @@ constexpr int kH = 64;      // hidden width
 constexpr int kF = 9;       // input features
 constexpr int kOut = 4;     // q (x, y), f (x, y)
 constexpr int kLayers = 3;  // message-passing layers
-constexpr int kDiffSteps[3] = {8, 32, 128};
+constexpr int kDiff1 = 8, kDiff2 = 32, kDiff3 = 128;  // diffusion steps of the three coordinate features
 constexpr float kCorr = 0.25f;  // bound of a head's correction, in core sizes
 
 // Parameter layout (floats): W0[kH][kF], b0[kH], per layer W[kH][2kH], b[kH],
@@ -64,7 +64,6 @@ inline int off_w(int l) { return kOffL + (l - 1) * kLayerParams; }
 inline int off_b(int l) { return off_w(l) + kH * 2 * kH; }
 
 constexpr int kT = 256;
-constexpr int kRowsPerBlock = 512;  // rows of one partial weight gradient
 inline int nblk(long long n, int t = kT) { return (int)((n + t - 1) / t); }
 
 // Device view of the bound netlist.
@@ -115,6 +114,65 @@ __global__ void k_pad_pins(int np, Net g, int *__restrict__ cnt) {
 __global__ void k_pad_feature(int nt, int nn, const int *__restrict__ cnt, float *__restrict__ X) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < nt) X[(size_t)(nn + t) * kF + 1] = log1pf((float)cnt[t]) * (1.f / 3.f);
+}
+
+// The terminals' pin lists (the transposed aggregation into terminals reads
+// them; training only): their starts by one block from the counts, the pins in
+// any order, then each list in pin order by counting the smaller ones (a block
+// per terminal; the lists are short).
+__global__ void __launch_bounds__(kT) k_pad_start(int nt, const int *__restrict__ cnt, int32_t *__restrict__ start,
+                                                  int *__restrict__ cursor) {
+    __shared__ int tot[kT / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int carry = 0;
+    for (int t0 = 0; t0 < nt; t0 += kT) {
+        const int t = t0 + threadIdx.x, v = t < nt ? cnt[t] : 0;
+        int x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        __syncthreads();
+        if (lane == 31) tot[w] = x;
+        __syncthreads();
+        int before = carry;
+        for (int k = 0; k < kT / 32; k++) {
+            if (k < w) before += tot[k];
+            carry += tot[k];
+        }
+        if (t < nt) start[t] = cursor[t] = before + x - v;
+    }
+    if (threadIdx.x == 0) start[nt] = carry;
+}
+
+__global__ void k_pad_fill(int np, Net g, int *__restrict__ cursor, int32_t *__restrict__ pins) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < np && g.owner[p] >= g.n_obj) pins[atomicAdd(&cursor[g.owner[p] - g.n_obj], 1)] = p;
+}
+
+__global__ void __launch_bounds__(64) k_pad_sort(Net g, const int32_t *__restrict__ start,
+                                                 const int32_t *__restrict__ pins, int32_t *__restrict__ nets) {
+    const int b = start[blockIdx.x], e = start[blockIdx.x + 1];
+    for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
+        const int p = pins[i];
+        int rank = 0;
+        for (int j = b; j < e; j++) rank += pins[j] < p;
+        nets[b + rank] = g.pin_net[p];
+    }
+}
+
+// Targets normalised to the core in place; terminals (c >= nn) have none.
+__global__ void k_target(int N, int nn, float llx, float lly, float w, float h, float4 *__restrict__ t) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= N) return;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < nn) {
+        v = t[c];
+        v = make_float4(__fdiv_rn(__fsub_rn(v.x, llx), w), __fdiv_rn(__fsub_rn(v.y, lly), h),
+                        __fdiv_rn(__fsub_rn(v.z, llx), w), __fdiv_rn(__fsub_rn(v.w, lly), h));
+    }
+    t[c] = v;
 }
 
 __global__ void k_inv_deg(int nnet, const int32_t *__restrict__ deg, float *__restrict__ inv) {
@@ -266,20 +324,37 @@ __global__ void k_node_mean(Net g, const float *__restrict__ inv_pins, const flo
     m[(size_t)c * 32 + lane] = s;
 }
 
-// transpose of node_mean: da[n] = sum over the pins of n on movable nodes c of dm[c] / pins(c)
-__global__ void k_node_mean_t(Net g, const float *__restrict__ inv_pins, const float2 *__restrict__ dm,
-                              float2 *__restrict__ da) {
-    const int n = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (n >= g.nnet) return;
+// transpose of node_mean: da[n] = sum over the pins of n on movable nodes c of
+// dm[c] / pins(c); nets above kWarpPins pins a block each, as in k_net_mean
+__device__ __forceinline__ void add_scaled(float2 &s, float2 t, float w) {
+    s.x += t.x * w;
+    s.y += t.y * w;
+}
+__global__ void __launch_bounds__(kT) k_node_mean_t(Net g, const float *__restrict__ inv_pins,
+                                                    const float2 *__restrict__ dm, float2 *__restrict__ da) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool big = (int)blockIdx.x < g.n_big;
+    const int k = big ? (int)blockIdx.x : g.n_big + ((int)blockIdx.x - g.n_big) * kBigWarps + w;
+    if (k >= g.nnet) return;
+    const int4 r = g.kinfo[k];
+    const int step = big ? kBigWarps : 1;
     float2 s = make_float2(0.f, 0.f);
-    for (int p = g.net_first[n], e = p + g.net_deg[n]; p < e; p++) {
+#pragma unroll 4
+    for (int p = r.x + (big ? w : 0), e = r.x + r.y; p < e; p += step) {
         const int c = g.pin_node[p];
-        if (c >= g.nn) continue;
-        const float2 t = dm[(size_t)c * 32 + lane];
-        s.x += t.x * inv_pins[c];
-        s.y += t.y * inv_pins[c];
+        if (c < g.nn) add_scaled(s, dm[(size_t)c * 32 + lane], inv_pins[c]);
     }
-    da[(size_t)n * 32 + lane] = s;
+    if (big) {
+        __shared__ float2 part[kBigWarps][32];
+        part[w][lane] = s;
+        __syncthreads();
+        if (w != 0) return;
+        for (int j = 1; j < kBigWarps; j++) {
+            s.x += part[j][lane].x;
+            s.y += part[j][lane].y;
+        }
+    }
+    da[(size_t)r.w * 32 + lane] = s;
 }
 
 // transpose of net_mean, added: dh[c] += sum over the pins of node c of da[net] / deg(net)
@@ -289,19 +364,17 @@ __global__ void k_net_mean_t_add(Net g, const float *__restrict__ inv_deg, const
     if (c >= g.N) return;
     float2 s = make_float2(0.f, 0.f);
     if (c < g.nn) {
-        for (int q = g.obj_pin_start[c]; q < g.obj_pin_start[c + 1]; q++) {
+#pragma unroll 4
+        for (int q = g.obj_pin_start[c], e = g.obj_pin_start[c + 1]; q < e; q++) {
             const int n = g.q_net[q];
-            const float2 t = da[(size_t)n * 32 + lane];
-            s.x += t.x * inv_deg[n];
-            s.y += t.y * inv_deg[n];
+            add_scaled(s, da[(size_t)n * 32 + lane], inv_deg[n]);
         }
     } else {
         const int t0 = c - g.nn;
-        for (int q = g.pad_start[t0]; q < g.pad_start[t0 + 1]; q++) {
+#pragma unroll 4
+        for (int q = g.pad_start[t0], e = g.pad_start[t0 + 1]; q < e; q++) {
             const int n = g.pad_net[q];
-            const float2 t = da[(size_t)n * 32 + lane];
-            s.x += t.x * inv_deg[n];
-            s.y += t.y * inv_deg[n];
+            add_scaled(s, da[(size_t)n * 32 + lane], inv_deg[n]);
         }
     }
     float2 &o = dh[(size_t)c * 32 + lane];
@@ -578,109 +651,257 @@ void launch_dense_tc(int grid, cudaStream_t st, int N, const float *XA, const fl
     cudaLaunchKernelEx(&cfg, k_dense_tc, N, XA, XB, W, b, Y, status, engine_status, wait_limit);
 }
 
-// dX = (dY .* (Y > 0)) W, split into dXA (KA cols) and dXB (KB cols).
-template <int KA, int KB>
+// ------------------------------------------------- dense, backward --------
+// FP32 on the CUDA cores, as before: gradients stay in 32 bits, and the hidden
+// layers' two products (0.82 GFLOP each at 50k nodes) are 14 us of FP32 FMAs.
+// One output per thread and two shared-memory reads per FMA made them 258 and
+// 323 us; a thread now holds 4 x 8 outputs and reads 3 (or 5) 16-byte vectors
+// per 32 FMAs, the next tile's rows in flight meanwhile.  50k nodes, us: dX
+// 258 -> 28, dW 323 -> 30.
+constexpr int kDxRows = 64;                       // rows of a tile
+constexpr int kDwRows = 32;
+constexpr int kDwBlocks = 148 * 2;                // partial weight gradients, at most
+constexpr size_t kDxSmem = sizeof(float) * (kH * 2 * kH + kDxRows * kH);
+
+__device__ __forceinline__ float4 relu_mask(float4 d, float4 y) {
+    return make_float4(y.x > 0.f ? d.x : 0.f, y.y > 0.f ? d.y : 0.f, y.z > 0.f ? d.z : 0.f, y.w > 0.f ? d.w : 0.f);
+}
+__device__ __forceinline__ void fma4(float4 &a, float s, float4 w) {
+    a.x = fmaf(s, w.x, a.x);
+    a.y = fmaf(s, w.y, a.y);
+    a.z = fmaf(s, w.z, a.z);
+    a.w = fmaf(s, w.w, a.w);
+}
+
+// dX = (dY .* (Y > 0)) W of a hidden layer, split into dXA and dXB (kH columns
+// each).  Blocks take tiles of kDxRows rows in turn, W (FP32) staged once; thread
+// (tx, ty): rows 4 ty .. 4 ty + 3, columns 4 tx .. 4 tx + 3 of each half; every
+// output adds o = 0 .. 63 in order.
 __global__ void __launch_bounds__(kT) k_dense_dx(int N, const float *__restrict__ dY, const float *__restrict__ Y,
                                                  const __nv_bfloat16 *__restrict__ W, float *__restrict__ dXA,
                                                  float *__restrict__ dXB) {
-    constexpr int K = KA + KB, PER = (K + 3) / 4;
-    extern __shared__ float sm[];
-    float *Ws = sm;           // [kH][K]
-    float *Zs = sm + kH * K;  // [64][kH + 1]
-    for (int i = threadIdx.x; i < kH * K; i += kT) Ws[i] = bf(W[i]);
-    const int r0 = blockIdx.x * 64;
-    for (int i = threadIdx.x; i < 64 * kH; i += kT) {
-        const int r = i / kH, o = i - r * kH, row = r0 + r;
-        float z = 0.f;
-        if (row < N) {
-            const size_t at = (size_t)row * kH + o;
-            z = Y[at] > 0.f ? dY[at] : 0.f;
+    extern __shared__ float4 sm4[];
+    float4 *Ws = sm4;                        // [kH][2 kH / 4]
+    float4 *Zs = sm4 + kH * 2 * kH / 4;      // [kDxRows][kH / 4]
+    for (int i = threadIdx.x; i < kH * 2 * kH / 4; i += kT) {
+        const __nv_bfloat16 *w = W + 4 * i;
+        Ws[i] = make_float4(bf(w[0]), bf(w[1]), bf(w[2]), bf(w[3]));
+    }
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int tiles = (N + kDxRows - 1) / kDxRows;
+    constexpr int kPer = kDxRows * (kH / 4) / kT;  // float4 of a tile per thread
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 d[kPer], y[kPer];
+    auto load = [&](int tile) {
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            const int i = threadIdx.x + u * kT, row = tile * kDxRows + (i >> 4);
+            const size_t at = (size_t)row * (kH / 4) + (i & 15);
+            d[u] = row < N ? reinterpret_cast<const float4 *>(dY)[at] : zero;
+            y[u] = row < N ? reinterpret_cast<const float4 *>(Y)[at] : zero;
         }
-        Zs[r * (kH + 1) + o] = z;
-    }
-    __syncthreads();
-    const int r = threadIdx.x >> 2, k0 = (threadIdx.x & 3) * PER;
-    float acc[PER];
+    };
+    load(blockIdx.x);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        __syncthreads();  // the tile before has been read (first: nothing)
 #pragma unroll
-    for (int j = 0; j < PER; j++) acc[j] = 0.f;
-    for (int o = 0; o < kH; o++) {
-        const float z = Zs[r * (kH + 1) + o];
+        for (int u = 0; u < kPer; u++) Zs[threadIdx.x + u * kT] = relu_mask(d[u], y[u]);
+        __syncthreads();
+        load(tile + gridDim.x);
+        float4 a[4], b[4];
 #pragma unroll
-        for (int j = 0; j < PER; j++)
-            if (k0 + j < K) acc[j] = fmaf(z, Ws[o * K + k0 + j], acc[j]);
-    }
-    const int row = r0 + r;
-    if (row >= N) return;
+        for (int i = 0; i < 4; i++) a[i] = b[i] = zero;
+#pragma unroll 4
+        for (int o4 = 0; o4 < kH / 4; o4++) {
+            float z[4][4];
 #pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const int k = k0 + j;
-        if (k < KA)
-            dXA[(size_t)row * KA + k] = acc[j];
-        else if (k < K && dXB)
-            dXB[(size_t)row * KB + (k - KA)] = acc[j];
+            for (int i = 0; i < 4; i++) {
+                const float4 v = Zs[(4 * ty + i) * (kH / 4) + o4];
+                z[i][0] = v.x;
+                z[i][1] = v.y;
+                z[i][2] = v.z;
+                z[i][3] = v.w;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float4 wa = Ws[(4 * o4 + j) * (2 * kH / 4) + tx], wb = Ws[(4 * o4 + j) * (2 * kH / 4) + 16 + tx];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    fma4(a[i], z[i][j], wa);
+                    fma4(b[i], z[i][j], wb);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int row = tile * kDxRows + 4 * ty + i;
+            if (row >= N) continue;
+            reinterpret_cast<float4 *>(dXA)[(size_t)row * (kH / 4) + tx] = a[i];
+            reinterpret_cast<float4 *>(dXB)[(size_t)row * (kH / 4) + tx] = b[i];
+        }
     }
 }
 
-// Per-block partial weight gradient: P[o][k] = sum_r Z[r][o] X[r][k] and
-// P[O*K + o] = sum_r Z[r][o] over the block's rows, Z = dY .* (Y > 0) when Y
-// is given (ReLU layers) else dY.  Rows are read in 32-row tiles.
-template <int O, int KA, int KB>
-__global__ void __launch_bounds__(kT) k_dweight(int N, int rows_per_block, const float *__restrict__ dY,
-                                                const float *__restrict__ Y, const float *__restrict__ XA,
-                                                const float *__restrict__ XB, float *__restrict__ partial) {
-    constexpr int K = KA + KB, OK = O * K, PER = (OK + kT - 1) / kT, TR = 32;
-    __shared__ float Zs[TR][O + 1];
-    __shared__ float Xs[TR][K + 1];
-    float acc[PER], bacc = 0.f;
+// Rows [rb, re) of a block's partial weight gradient: equal runs of whole tiles.
+__device__ __forceinline__ void dw_rows(int N, int &rb, int &re) {
+    const int tiles = (N + kDwRows - 1) / kDwRows, per = (tiles + gridDim.x - 1) / gridDim.x;
+    rb = min(N, (int)blockIdx.x * per * kDwRows);
+    re = min(N, rb + per * kDwRows);
+}
+
+// Per-block partial weight gradient of a hidden layer: P[o][k] = sum_r Z[r][o]
+// X[r][k] and P[kH 2kH + o] = sum_r Z[r][o] over the block's rows, Z = dY .* (Y >
+// 0), X = [XA | XB].  Thread (tx, ty): outputs 4 ty .. 4 ty + 3 x columns 4 tx ..
+// of each half, rows in order.
+__global__ void __launch_bounds__(kT, 2) k_dw_hidden(int N, const float *__restrict__ dY, const float *__restrict__ Y,
+                                                     const float *__restrict__ XA, const float *__restrict__ XB,
+                                                     float *__restrict__ partial) {
+    __shared__ float4 Zs[kDwRows][kH / 4], As[kDwRows][kH / 4], Bs[kDwRows][kH / 4];
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    int rb, re;
+    dw_rows(N, rb, re);
+    constexpr int kPer = kDwRows * (kH / 4) / kT;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 d[kPer], y[kPer], xa[kPer], xb[kPer];
+    auto load = [&](int t0) {
 #pragma unroll
-    for (int j = 0; j < PER; j++) acc[j] = 0.f;
-    const int rb = blockIdx.x * rows_per_block, re = min(N, rb + rows_per_block);
-    for (int t0 = rb; t0 < re; t0 += TR) {
+        for (int u = 0; u < kPer; u++) {
+            const int i = threadIdx.x + u * kT, row = t0 + (i >> 4);
+            const size_t at = (size_t)row * (kH / 4) + (i & 15);
+            const bool in = row < re;
+            d[u] = in ? reinterpret_cast<const float4 *>(dY)[at] : zero;
+            y[u] = in ? reinterpret_cast<const float4 *>(Y)[at] : zero;
+            xa[u] = in ? reinterpret_cast<const float4 *>(XA)[at] : zero;
+            xb[u] = in ? reinterpret_cast<const float4 *>(XB)[at] : zero;
+        }
+    };
+    float4 a[4], b[4];
+    float bias[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; i++) a[i] = b[i] = zero;
+    load(rb);
+    for (int t0 = rb; t0 < re; t0 += kDwRows) {
         __syncthreads();
-        for (int i = threadIdx.x; i < TR * O; i += kT) {
-            const int r = i / O, o = i - r * O, row = t0 + r;
-            float z = 0.f;
-            if (row < re) {
-                const size_t at = (size_t)row * O + o;
-                z = (!Y || Y[at] > 0.f) ? dY[at] : 0.f;
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            const int i = threadIdx.x + u * kT;
+            (&Zs[0][0])[i] = relu_mask(d[u], y[u]);
+            (&As[0][0])[i] = xa[u];
+            (&Bs[0][0])[i] = xb[u];
+        }
+        __syncthreads();
+        load(t0 + kDwRows);
+#pragma unroll 8
+        for (int r = 0; r < kDwRows; r++) {
+            const float4 z4 = Zs[r][ty], va = As[r][tx], vb = Bs[r][tx];
+            const float z[4] = {z4.x, z4.y, z4.z, z4.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                fma4(a[i], z[i], va);
+                fma4(b[i], z[i], vb);
+                bias[i] += z[i];
             }
-            Zs[r][o] = z;
         }
-        for (int i = threadIdx.x; i < TR * K; i += kT) {
-            const int r = i / K, k = i - r * K, row = t0 + r;
-            float v = 0.f;
-            if (row < re) v = k < KA ? XA[(size_t)row * KA + k] : XB[(size_t)row * KB + (k - KA)];
-            Xs[r][k] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < PER; j++) {
-            const int i = threadIdx.x + j * kT;
-            if (i >= OK) break;
-            const int o = i / K, k = i - o * K;
-            float s = acc[j];
-            for (int r = 0; r < TR; r++) s = fmaf(Zs[r][o], Xs[r][k], s);
-            acc[j] = s;
-        }
-        if (threadIdx.x < O)
-            for (int r = 0; r < TR; r++) bacc += Zs[r][threadIdx.x];
     }
-    float *P = partial + (size_t)blockIdx.x * (OK + O);
+    float *P = partial + (size_t)blockIdx.x * (kH * 2 * kH + kH);
 #pragma unroll
-    for (int j = 0; j < PER; j++) {
-        const int i = threadIdx.x + j * kT;
-        if (i < OK) P[i] = acc[j];
+    for (int i = 0; i < 4; i++) {
+        float4 *row = reinterpret_cast<float4 *>(P + (size_t)(4 * ty + i) * 2 * kH);
+        row[tx] = a[i];
+        row[kH / 4 + tx] = b[i];
+        if (tx == 0) P[kH * 2 * kH + 4 * ty + i] = bias[i];
     }
-    if (threadIdx.x < O) P[OK + threadIdx.x] = bacc;
+}
+
+// The same of the input layer (kF columns): lane o of four row groups, the
+// groups' sums added in order.
+__global__ void __launch_bounds__(kT) k_dw_input(int N, const float *__restrict__ dY, const float *__restrict__ Y,
+                                                 const float *__restrict__ X, float *__restrict__ partial) {
+    constexpr int kG = kT / kH;
+    __shared__ float sums[kG][kF + 1][kH];
+    const int o = threadIdx.x & (kH - 1), grp = threadIdx.x / kH;
+    int rb, re;
+    dw_rows(N, rb, re);
+    float acc[kF + 1];
+#pragma unroll
+    for (int k = 0; k <= kF; k++) acc[k] = 0.f;
+#pragma unroll 4
+    for (int r = rb + grp; r < re; r += kG) {
+        const size_t at = (size_t)r * kH + o;
+        const float z = Y[at] > 0.f ? dY[at] : 0.f;
+        const float *x = X + (size_t)r * kF;
+#pragma unroll
+        for (int k = 0; k < kF; k++) acc[k] = fmaf(z, __ldg(x + k), acc[k]);
+        acc[kF] += z;
+    }
+#pragma unroll
+    for (int k = 0; k <= kF; k++) sums[grp][k][o] = acc[k];
+    __syncthreads();
+    float *P = partial + (size_t)blockIdx.x * (kH * kF + kH);
+    for (int i = threadIdx.x; i < kH * (kF + 1); i += kT) {
+        const int oo = i & (kH - 1), k = i / kH;
+        float v = sums[0][k][oo];
+        for (int j = 1; j < kG; j++) v += sums[j][k][oo];
+        P[k < kF ? oo * kF + k : kH * kF + oo] = v;
+    }
+}
+
+// The same of the output layer: P[j][k] = sum_r dout[r][j] h[r][k], lane k of
+// four row groups.
+__global__ void __launch_bounds__(kT) k_dw_output(int N, const float4 *__restrict__ dout, const float *__restrict__ h,
+                                                  float *__restrict__ partial) {
+    constexpr int kG = kT / kH;
+    __shared__ float sums[kG][kOut][kH], bsum[kG][kOut];
+    const int k = threadIdx.x & (kH - 1), grp = threadIdx.x / kH;
+    int rb, re;
+    dw_rows(N, rb, re);
+    float acc[kOut] = {0.f, 0.f, 0.f, 0.f}, b[kOut] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int r = rb + grp; r < re; r += kG) {
+        const float4 d = dout[r];
+        const float x = h[(size_t)r * kH + k], dd[kOut] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+        for (int j = 0; j < kOut; j++) {
+            acc[j] = fmaf(dd[j], x, acc[j]);
+            b[j] += dd[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kOut; j++) {
+        sums[grp][j][k] = acc[j];
+        if (k == 0) bsum[grp][j] = b[j];
+    }
+    __syncthreads();
+    float *P = partial + (size_t)blockIdx.x * (kOut * kH + kOut);
+    for (int i = threadIdx.x; i < kOut * kH; i += kT) {
+        const int j = i / kH, kk = i & (kH - 1);
+        float v = sums[0][j][kk];
+        for (int q = 1; q < kG; q++) v += sums[q][j][kk];
+        P[i] = v;
+    }
+    if (threadIdx.x < kOut) {
+        float v = bsum[0][threadIdx.x];
+        for (int q = 1; q < kG; q++) v += bsum[q][threadIdx.x];
+        P[kOut * kH + threadIdx.x] = v;
+    }
 }
 
 // grad[w_off + i] = sum over blocks of partial[blk][i] (weights), then biases.
-__global__ void k_reduce_partials(int blocks, int OK, int O, const float *__restrict__ partial, float *__restrict__ grad,
-                                  int w_off, int b_off) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= OK + O) return;
+// 32 outputs per block; thread row j adds the blocks j, j + 8, ... in order, the
+// eight sums are added in order.
+__global__ void __launch_bounds__(kT) k_reduce_partials(int blocks, int OK, int O, const float *__restrict__ partial,
+                                                        float *__restrict__ grad, int w_off, int b_off) {
+    __shared__ float part[kT / 32][32];
+    const int lane = threadIdx.x & 31, j = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int b = 0; b < blocks; b++) s += partial[(size_t)b * (OK + O) + i];
+    if (i < OK + O) {
+#pragma unroll 8
+        for (int b = j; b < blocks; b += kT / 32) s += partial[(size_t)b * (OK + O) + i];
+    }
+    part[j][lane] = s;
+    __syncthreads();
+    if (j != 0 || i >= OK + O) return;
+    for (int k = 1; k < kT / 32; k++) s += part[k][lane];
     if (i < OK)
         grad[w_off + i] = s;
     else
@@ -750,11 +971,14 @@ __global__ void k_loss(int N, int nn, const float4 *__restrict__ raw, const floa
     }
 }
 
-__global__ void k_sum_loss(int n, const double *__restrict__ part, int nn, double *__restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    for (int i = 0; i < n; i++) s += part[i];
-    out[0] = s / (2.0 * nn);
+// One block: thread t adds the partials t, t + kT, ... in order, then a fixed tree.
+__global__ void __launch_bounds__(kT) k_sum_loss(int n, const double *__restrict__ part, int nn,
+                                                 double *__restrict__ out) {
+    __shared__ double sh[32];
+    double s[1] = {0.0};
+    for (int i = threadIdx.x; i < n; i += kT) s[0] += part[i];
+    block_sum<1>(s, sh);
+    if (threadIdx.x == 0) out[0] = s[0] / (2.0 * nn);
 }
 
 // dh[c][k] = sum_j dout[c][j] W4[j][k]
@@ -821,11 +1045,11 @@ struct ep_gnn {
     Net net{};
     EngineGraph eg{};
     // capacities and buffers
-    size_t capN = 0, capNet = 0, capPad = 0, capT = 0, capP = 0;
+    size_t capN = 0, capNet = 0, capT = 0, capP = 0;
     float *X = nullptr, *inv_pins = nullptr, *inv_deg = nullptr;
     float2 *v = nullptr, *netv = nullptr;
-    int *padcnt = nullptr;
-    int32_t *pad_start = nullptr, *pad_net = nullptr;
+    int *padcnt = nullptr, *pad_cursor = nullptr;
+    int32_t *pad_start = nullptr, *pad_net = nullptr, *pad_pins = nullptr;
     int4 *kinfo = nullptr;
     int32_t *pin_node = nullptr, *q_net = nullptr;
     float *h[kLayers + 1] = {}, *m[kLayers + 1] = {};
@@ -849,7 +1073,6 @@ namespace {
     } while (0)
 
 size_t smem_dense(int K) { return sizeof(float) * ((size_t)K * kH + (size_t)kDenseRows * (K + 1)); }
-size_t smem_dx(int K) { return sizeof(float) * ((size_t)kH * K + 64 * (size_t)(kH + 1)); }
 
 void set_smem_attrs() {
     static std::vector<int> done;
@@ -859,7 +1082,7 @@ void set_smem_attrs() {
     done.push_back(dev);
     cudaFuncSetAttribute(k_dense<kF, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dense(kF));
     cudaFuncSetAttribute(k_dense_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
-    cudaFuncSetAttribute(k_dense_dx<kH, kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dx(2 * kH));
+    cudaFuncSetAttribute(k_dense_dx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDxSmem);
 }
 
 template <typename T>
@@ -880,8 +1103,6 @@ ep_status reserve(ep_gnn *g, size_t N, size_t nnet, size_t nt, size_t np) {
     g->ws.clear();
     g->uid = 0;
     g->pads_ready = false;
-    g->capPad = 0;
-    g->pad_net = nullptr;
     // a quarter of headroom on every dimension, so designs of about the same
     // size do not each grow the workspace again (a growth frees and
     // reallocates all of it)
@@ -892,9 +1113,10 @@ ep_status reserve(ep_gnn *g, size_t N, size_t nnet, size_t nt, size_t np) {
     np = grow(np, g->capP);
     bool ok = walloc(g, g->X, N * kF) && walloc(g, g->inv_pins, N) && walloc(g, g->inv_deg, nnet) &&
               walloc(g, g->v, N) && walloc(g, g->netv, nnet) && walloc(g, g->padcnt, nt) &&
-              walloc(g, g->pad_start, nt + 1) && walloc(g, g->a, nnet * kH) && walloc(g, g->dh, N * kH) &&
+              walloc(g, g->pad_start, nt + 1) && walloc(g, g->pad_cursor, nt) && walloc(g, g->pad_net, np) &&
+              walloc(g, g->pad_pins, np) && walloc(g, g->a, nnet * kH) && walloc(g, g->dh, N * kH) &&
               walloc(g, g->dx, N * kH) && walloc(g, g->dm, N * kH) && walloc(g, g->da, nnet * kH) &&
-              walloc(g, g->partial, (size_t)nblk((long long)N, kRowsPerBlock) * (kH * 2 * kH + kH)) &&
+              walloc(g, g->partial, (size_t)kDwBlocks * (kH * 2 * kH + kH)) &&
               walloc(g, g->raw, N) && walloc(g, g->pred, N) && walloc(g, g->dout, N) && walloc(g, g->target, N) &&
               walloc(g, g->xy, N) && walloc(g, g->loss_part, nblk((long long)N)) && walloc(g, g->kinfo, nnet) &&
               walloc(g, g->pin_node, np) && walloc(g, g->q_net, np);
@@ -967,11 +1189,11 @@ ep_status bind(ep_gnn *g, ep_engine *e) {
     k_inv_deg<<<nblk(eg.nnet), kT, 0, st>>>(eg.nnet, eg.d_net_deg, g->inv_deg);
     k_graph_index<<<nblk(std::max(eg.nnet, eg.np)), kT, 0, st>>>(n, eg.np, g->kinfo, g->pin_node, g->q_net);
     int col = 3;
-    for (int k = 1; k <= kDiffSteps[2]; k++) {
+    for (int k = 1; k <= kDiff3; k++) {
         // programmatic serialisation: the next pass's blocks wait resident
         launch_k(k_diff_net, nblk(31LL * n.n_big + eg.nnet), kT, 0, st, n, (const float2 *)g->v, g->netv);
         launch_k(k_diff_node, nblk(eg.nn), kT, 0, st, n, (const float *)g->inv_pins, (const float2 *)g->netv, g->v);
-        if (k == kDiffSteps[0] || k == kDiffSteps[1] || k == kDiffSteps[2]) {
+        if (k == kDiff1 || k == kDiff2 || k == kDiff3) {
             launch_k(k_store_feature, nblk(N), kT, 0, st, N, (const float2 *)g->v, g->X, col);
             col += 2;
         }
@@ -981,40 +1203,17 @@ ep_status bind(ep_gnn *g, ep_engine *e) {
     return EP_OK;
 }
 
-// The terminals' pin lists (the transposed aggregation into terminals needs
-// them; training only), built on the host from the engine's pin owners.
+// The terminals' pin lists of the bound netlist.
 ep_status bind_pads(ep_gnn *g) {
     if (g->pads_ready) return EP_OK;
     const EngineGraph &eg = g->eg;
-    std::vector<int32_t> start(eg.nt + 1, 0), nets;
-    for (int p = 0; p < eg.np; p++)
-        if (eg.pin_owner[p] >= eg.n_obj) start[eg.pin_owner[p] - eg.n_obj + 1]++;
-    for (int t = 0; t < eg.nt; t++) start[t + 1] += start[t];
-    nets.resize(std::max(start[eg.nt], 1));
-    {
-        std::vector<int32_t> fill(start.begin(), start.end() - 1);
-        for (int p = 0; p < eg.np; p++)
-            if (eg.pin_owner[p] >= eg.n_obj) nets[fill[eg.pin_owner[p] - eg.n_obj]++] = eg.pin_net[p];
+    cudaStream_t st = eg.st;
+    if (eg.nt > 0) {
+        k_pad_start<<<1, kT, 0, st>>>(eg.nt, g->padcnt, g->pad_start, g->pad_cursor);
+        k_pad_fill<<<nblk(eg.np), kT, 0, st>>>(eg.np, g->net, g->pad_cursor, g->pad_pins);
+        k_pad_sort<<<eg.nt, 64, 0, st>>>(g->net, g->pad_start, g->pad_pins, g->pad_net);
+        GK(cudaGetLastError());
     }
-    if (nets.size() > g->capPad) {
-        if (g->pad_net) {
-            cudaStreamSynchronize(eg.st);
-            cudaFree(g->pad_net);
-            g->ws.erase(std::find(g->ws.begin(), g->ws.end(), (void *)g->pad_net));
-            g->pad_net = nullptr;
-        }
-        if (!walloc(g, g->pad_net, nets.size())) {
-            g->capPad = 0;
-            g->err = "cudaMalloc failed for the terminals' pin lists";
-            return EP_ERR_NOMEM;
-        }
-        g->capPad = nets.size();
-    }
-    GK(cudaMemcpyAsync(g->pad_start, start.data(), sizeof(int32_t) * start.size(), cudaMemcpyHostToDevice, eg.st));
-    GK(cudaMemcpyAsync(g->pad_net, nets.data(), sizeof(int32_t) * nets.size(), cudaMemcpyHostToDevice, eg.st));
-    GK(cudaStreamSynchronize(eg.st));  // the host vectors go out of scope
-    g->net.pad_start = g->pad_start;
-    g->net.pad_net = g->pad_net;
     g->pads_ready = true;
     return EP_OK;
 }
@@ -1059,31 +1258,31 @@ ep_status backward(ep_gnn *g) {
     const __nv_bfloat16 *wb = g->wb;
     const int lb = nblk(N);
     k_loss<<<lb, kT, 0, st>>>(N, n.nn, g->raw, g->pred, g->target, g->dout, g->loss_part);
-    k_sum_loss<<<1, 32, 0, st>>>(lb, g->loss_part, n.nn, g->loss);
-    const int pb = nblk(N, kRowsPerBlock);
+    k_sum_loss<<<1, kT, 0, st>>>(lb, g->loss_part, n.nn, g->loss);
+    const int pb = std::min(nblk(N, kDwRows), kDwBlocks);
+    auto reduce = [&](int OK, int O, int w_off, int b_off) {
+        k_reduce_partials<<<nblk(OK + O, 32), kT, 0, st>>>(pb, OK, O, g->partial, g->grad, w_off, b_off);
+    };
     // output layer
-    k_dweight<kOut, kH, 0><<<pb, kT, 0, st>>>(N, kRowsPerBlock, (const float *)g->dout, nullptr, g->h[kLayers],
-                                             nullptr, g->partial);
-    k_reduce_partials<<<nblk(kOut * kH + kOut), kT, 0, st>>>(pb, kOut * kH, kOut, g->partial, g->grad, kOffW4,
-                                                             kOffB4);
+    k_dw_output<<<pb, kT, 0, st>>>(N, g->dout, g->h[kLayers], g->partial);
+    reduce(kOut * kH, kOut, kOffW4, kOffB4);
     k_output_dh<<<nblk((long long)N * kH), kT, 0, st>>>(N, g->dout, wb + kOffW4, g->dh);
     // message-passing layers, last to first; dh holds d loss / d h_l
     float *dh = g->dh, *dx = g->dx;
     for (int l = kLayers; l >= 1; l--) {
-        k_dweight<kH, kH, kH><<<pb, kT, 0, st>>>(N, kRowsPerBlock, dh, g->h[l], g->h[l - 1], g->m[l], g->partial);
-        k_reduce_partials<<<nblk(kH * 2 * kH + kH), kT, 0, st>>>(pb, kH * 2 * kH, kH, g->partial, g->grad, off_w(l),
-                                                                 off_b(l));
+        k_dw_hidden<<<pb, kT, 0, st>>>(N, dh, g->h[l], g->h[l - 1], g->m[l], g->partial);
+        reduce(kH * 2 * kH, kH, off_w(l), off_b(l));
         // d h_{l-1} (direct part) into dx, d m_l into g->dm
-        k_dense_dx<kH, kH><<<nblk(N, 64), kT, smem_dx(2 * kH), st>>>(N, dh, g->h[l], wb + off_w(l), dx, g->dm);
-        k_node_mean_t<<<nblk((long long)n.nnet * 32), kT, 0, st>>>(n, g->inv_pins, (const float2 *)g->dm,
-                                                                   (float2 *)g->da);
+        k_dense_dx<<<std::min(nblk(N, kDxRows), 148 * 2), kT, kDxSmem, st>>>(N, dh, g->h[l], wb + off_w(l), dx, g->dm);
+        k_node_mean_t<<<n.n_big + nblk(n.nnet - n.n_big, kBigWarps), kT, 0, st>>>(n, g->inv_pins, (const float2 *)g->dm,
+                                                                                 (float2 *)g->da);
         k_net_mean_t_add<<<nblk((long long)N * 32), kT, 0, st>>>(n, g->inv_deg, (const float2 *)g->da,
                                                                  (float2 *)dx);
         std::swap(dh, dx);
     }
     // input layer
-    k_dweight<kH, kF, 0><<<pb, kT, 0, st>>>(N, kRowsPerBlock, dh, g->h[0], g->X, nullptr, g->partial);
-    k_reduce_partials<<<nblk(kH * kF + kH), kT, 0, st>>>(pb, kH * kF, kH, g->partial, g->grad, kOffW0, kOffB0);
+    k_dw_input<<<pb, kT, 0, st>>>(N, dh, g->h[0], g->X, g->partial);
+    reduce(kH * kF, kH, kOffW0, kOffB0);
     GK(cudaGetLastError());
     return EP_OK;
 }
@@ -1092,13 +1291,10 @@ ep_status backward(ep_gnn *g) {
 // placement x, y, final x, y), normalised to the core.
 ep_status upload_target(ep_gnn *g, const float *t4) {
     const Grid &gr = g->eg.grid;
-    const float W = gr.urx - gr.llx, H = gr.ury - gr.lly;
-    std::vector<float4> t(g->net.N, make_float4(0.f, 0.f, 0.f, 0.f));
-    for (int c = 0; c < g->net.nn; c++)
-        t[c] = make_float4((t4[4 * c] - gr.llx) / W, (t4[4 * c + 1] - gr.lly) / H, (t4[4 * c + 2] - gr.llx) / W,
-                           (t4[4 * c + 3] - gr.lly) / H);
-    GK(cudaMemcpyAsync(g->target, t.data(), sizeof(float4) * t.size(), cudaMemcpyHostToDevice, g->eg.st));
-    GK(cudaStreamSynchronize(g->eg.st));
+    GK(cudaMemcpyAsync(g->target, t4, sizeof(float4) * g->net.nn, cudaMemcpyHostToDevice, g->eg.st));
+    k_target<<<nblk(g->net.N), kT, 0, g->eg.st>>>(g->net.N, g->net.nn, gr.llx, gr.lly, gr.urx - gr.llx, gr.ury - gr.lly,
+                                                 g->target);
+    GK(cudaGetLastError());
     return EP_OK;
 }
 
