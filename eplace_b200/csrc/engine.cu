@@ -109,6 +109,7 @@ struct ep_engine {
     int32_t *net_first = nullptr, *net_deg = nullptr, *pin_net = nullptr;
     int32_t *net_dev_order = nullptr;  // nets in device pin order (grouped by degree)
     int n_big_nets = 0;                // nets above kWarpPins pins (the head of that order)
+    int max_net_pins = 0, max_node_pins = 0;
     double create_s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // ep_create phases (ep_info.create_seconds)
     int64_t qp_launches = 0;                         // kernels of the current quadratic placement call
     uint64_t uid = 0;  // distinct per engine created in this process
@@ -915,7 +916,10 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
                 if (o < nn) h_npins[o] = (float)at;
             }
         });
-        for (int o = 0; o < no; o++) ops[o + 1] += ops[o];
+        for (int o = 0; o < no; o++) {
+            e->max_node_pins = std::max(e->max_node_pins, ops[o + 1]);
+            ops[o + 1] += ops[o];
+        }
         parallel_ranges(np, nth, [&](int t, int p0, int p1) {
             for (int p = p0; p < p1; p++)
                 if (owner[p] < no) pin_slot[p] = ops[owner[p]] + cnt[t][owner[p]]++;
@@ -936,6 +940,7 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
         for (int n = 0; n < nnet; n++) {
             int deg = net_start[n + 1] - net_start[n];
             (deg > kWarpPins ? big_list : by_deg[deg]).push_back(n);
+            e->max_net_pins = std::max(e->max_net_pins, deg);
         }
         // by lowest owner inside a degree, so that neighbouring nets read
         // neighbouring centres: a counting sort over runs of 64 objects
@@ -2335,6 +2340,8 @@ int engine_graph(ep_engine *e, EngineGraph *g) {
     g->d_pin_net = e->pin_net;
     g->d_net_dev_order = e->net_dev_order;
     g->n_big_nets = e->n_big_nets;
+    g->max_net_pins = e->max_net_pins;
+    g->max_node_pins = e->max_node_pins;
     g->d_obj_pin_start = e->obj_pin_start;
     g->d_obj_pin_dev = e->obj_pin_dev;
     g->d_area = e->area;

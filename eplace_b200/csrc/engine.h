@@ -196,6 +196,7 @@ struct EngineGraph {
     const int32_t *d_pin_owner, *d_net_first, *d_net_deg, *d_pin_net;
     const int32_t *d_net_dev_order;  // [nnet] nets in device pin order (grouped by degree)
     int n_big_nets;                  // nets above kWarpPins pins: the first n_big_nets of that order
+    int max_net_pins, max_node_pins;  // most pins of a net, of a movable node
     const int32_t *d_obj_pin_start, *d_obj_pin_dev;  // object -> its device pins
     const float *d_area, *d_npins;                   // [n_obj]
     const void *d_pos;                               // [n_obj + nt] centres, vec2<R>

@@ -260,6 +260,192 @@ __global__ void k_store_feature(int N, const float2 *__restrict__ v, float *__re
     X[(size_t)c * kF + col + 1] = v[c].y;
 }
 
+// ---- the diffusion as one launch -----------------------------------------------
+// 256 dependent passes of a few microseconds: launched one by one they cost 4.2
+// us each however small the design.  Here a CTA per SM keeps its share of the
+// indices in shared memory for all of them -- a run of nets and a run of movable
+// nodes, cut so that every CTA has about the same number of pins -- and the CTAs
+// meet at a barrier in global memory after each pass (a cooperative launch, so
+// they are resident together).  In a pass all threads gather their CTA's pin
+// values into shared memory, every load in flight at once (the barrier's acquire
+// is what makes the L1 fetch them anew), and then a thread per row (a warp per net above kWarpPins
+// pins) adds them in the order of k_diff_net and k_diff_node: the same sums bit
+// for bit.  Taken when the share fits (kDiffSmem); the pass-by-pass kernels above
+// stay for larger designs and devices without cooperative launches.  128 steps,
+// us: 2k cells 1050 -> 590, 50k 1190 -> 790, 200k 1910 -> 1400.
+constexpr int kDiffThreads = 1024;
+constexpr size_t kDiffSmem = 216 * 1024;
+constexpr unsigned kBarrierPolls = 1u << 22;  // about a second or two
+
+struct DiffShare {  // pins a CTA's share can have (net phase, node phase)
+    int net_pins, node_pins;
+};
+__host__ __device__ __forceinline__ size_t diff_smem(DiffShare s) {
+    const int most = max(s.net_pins, s.node_pins);
+    return sizeof(float2) * ((size_t)most + most / 16 + 1) + sizeof(int32_t) * ((size_t)s.net_pins + s.node_pins);
+}
+// Place of pin i's value: skewed, so that the threads of a warp, whose rows start
+// 2, 4, ... 32 pins apart, read different banks.
+__device__ __forceinline__ int skew(int i) { return i + (i >> 4); }
+
+// First k in [0, n) whose key(k) >= x (keys ascending), n if there is none.
+template <class Key>
+__device__ __forceinline__ int first_at_least(int n, int x, Key &&key) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (key(mid) >= x)
+            hi = mid;
+        else
+            lo = mid + 1;
+    }
+    return lo;
+}
+
+// All CTAs have written what they wrote before it; false when the wait gave up.
+__device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+        int got = 0;
+        for (unsigned it = 0; it < kBarrierPolls && !got; it++) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            got = v >= target;
+        }
+        ok = got;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+__device__ __forceinline__ void gather_pins(const int32_t *__restrict__ idx, int n, const float2 *src,
+                                            float2 *__restrict__ val) {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < n; i += kDiffThreads) val[skew(i)] = src[idx[i]];
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kDiffThreads, 1)
+k_diffuse(Net g, int np, DiffShare share, const float *__restrict__ inv_pins, float2 *v, float2 *a,
+          float *__restrict__ X, unsigned *__restrict__ count, int *__restrict__ status, int *__restrict__ engine_status) {
+    extern __shared__ __align__(16) unsigned char diff_sm[];
+    float2 *val = reinterpret_cast<float2 *>(diff_sm);
+    int32_t *net_idx = reinterpret_cast<int32_t *>(val + skew(max(share.net_pins, share.node_pins)) + 1);
+    int32_t *node_idx = net_idx + share.net_pins;
+    __shared__ int cut[4];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, G = gridDim.x, b = blockIdx.x;
+    const int nq = g.obj_pin_start[g.nn];
+    if (tid < 2)  // nets [cut 0, cut 1): those whose first pin lies in this CTA's run of pins
+        cut[tid] = b + tid == G ? g.nnet
+                                : first_at_least(g.nnet, (int)((long long)np * (b + tid) / G), [&](int k) { return g.kinfo[k].x; });
+    else if (tid < 4)  // nodes [cut 2, cut 3) likewise
+        cut[tid] = b + tid - 2 == G ? g.nn
+                                    : first_at_least(g.nn, (int)((long long)nq * (b + tid - 2) / G),
+                                                     [&](int c) { return g.obj_pin_start[c]; });
+    __syncthreads();
+    const int k0 = cut[0], k1 = cut[1], c0 = cut[2], c1 = cut[3];
+    const int p0 = k0 < g.nnet ? g.kinfo[k0].x : np, p1 = k1 < g.nnet ? g.kinfo[k1].x : np;
+    const int q0 = g.obj_pin_start[c0], q1 = g.obj_pin_start[c1];
+    for (int i = tid; i < p1 - p0; i += kDiffThreads) net_idx[i] = g.pin_node[p0 + i];
+    for (int i = tid; i < q1 - q0; i += kDiffThreads) node_idx[i] = g.q_net[q0 + i];
+    // the terminals' coordinates stay
+    for (int c = g.nn + b * kDiffThreads + tid; c < g.N; c += G * kDiffThreads)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            X[(size_t)c * kF + 3 + 2 * j] = v[c].x;
+            X[(size_t)c * kF + 4 + 2 * j] = v[c].y;
+        }
+    const int kb = min(max(g.n_big, k0), k1);  // nets [k0, kb) of this CTA take a warp each
+    // a thread's first rows, the same in every step
+    constexpr int kKept = 2;
+    int4 net[kKept];
+    int node_s[kKept], node_e[kKept];
+    float node_inv[kKept];
+#pragma unroll
+    for (int u = 0; u < kKept; u++) {
+        const int k = kb + tid + u * kDiffThreads, c = c0 + tid + u * kDiffThreads;
+        net[u] = k < k1 ? g.kinfo[k] : make_int4(0, 0, 0, 0);
+        node_s[u] = c < c1 ? g.obj_pin_start[c] - q0 : 0;
+        node_e[u] = c < c1 ? g.obj_pin_start[c + 1] - q0 : 0;
+        node_inv[u] = c < c1 ? inv_pins[c] : 0.f;
+    }
+    __syncthreads();
+    unsigned target = 0;
+    bool ok = true;
+    for (int step = 1; step <= kDiff3; step++) {
+        gather_pins(net_idx, p1 - p0, v, val);
+        for (int k = k0 + wid; k < kb; k += kDiffThreads / 32) {
+            const int4 r = g.kinfo[k];
+            float sx = 0.f, sy = 0.f;
+            for (int p = r.x - p0 + lane, e = r.x - p0 + r.y; p < e; p += 32) {
+                const float2 t = val[skew(p)];
+                sx += t.x;
+                sy += t.y;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sx += __shfl_xor_sync(0xffffffffu, sx, o);
+                sy += __shfl_xor_sync(0xffffffffu, sy, o);
+            }
+            const float inv = __int_as_float(r.z);
+            if (lane == 0) a[r.w] = make_float2(sx * inv, sy * inv);
+        }
+        auto sum_net = [&](const int4 r) {
+            float sx = 0.f, sy = 0.f;
+#pragma unroll 4
+            for (int p = r.x - p0, e = p + r.y; p < e; p++) {
+                const float2 t = val[skew(p)];
+                sx += t.x;
+                sy += t.y;
+            }
+            const float inv = __int_as_float(r.z);
+            a[r.w] = make_float2(sx * inv, sy * inv);
+        };
+#pragma unroll
+        for (int u = 0; u < kKept; u++)
+            if (kb + tid + u * kDiffThreads < k1) sum_net(net[u]);
+        for (int k = kb + tid + kKept * kDiffThreads; k < k1; k += kDiffThreads) sum_net(g.kinfo[k]);
+        ok = grid_barrier(count, target += G);
+        if (!ok) break;
+        gather_pins(node_idx, q1 - q0, a, val);
+        const int col = step == kDiff1 ? 3 : step == kDiff2 ? 5 : step == kDiff3 ? 7 : 0;
+        auto sum_node = [&](int c, int s, int e, float inv) {
+            float2 t = make_float2(0.5f, 0.5f);  // a node on no net stays at the centre
+            if (e > s) {
+                float sx = 0.f, sy = 0.f;
+#pragma unroll 4
+                for (int q = s; q < e; q++) {
+                    const float2 w = val[skew(q)];
+                    sx += w.x;
+                    sy += w.y;
+                }
+                t = make_float2(sx * inv, sy * inv);
+                v[c] = t;
+            }
+            if (col) {
+                X[(size_t)c * kF + col] = t.x;
+                X[(size_t)c * kF + col + 1] = t.y;
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < kKept; u++) {
+            const int c = c0 + tid + u * kDiffThreads;
+            if (c < c1) sum_node(c, node_s[u], node_e[u], node_inv[u]);
+        }
+        for (int c = c0 + tid + kKept * kDiffThreads; c < c1; c += kDiffThreads)
+            sum_node(c, g.obj_pin_start[c] - q0, g.obj_pin_start[c + 1] - q0, inv_pins[c]);
+        if (step == kDiff3) break;
+        ok = grid_barrier(count, target += G);
+        if (!ok) break;
+    }
+    if (!ok && tid == 0) {
+        *(volatile int *)status = 1;  // mapped host memory: a plain store
+        atomicOr(engine_status, 1 << EP_ERR_TIMEOUT);
+    }
+}
+
 // ------------------------------------------------------ aggregations ------
 // One warp per row, a float2 of channels per lane.  k_net_mean: the first
 // n_big blocks take the nets above kWarpPins pins, a block each (warp w sums
@@ -1037,6 +1223,8 @@ struct ep_gnn {
     int *tc_flag_h = nullptr, *tc_flag_d = nullptr;  // mapped: EP_ERR_TIMEOUT bit of the tensor-core layers
     unsigned tc_wait_limit = tc::kWaitLimit;          // polls of their mbarrier wait (ep_gnn_set_wait_limit)
     int sms = 148;
+    int cooperative = 0;         // the device takes cooperative launches
+    unsigned *barrier = nullptr;  // the diffusion's arrival count
     double *loss = nullptr;
     int64_t step = 0;
     // bound netlist
@@ -1082,6 +1270,7 @@ void set_smem_attrs() {
     done.push_back(dev);
     cudaFuncSetAttribute(k_dense<kF, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dense(kF));
     cudaFuncSetAttribute(k_dense_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
+    cudaFuncSetAttribute(k_diffuse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiffSmem);
     cudaFuncSetAttribute(k_dense_dx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDxSmem);
 }
 
@@ -1131,6 +1320,39 @@ ep_status reserve(ep_gnn *g, size_t N, size_t nnet, size_t nt, size_t np) {
     g->capT = nt;
     g->capP = np;
     return EP_OK;
+}
+
+// The diffusion as one cooperative launch; false when the design's share of a CTA
+// does not fit or the device cannot, and the passes have to go one by one.
+bool diffuse_at_once(ep_gnn *g, ep_status &status) {
+    const EngineGraph &eg = g->eg;
+    // enough pins for every CTA to be worth its place at the barrier
+    const int G = std::max(1, std::min(g->sms, (eg.np + 255) / 256));
+    const DiffShare share{eg.np / G + 1 + eg.max_net_pins, eg.np / G + 1 + eg.max_node_pins};
+    if (!g->cooperative || diff_smem(share) > kDiffSmem) return false;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(G);
+    cfg.blockDim = dim3(kDiffThreads);
+    cfg.dynamicSmemBytes = diff_smem(share);
+    cfg.stream = eg.st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t rc = cudaMemsetAsync(g->barrier, 0, sizeof(unsigned), eg.st);
+    if (rc == cudaSuccess)
+        rc = cudaLaunchKernelEx(&cfg, k_diffuse, g->net, eg.np, share, (const float *)g->inv_pins, g->v, g->netv, g->X,
+                                g->barrier, g->tc_flag_d, eg.d_status);
+    if (rc == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device's are ours
+        cudaGetLastError();
+        return false;
+    }
+    if (rc != cudaSuccess) {
+        g->err = std::string("diffusion launch: ") + cudaGetErrorString(rc);
+        status = EP_ERR_CUDA;
+    }
+    return true;
 }
 
 // Bind an engine's netlist: its device arrays, the features (computed on the
@@ -1188,16 +1410,20 @@ ep_status bind(ep_gnn *g, ep_engine *e) {
     }
     k_inv_deg<<<nblk(eg.nnet), kT, 0, st>>>(eg.nnet, eg.d_net_deg, g->inv_deg);
     k_graph_index<<<nblk(std::max(eg.nnet, eg.np)), kT, 0, st>>>(n, eg.np, g->kinfo, g->pin_node, g->q_net);
-    int col = 3;
-    for (int k = 1; k <= kDiff3; k++) {
-        // programmatic serialisation: the next pass's blocks wait resident
-        launch_k(k_diff_net, nblk(31LL * n.n_big + eg.nnet), kT, 0, st, n, (const float2 *)g->v, g->netv);
-        launch_k(k_diff_node, nblk(eg.nn), kT, 0, st, n, (const float *)g->inv_pins, (const float2 *)g->netv, g->v);
-        if (k == kDiff1 || k == kDiff2 || k == kDiff3) {
-            launch_k(k_store_feature, nblk(N), kT, 0, st, N, (const float2 *)g->v, g->X, col);
-            col += 2;
+    ep_status ds = EP_OK;
+    if (!diffuse_at_once(g, ds)) {
+        int col = 3;
+        for (int k = 1; k <= kDiff3; k++) {
+            // programmatic serialisation: the next pass's blocks wait resident
+            launch_k(k_diff_net, nblk(31LL * n.n_big + eg.nnet), kT, 0, st, n, (const float2 *)g->v, g->netv);
+            launch_k(k_diff_node, nblk(eg.nn), kT, 0, st, n, (const float *)g->inv_pins, (const float2 *)g->netv, g->v);
+            if (k == kDiff1 || k == kDiff2 || k == kDiff3) {
+                launch_k(k_store_feature, nblk(N), kT, 0, st, N, (const float2 *)g->v, g->X, col);
+                col += 2;
+            }
         }
     }
+    if (ds) return ds;
     GK(cudaGetLastError());
     g->uid = eg.uid;
     return EP_OK;
@@ -1223,7 +1449,7 @@ ep_status bind_pads(ep_gnn *g) {
 ep_status tc_give_up(ep_gnn *g) {
     if (!*(volatile int *)g->tc_flag_h) return EP_OK;
     *(volatile int *)g->tc_flag_h = 0;
-    g->err = "a bounded wait of the tensor-core dense layers gave up";
+    g->err = "a bounded wait of the network's kernels gave up";
     return EP_ERR_TIMEOUT;
 }
 
@@ -1325,6 +1551,7 @@ ep_status ep_gnn_create(int32_t device, uint64_t seed, ep_gnn **out) try {
         cudaMalloc(&g->wb, sizeof(__nv_bfloat16) * kParams) != cudaSuccess ||
         cudaMalloc(&g->wt, sizeof(float) * kWtSize) != cudaSuccess ||
         cudaMalloc(&g->loss, sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&g->barrier, sizeof(unsigned)) != cudaSuccess ||
         cudaHostAlloc(&g->tc_flag_h, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&g->tc_flag_d, g->tc_flag_h, 0) != cudaSuccess) {
         g->err = "cudaMalloc failed for the network's weights";
@@ -1332,6 +1559,7 @@ ep_status ep_gnn_create(int32_t device, uint64_t seed, ep_gnn **out) try {
     }
     *g->tc_flag_h = 0;
     cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, device);
+    cudaDeviceGetAttribute(&g->cooperative, cudaDevAttrCooperativeLaunch, device);
     // Glorot-uniform weights, zero biases; the output layer starts small so
     // the first predictions stay near the diffusion coordinates
     std::vector<float> w(kParams, 0.f);
@@ -1354,7 +1582,7 @@ void ep_gnn_destroy(ep_gnn *g) {
     cudaDeviceSynchronize();
     for (void *p : g->ws) cudaFree(p);
     for (void *p : {(void *)g->w, (void *)g->grad, (void *)g->adam_m, (void *)g->adam_v, (void *)g->wb,
-                    (void *)g->wt, (void *)g->loss})
+                    (void *)g->wt, (void *)g->loss, (void *)g->barrier})
         if (p) cudaFree(p);
     if (g->tc_flag_h) cudaFreeHost(g->tc_flag_h);
     delete g;
