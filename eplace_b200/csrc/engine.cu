@@ -77,6 +77,7 @@ struct ep_engine {
     unsigned long long *node_q = nullptr, *filler_q = nullptr;
     DevScalars *S = nullptr;
     DevScalars *hS = nullptr;  // pinned mirror
+    int *progress = nullptr;   // behind it: the running stage's progress, written by the device
     // device memory: buffers are carved from a few large chunks (one
     // cudaMalloc per chunk, chunks doubling from 4 MiB), freed together
     std::vector<void *> allocs;
@@ -380,13 +381,13 @@ void enqueue_loop_step(ep_engine *e) {
     }
     enqueue_eval_to(e, 1, e->g, e->g_prev, e->y_prev, false);
     launch_update_scatter(e->kc, e->dn, e->pos, e->x, e->g, e->y_prev, e->g_prev, e->node_q, e->S,
-                          e->st);
+                          e->progress, e->st);
     e->launches += 1;
 }
 
 void enqueue_step(ep_engine *e) {
     enqueue_eval(e, 1);
-    launch_update(e->kc, e->dn, e->pos, e->x, e->g, e->y_prev, e->g_prev, e->S, e->st);
+    launch_update(e->kc, e->dn, e->pos, e->x, e->g, e->y_prev, e->g_prev, e->S, e->progress, e->st);
     e->launches += 1;
 }
 
@@ -1114,8 +1115,10 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
     CK(cudaMemset(e->y_prev, 0, v2 * no));
     CK(cudaMemset(e->x, 0, v2 * no));
     CK(cudaMemset(e->pin_grad, 0, v2 * std::max(np, 1)));
-    CK(cudaMallocHost((void **)&e->hS, sizeof(DevScalars)));
-    std::memset(e->hS, 0, sizeof(DevScalars));
+    constexpr size_t kMirror = (sizeof(DevScalars) + 255) & ~(size_t)255;
+    CK(cudaMallocHost((void **)&e->hS, kMirror + sizeof(int)));
+    std::memset(e->hS, 0, kMirror + sizeof(int));
+    e->progress = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(e->hS) + kMirror);
     e->hS->a = 1.0;
     e->hS->stage = EP_STAGE_MGP;
     e->hS->max_iter = P.max_iterations > 0 ? P.max_iterations : 1000;
@@ -1299,9 +1302,13 @@ ep_status ep_get_positions(ep_engine *e, int32_t view, float *xy, int32_t count)
     ep_status s = check_view(e, view, count);
     if (s) return s;
     if (count == 0) return EP_OK;
-    gather_view(e, view, e->pos, count);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(xy, e->staging, sizeof(float2) * count, cudaMemcpyDeviceToHost, e->st));
+    const void *src = e->pos;
+    if (view != EP_STAGE_MGP || e->fp64) {  // the mGP view is every object in order
+        gather_view(e, view, e->pos, count);
+        CK(cudaGetLastError());
+        src = e->staging;
+    }
+    CK(cudaMemcpyAsync(xy, src, sizeof(float2) * count, cudaMemcpyDeviceToHost, e->st));
     CK(cudaStreamSynchronize(e->st));
     return EP_OK;
 }
@@ -1336,16 +1343,10 @@ ep_status ep_eval_gradient(ep_engine *e) {
 
 ep_status ep_initialize(ep_engine *e) try {
     if (!e) return EP_ERR_ARG;
-    ep_status s = update_scalars(e, [](DevScalars &h) {
-        h.lambda0_mode = 1;
-        h.lambda = 0.0;
-        h.status = 0;
-        h.done = 0;
-    });
-    if (s) return s;
+    launch_set_scalars(e->S, ScalarSet::kInitialize, 0.0, e->st);
     enqueue_eval(e, 0);
     CK(cudaGetLastError());
-    s = fetch_scalars(e);
+    ep_status s = fetch_scalars(e);
     if (s) return s;
     e->initialized = true;
     return device_status(e);
@@ -1358,9 +1359,13 @@ ep_status ep_get_gradient(ep_engine *e, int32_t view, float *xy, int32_t count) 
     ep_status s = check_view(e, view, count);
     if (s) return s;
     if (count == 0) return EP_OK;
-    gather_view(e, view, e->g, count);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(xy, e->staging, sizeof(float2) * count, cudaMemcpyDeviceToHost, e->st));
+    const void *src = e->g;
+    if (view != EP_STAGE_MGP || e->fp64) {
+        gather_view(e, view, e->g, count);
+        CK(cudaGetLastError());
+        src = e->staging;
+    }
+    CK(cudaMemcpyAsync(xy, src, sizeof(float2) * count, cudaMemcpyDeviceToHost, e->st));
     CK(cudaStreamSynchronize(e->st));
     return EP_OK;
 }
@@ -1428,6 +1433,11 @@ ep_status ep_get_positions_f64(ep_engine *e, int32_t view, double *xy, int32_t c
     ep_status s = check_view(e, view, count);
     if (s) return s;
     if (count == 0) return EP_OK;
+    if (view == EP_STAGE_MGP && e->fp64) {
+        CK(cudaMemcpyAsync(xy, e->pos, sizeof(double2) * count, cudaMemcpyDeviceToHost, e->st));
+        CK(cudaStreamSynchronize(e->st));
+        return EP_OK;
+    }
     if (!e->staging64 && (s = dalloc(e, e->staging64, e->n_obj))) return s;
     const int32_t *idx = e->view_idx[view];
     if (e->fp64)
@@ -1560,18 +1570,20 @@ ep_status ep_query(ep_engine *e, ep_scalars *out) {
 
 ep_status ep_set_lambda(ep_engine *e, double lambda) {
     if (!e) return EP_ERR_ARG;
-    return update_scalars(e, [lambda](DevScalars &h) { h.lambda = lambda; });
+    launch_set_scalars(e->S, ScalarSet::kLambda, lambda, e->st);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(e->st));
+    return EP_OK;
 }
 
 ep_status ep_penalty_init(ep_engine *e) {
     // lambda_0 from the component gradients of the last evaluation needs them
     // resident; the engine computes it inside ep_initialize's evaluation.
     if (!e) return EP_ERR_ARG;
-    ep_status s = update_scalars(e, [](DevScalars &h) { h.lambda0_mode = 1; });
-    if (s) return s;
+    launch_set_scalars(e->S, ScalarSet::kLambda0, 0.0, e->st);
     enqueue_eval(e, 0);
     CK(cudaGetLastError());
-    s = fetch_scalars(e);
+    ep_status s = fetch_scalars(e);
     if (s) return s;
     return device_status(e);
 }
@@ -1646,19 +1658,25 @@ ep_status ep_switch_stage(ep_engine *e, int32_t stage, const float *filler_xy) t
     return host_oom(e);
 }
 
-ep_status ep_nesterov_begin(ep_engine *e) {
-    if (!e) return EP_ERR_ARG;
+extern "C++" {
+// EplaceNesterovOpt::init, the stage's step limit with it (0: none).
+static ep_status begin_stage(ep_engine *e, int step_cap) {
     if (!e->initialized) {
         e->err = "ep_initialize must run before the optimizer";
         return EP_ERR_STATE;
     }
-    ep_status s = update_scalars(e, [](DevScalars &h) { h.step_cap = 0; });
-    if (s) return s;
-    launch_stage_begin(e->kc, e->dn, e->pos, e->x, e->S, e->st);
+    *(volatile int *)e->progress = -1;
+    launch_stage_begin(e->kc, e->dn, e->pos, e->x, step_cap, e->S, e->progress, e->st);
     e->launches += 1;
     CK(cudaGetLastError());
     e->in_run = true;
     return EP_OK;
+}
+}  // extern "C++"
+
+ep_status ep_nesterov_begin(ep_engine *e) {
+    if (!e) return EP_ERR_ARG;
+    return begin_stage(e, 0);
 }
 
 ep_status ep_nesterov_step(ep_engine *e, int32_t *stopped) try {
@@ -1712,14 +1730,13 @@ struct RunState {
     int K = 8;
     bool bktrk = false;
     int64_t launches0 = 0;
-    int cap = 0, launched = 0;
+    int cap = 0, launched = 0, max_steps = 0;
 };
 
 ep_status run_start(ep_engine *e, int32_t max_steps, RunState &r) {
-    ep_status s = ep_nesterov_begin(e);
+    ep_status s = begin_stage(e, max_steps > 0 ? max_steps : 0);
     if (s) return s;
-    s = update_scalars(e, [max_steps](DevScalars &h) { h.step_cap = max_steps > 0 ? max_steps : 0; });
-    if (s) return s;
+    r.max_steps = max_steps > 0 ? max_steps : 0;
     r.bktrk = e->prm.step_rule == EP_STEP_BKTRK;
     if (!r.bktrk && (!e->graph || e->graph_iters != r.K)) {
         s = build_graph(e, r.K);
@@ -1737,8 +1754,8 @@ ep_status run_start(ep_engine *e, int32_t max_steps, RunState &r) {
     return EP_OK;
 }
 
-// Enqueue the next K steps (one graph replay) and the read-back of `done`;
-// backtracking steps run one at a time from the host.
+// Enqueue the next K steps (one graph replay); backtracking steps run one at a
+// time from the host.
 ep_status run_launch(ep_engine *e, RunState &r) {
     if (r.bktrk) {
         ep_status s = fetch_scalars(e);
@@ -1749,18 +1766,43 @@ ep_status run_launch(ep_engine *e, RunState &r) {
     CK(cudaGraphLaunch(e->graph, e->st));
     e->launches += e->graph_kernels;
     r.launched += r.K;
-    CK(cudaMemcpyAsync(&e->hS->done, &e->S->done, sizeof(int), cudaMemcpyDeviceToHost, e->st));
-    CK(cudaEventRecord(e->ev_poll, e->st));
     return EP_OK;
 }
 
+// Whether another replay is wanted.  The device writes its progress into host
+// memory at the end of every step; the host waits until kAhead steps are left
+// of what it enqueued, so that the next replay is there before the device runs
+// dry (a read-back after each replay left it idle for some 15 us).  A stage that
+// stops within those steps costs one replay of kernels that return at once.
 ep_status run_check(ep_engine *e, RunState &r, bool &more) {
+    constexpr int kAhead = 2;
     if (r.bktrk) {
         more = !e->hS->done && r.launched <= r.cap;
         return EP_OK;
     }
-    CK(cudaEventSynchronize(e->ev_poll));
-    more = !(e->hS->done || r.launched > r.cap + r.K);
+    if (r.max_steps > 0 && r.launched >= r.max_steps) {  // the device stops at the limit by itself
+        more = false;
+        return EP_OK;
+    }
+    for (unsigned spins = 0;; spins++) {
+        const int p = *(volatile int *)e->progress;
+        if (p >= 0 && (p & kProgressDone)) {
+            more = false;
+            return EP_OK;
+        }
+        if (p >= 0 && p >= r.launched - kAhead) break;
+        if ((spins & 1023) == 1023) {
+            // an error ends the wait, and so does a stream with nothing left to do
+            const cudaError_t q = cudaStreamQuery(e->st);
+            if (q == cudaSuccess) {
+                more = !(*(volatile int *)e->progress & kProgressDone) && r.launched <= r.cap + r.K;
+                return EP_OK;
+            }
+            if (q != cudaErrorNotReady) CK(q);
+            std::this_thread::yield();
+        }
+    }
+    more = r.launched <= r.cap + r.K;
     return EP_OK;
 }
 
@@ -1770,8 +1812,7 @@ ep_status run_finish(ep_engine *e, RunState &r, ep_run_stats *stats) {
         // scatters (the stopping step scatters nothing, so this is a no-op
         // unless the loop was cut off)
         const size_t nb = (size_t)e->grid.nx * e->grid.ny;
-        CK(cudaMemsetAsync(e->node_q, 0, sizeof(unsigned long long) * nb, e->st));
-        CK(cudaMemsetAsync(e->filler_q, 0, sizeof(unsigned long long) * nb, e->st));
+        CK(cudaMemsetAsync(e->node_q, 0, 2 * sizeof(unsigned long long) * nb, e->st));  // both maps
     }
     enqueue_hpwl(e, 2);  // the lambda update owed by the last step
     launch_wrap_up(e->kc, e->dn, e->pos, e->x, e->st);
@@ -2070,7 +2111,7 @@ ep_status ep_time_kernels(ep_engine *e, int32_t reps, ep_kernel_times *out) try 
               }, nothing);
     if (s) return s;
     s = timed("update", 1, (9.0 + 56.0 * q) * nobj, 0.0,
-              [&] { launch_update(e->kc, d, e->pos, e->x, e->g, e->y_prev, e->g_prev, e->S, e->st); },
+              [&] { launch_update(e->kc, d, e->pos, e->x, e->g, e->y_prev, e->g_prev, e->S, e->progress, e->st); },
               [&] {
                   // a pending stop would make the following repetitions no-ops
                   cudaMemsetAsync(&e->S->stop_pending, 0, sizeof(int), e->st);

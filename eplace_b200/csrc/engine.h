@@ -165,18 +165,26 @@ void launch_combine(const KernelCtx &c, const DeviceNetlist &d, const void *fiel
                     const void *g_prev, const void *y_prev, void *dump_gd, void *dump_gwl, int stepping, DevScalars *S,
                     cudaStream_t st);
 void launch_update(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g, void *y_prev,
-                   void *g_prev, DevScalars *S, cudaStream_t st);
+                   void *g_prev, DevScalars *S, int *progress, cudaStream_t st);
 // The update of the captured loop: also scatters the new positions into the
 // (clear) density maps for the next evaluation, unless the step ends the stage.
 void launch_update_scatter(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
-                           void *y_prev, void *g_prev, unsigned long long *maps, DevScalars *S, cudaStream_t st);
+                           void *y_prev, void *g_prev, unsigned long long *maps, DevScalars *S, int *progress,
+                           cudaStream_t st);
 // Backtracking step rule: one trial move from y_k (ysave) along g_k, and the
 // scalar commit of an accepted trial (combine in stepping mode 2 decides).
 void launch_bktrk_move(const KernelCtx &c, const DeviceNetlist &d, const void *ysave, const void *g, const void *x,
                        void *pos, void *xtrial, const DevScalars *S, cudaStream_t st);
 void launch_bktrk_commit(DevScalars *S, cudaStream_t st);
-void launch_stage_begin(const KernelCtx &c, const DeviceNetlist &d, const void *pos, void *x, DevScalars *S,
-                        cudaStream_t st);
+void launch_stage_begin(const KernelCtx &c, const DeviceNetlist &d, const void *pos, void *x, int step_cap,
+                        DevScalars *S, int *progress, cudaStream_t st);
+// Scalars set in stream order: kInitialize (initialization()'s start), kLambda0
+// (the next evaluation makes lambda_0), kLambda (value).
+enum class ScalarSet { kInitialize, kLambda0, kLambda };
+void launch_set_scalars(DevScalars *S, ScalarSet what, double value, cudaStream_t st);
+// The word of host memory that a run's kernels keep: steps taken, and this bit
+// once the stage has ended.
+constexpr int kProgressDone = 1 << 30;
 void launch_wrap_up(const KernelCtx &c, const DeviceNetlist &d, void *pos, const void *x, cudaStream_t st);
 // HPWL at the current positions; mode 0 stores it, mode 1 also applies the
 // updatePenaltyFactor rule, mode 2 applies it only if a lambda update is pending.

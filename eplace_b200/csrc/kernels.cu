@@ -1163,27 +1163,39 @@ __device__ __forceinline__ vec2<R> nesterov_move(const Grid &g, int o, R s, R c,
     return p;
 }
 
-// The scalar side of the end of a step (last block of the update).
-__device__ __forceinline__ void end_step(DevScalars *S) {
-    S->iter += 1;
+// The scalar side of the end of a step (last block of the update), from scalars
+// its thread loaded at the kernel's start.  progress: host memory (mapped) that
+// the host watches during a run: steps taken, kProgressDone once the stage has
+// ended.
+struct StepEnd {
+    int iter, stop_pending, stage;
+};
+__device__ __forceinline__ StepEnd load_step_end(const DevScalars *S) {
+    return StepEnd{S->iter, S->stop_pending, S->stage};
+}
+__device__ __forceinline__ void end_step(DevScalars *S, const StepEnd &e, volatile int *progress) {
+    const int iter = e.iter + 1;
+    S->iter = iter;
     S->lambda_pending = 1;
-    if (S->stop_pending) {
+    if (e.stop_pending) {
         S->done = 1;
-        if (S->stage == EP_STAGE_MGP) S->mgp_iterations = S->iter;
+        if (e.stage == EP_STAGE_MGP) S->mgp_iterations = iter;
     }
+    *progress = iter | (e.stop_pending ? kProgressDone : 0);
 }
 
 template <typename R>
 __global__ void __launch_bounds__(kThreads)
 k_update(Grid g, int n, const uint8_t *__restrict__ flags, const float2 *__restrict__ size, vec2<R> *__restrict__ pos,
          vec2<R> *__restrict__ x, const vec2<R> *__restrict__ gin, vec2<R> *__restrict__ y_prev,
-         vec2<R> *__restrict__ g_prev, DevScalars *__restrict__ S) {
+         vec2<R> *__restrict__ g_prev, DevScalars *__restrict__ S, int *progress) {
     pdl_begin();
     if (S->done) return;
+    const StepEnd end = load_step_end(S);
     int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o < n && (flags[o] & kInView))
         nesterov_move<R>(g, o, (R)S->step, (R)S->coef, size[o], pos, x, gin, y_prev, g_prev);
-    if (threadIdx.x == 0 && last_block(&S->cnt_upd, gridDim.x)) end_step(S);
+    if (threadIdx.x == 0 && last_block(&S->cnt_upd, gridDim.x)) end_step(S, end, progress);
 }
 
 // The update of the captured loop, with the next evaluation's scatter fused
@@ -1198,7 +1210,7 @@ template <int MINB, typename R>
 __global__ void __launch_bounds__(kThreads, MINB)
 k_update_scatter(Grid g, DeviceNetlist d, int big_blocks, vec2<R> *__restrict__ pos, vec2<R> *__restrict__ x,
                  const vec2<R> *__restrict__ gin, vec2<R> *__restrict__ y_prev, vec2<R> *__restrict__ g_prev,
-                 double qscale, ull *__restrict__ maps, DevScalars *__restrict__ S) {
+                 double qscale, ull *__restrict__ maps, DevScalars *__restrict__ S, int *progress) {
     __shared__ vec2<R> big_pos[kThreads / 32];
     const ObjectUnit u = object_unit(d, big_blocks);
     const bool valid = u.o < d.n_obj;
@@ -1208,7 +1220,8 @@ k_update_scatter(Grid g, DeviceNetlist d, int big_blocks, vec2<R> *__restrict__ 
     pdl_begin();
     if (S->done) return;
     const R s = (R)S->step, c = (R)S->coef;
-    const bool scatter = !S->stop_pending;
+    const StepEnd end = load_step_end(S);
+    const bool scatter = !end.stop_pending;
     auto move = [&] {
         return (f & kInView) ? nesterov_move<R>(g, u.o, s, c, sz, pos, x, gin, y_prev, g_prev) : pos[u.o];
     };
@@ -1222,7 +1235,7 @@ k_update_scatter(Grid g, DeviceNetlist d, int big_blocks, vec2<R> *__restrict__ 
         __syncthreads();  // block-uniform: every unit of this block has several threads
         if (valid && scatter) scatter_big<R>(g, big_pos[slot], sz, sxy, f, qscale, u.rank, u.count, maps);
     }
-    if (threadIdx.x == 0 && last_block(&S->cnt_upd, gridDim.x)) end_step(S);
+    if (threadIdx.x == 0 && last_block(&S->cnt_upd, gridDim.x)) end_step(S, end, progress);
 }
 
 // Backtracking trial move (opt_step_bktrk, Optimization/nesterov.hpp:337-349):
@@ -1264,7 +1277,7 @@ __global__ void k_bktrk_commit(DevScalars *__restrict__ S) {
 // EplaceNesterovOpt::init (nesterov.hpp:207-214): x_0 = current positions.
 template <typename R>
 __global__ void k_stage_begin(int n, const uint8_t *__restrict__ flags, const vec2<R> *__restrict__ pos,
-                              vec2<R> *__restrict__ x, DevScalars *__restrict__ S) {
+                              vec2<R> *__restrict__ x, int step_cap, DevScalars *__restrict__ S, int *progress) {
     pdl_begin();
     for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < n; o += gridDim.x * blockDim.x)
         if (flags[o] & kInView) x[o] = pos[o];
@@ -1283,7 +1296,25 @@ __global__ void k_stage_begin(int n, const uint8_t *__restrict__ flags, const ve
         else
             stop = tau < (double)0.07f;
         S->done = stop;
+        S->step_cap = step_cap;
         if (stop && S->stage == EP_STAGE_MGP) S->mgp_iterations = 0;
+        *(volatile int *)progress = stop ? kProgressDone : 0;
+    }
+}
+
+// Scalars that a call sets before its kernels, in stream order (a read-back, a
+// change on the host and a copy cost two synchronisations).
+__global__ void k_set_scalars(DevScalars *__restrict__ S, ScalarSet what, double value) {
+    pdl_begin();
+    if (what == ScalarSet::kLambda) {
+        S->lambda = value;
+        return;
+    }
+    S->lambda0_mode = 1;  // the next evaluation is initialization()'s
+    if (what == ScalarSet::kInitialize) {
+        S->lambda = 0.0;
+        S->status = 0;
+        S->done = 0;
     }
 }
 
@@ -1347,18 +1378,18 @@ void launch_scatter(const KernelCtx &c, const DeviceNetlist &d, ull *maps, const
 
 template <typename R>
 static void update_scatter_t(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
-                             void *y_prev, void *g_prev, ull *maps, DevScalars *S, cudaStream_t st) {
+                             void *y_prev, void *g_prev, ull *maps, DevScalars *S, int *progress, cudaStream_t st) {
     const int bb = big_blocks(d);
     const int blocks = bb + blocks_for(d.n_obj, kThreads);
     constexpr int kMany = sizeof(R) == 8 ? 5 : 6;
     launch_k(blocks <= kSms * 4 ? k_update_scatter<1, R> : k_update_scatter<kMany, R>, blocks, kThreads, 0, st, c.grid,
-             d, bb, V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), c.qscale, maps, S);
+             d, bb, V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), c.qscale, maps, S, progress);
 }
 
 void launch_update_scatter(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
-                           void *y_prev, void *g_prev, ull *maps, DevScalars *S, cudaStream_t st) {
-    c.fp64 ? update_scatter_t<double>(c, d, pos, x, g, y_prev, g_prev, maps, S, st)
-           : update_scatter_t<float>(c, d, pos, x, g, y_prev, g_prev, maps, S, st);
+                           void *y_prev, void *g_prev, ull *maps, DevScalars *S, int *progress, cudaStream_t st) {
+    c.fp64 ? update_scatter_t<double>(c, d, pos, x, g, y_prev, g_prev, maps, S, progress, st)
+           : update_scatter_t<float>(c, d, pos, x, g, y_prev, g_prev, maps, S, progress, st);
 }
 
 void launch_prep(const KernelCtx &c, ull *node_q, ull *filler_q, const float2 *static_map, void *rho,
@@ -1419,15 +1450,15 @@ void launch_combine(const KernelCtx &c, const DeviceNetlist &d, const void *fiel
 
 template <typename R>
 static void update_t(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g, void *y_prev,
-                     void *g_prev, DevScalars *S, cudaStream_t st) {
+                     void *g_prev, DevScalars *S, int *progress, cudaStream_t st) {
     launch_k(k_update<R>, blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d.n_obj, d.flags, d.size,
-             V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), S);
+             V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), S, progress);
 }
 
 void launch_update(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g, void *y_prev,
-                   void *g_prev, DevScalars *S, cudaStream_t st) {
-    c.fp64 ? update_t<double>(c, d, pos, x, g, y_prev, g_prev, S, st)
-           : update_t<float>(c, d, pos, x, g, y_prev, g_prev, S, st);
+                   void *g_prev, DevScalars *S, int *progress, cudaStream_t st) {
+    c.fp64 ? update_t<double>(c, d, pos, x, g, y_prev, g_prev, S, progress, st)
+           : update_t<float>(c, d, pos, x, g, y_prev, g_prev, S, progress, st);
 }
 
 template <typename R>
@@ -1445,13 +1476,19 @@ void launch_bktrk_move(const KernelCtx &c, const DeviceNetlist &d, const void *y
 
 void launch_bktrk_commit(DevScalars *S, cudaStream_t st) { launch_k(k_bktrk_commit, 1, 1, 0, st, S); }
 
-void launch_stage_begin(const KernelCtx &c, const DeviceNetlist &d, const void *pos, void *x, DevScalars *S,
-                        cudaStream_t st) {
-    const int blocks = std::min(blocks_for(d.n_obj, kThreads), 148 * 4);
+void launch_stage_begin(const KernelCtx &c, const DeviceNetlist &d, const void *pos, void *x, int step_cap,
+                        DevScalars *S, int *progress, cudaStream_t st) {
+    const int blocks = std::min(blocks_for(d.n_obj, kThreads), kSms * 4);
     if (c.fp64)
-        launch_k(k_stage_begin<double>, blocks, kThreads, 0, st, d.n_obj, d.flags, V<double>(pos), V<double>(x), S);
+        launch_k(k_stage_begin<double>, blocks, kThreads, 0, st, d.n_obj, d.flags, V<double>(pos), V<double>(x),
+                 step_cap, S, progress);
     else
-        launch_k(k_stage_begin<float>, blocks, kThreads, 0, st, d.n_obj, d.flags, V<float>(pos), V<float>(x), S);
+        launch_k(k_stage_begin<float>, blocks, kThreads, 0, st, d.n_obj, d.flags, V<float>(pos), V<float>(x), step_cap,
+                 S, progress);
+}
+
+void launch_set_scalars(DevScalars *S, ScalarSet what, double value, cudaStream_t st) {
+    launch_k(k_set_scalars, 1, 1, 0, st, S, what, value);
 }
 
 void launch_wrap_up(const KernelCtx &c, const DeviceNetlist &d, void *pos, const void *x, cudaStream_t st) {
@@ -1510,7 +1547,7 @@ void set_loop_carveout() {
         done_devices.push_back(dev);
     }
     const int carveout = carveout_percent(kLoopSmemBytes);
-    std::vector<const void *> fns = {(const void *)k_bktrk_commit};
+    std::vector<const void *> fns = {(const void *)k_bktrk_commit, (const void *)k_set_scalars};
     loop_kernels<float>(fns);
     loop_kernels<double>(fns);
     for (const void *f : fns) cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
