@@ -10,7 +10,7 @@
 // of a cell are added by neighbouring lanes.  What bounds it then is the L2's
 // rate of 64-bit adds: 9.5M in 37 us at 1M cells and fillers (42.8 before; 200k
 // 10.7 -> 8.4 us, FP64 12.7 -> 10.5; ep_density_scatter_noalloc with 300k objects
-// 25.3 -> 23.4 us in all).
+// 25.3 -> 23.4 us in all, and 19.2 with its launches overlapped).
 #pragma once
 #include "common.cuh"
 
