@@ -447,10 +447,52 @@ k_diffuse(Net g, int np, DiffShare share, const float *__restrict__ inv_pins, fl
 }
 
 // ------------------------------------------------------ aggregations ------
-// One warp per row, a float2 of channels per lane.  k_net_mean: the first
-// n_big blocks take the nets above kWarpPins pins, a block each (warp w sums
-// pins w, w + 8, ..., the 8 warp sums are added in warp order); the other
-// nets take a warp each.
+// Half a warp per row, a float4 of channels per lane, and the rows of four
+// pins in flight: a pin costs two dependent loads (its row's number, the row),
+// and most rows have two to five pins, so a warp that summed one row pin after
+// pin waited for the L2 most of the time.  A warp per row before, us: at 200k
+// cells k_net_mean 52.2 -> 32.5 and k_node_mean 52.6 -> 41.4, at 50k
+// k_node_mean_t 29.0 -> 15.1 and k_net_mean_t_add 16.2 -> 14.7 (18.9 with the
+// row's load behind its weight's).  What bounds them now is the L2's rate (256
+// bytes a pin) and, at 200k, writing the 51 MB of rows.
+// The nets above kWarpPins pins take the first n_big blocks of the per-net
+// passes, a block each (warp w sums pins w, w + 8, ..., with a float2 per
+// lane; the 8 warp sums are added in warp order).
+constexpr int kHalf = 16;  // lanes per row
+
+// Sum of rows idx[p], idx[p + 1], ..., idx[e - 1] of h, in that order, without
+// the rows from `limit` on; row i times weight[i] (Scaled).
+template <bool Scaled>
+__device__ __forceinline__ float4 sum_rows(const int32_t *__restrict__ idx, int p, int e, int limit,
+                                           const float4 *__restrict__ h, int lane, const float *__restrict__ weight) {
+    constexpr int kU = 4;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (; p < e; p += kU) {
+        int i[kU];
+        float w[kU];
+        float4 t[kU];
+#pragma unroll
+        for (int u = 0; u < kU; u++) i[u] = p + u < e ? idx[p + u] : limit;
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            if (i[u] < limit) {
+                t[u] = h[(size_t)i[u] * kHalf + lane];
+                if (Scaled) w[u] = weight[i[u]];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            if (i[u] < limit) {
+                s.x += Scaled ? t[u].x * w[u] : t[u].x;
+                s.y += Scaled ? t[u].y * w[u] : t[u].y;
+                s.z += Scaled ? t[u].z * w[u] : t[u].z;
+                s.w += Scaled ? t[u].w * w[u] : t[u].w;
+            }
+        }
+    }
+    return s;
+}
+
 constexpr int kBigWarps = kT / 32;
 __global__ void __launch_bounds__(kT) k_net_mean(Net g, const float2 *__restrict__ h,
                                                  float2 *__restrict__ a) {
@@ -478,36 +520,26 @@ __global__ void __launch_bounds__(kT) k_net_mean(Net g, const float2 *__restrict
         }
         return;
     }
-    const int k = g.n_big + ((int)(blockIdx.x - g.n_big) * kBigWarps + w);
+    const int k = g.n_big + ((int)blockIdx.x - g.n_big) * (kT / kHalf) + (int)threadIdx.x / kHalf;
     if (k >= g.nnet) return;
     const int4 r = g.kinfo[k];
-    const int n = r.w;
-    float2 s = make_float2(0.f, 0.f);
-#pragma unroll 4
-    for (int p = r.x, e = r.x + r.y; p < e; p++) {
-        const float2 q = h[(size_t)g.pin_node[p] * 32 + lane];
-        s.x += q.x;
-        s.y += q.y;
-    }
+    const int l = threadIdx.x & (kHalf - 1);
+    const float4 s = sum_rows<false>(g.pin_node, r.x, r.x + r.y, g.N, (const float4 *)h, l, nullptr);
     const float inv = __int_as_float(r.z);
-    a[(size_t)n * 32 + lane] = make_float2(s.x * inv, s.y * inv);
+    ((float4 *)a)[(size_t)r.w * kHalf + l] = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
 }
 
-__global__ void k_node_mean(Net g, const float *__restrict__ inv_pins, const float2 *__restrict__ a,
-                            float2 *__restrict__ m) {
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+__global__ void k_node_mean(Net g, const float *__restrict__ inv_pins, const float4 *__restrict__ a,
+                            float4 *__restrict__ m) {
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) / kHalf, l = threadIdx.x & (kHalf - 1);
     if (c >= g.N) return;
-    float2 s = make_float2(0.f, 0.f);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < g.nn) {
-        for (int q = g.obj_pin_start[c]; q < g.obj_pin_start[c + 1]; q++) {
-            const float2 t = a[(size_t)g.q_net[q] * 32 + lane];
-            s.x += t.x;
-            s.y += t.y;
-        }
-        s.x *= inv_pins[c];
-        s.y *= inv_pins[c];
+        const float inv = inv_pins[c];
+        s = sum_rows<false>(g.q_net, g.obj_pin_start[c], g.obj_pin_start[c + 1], g.nnet, a, l, nullptr);
+        s = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
     }
-    m[(size_t)c * 32 + lane] = s;
+    m[(size_t)c * kHalf + l] = s;
 }
 
 // transpose of node_mean: da[n] = sum over the pins of n on movable nodes c of
@@ -519,18 +551,14 @@ __device__ __forceinline__ void add_scaled(float2 &s, float2 t, float w) {
 __global__ void __launch_bounds__(kT) k_node_mean_t(Net g, const float *__restrict__ inv_pins,
                                                     const float2 *__restrict__ dm, float2 *__restrict__ da) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const bool big = (int)blockIdx.x < g.n_big;
-    const int k = big ? (int)blockIdx.x : g.n_big + ((int)blockIdx.x - g.n_big) * kBigWarps + w;
-    if (k >= g.nnet) return;
-    const int4 r = g.kinfo[k];
-    const int step = big ? kBigWarps : 1;
-    float2 s = make_float2(0.f, 0.f);
+    if ((int)blockIdx.x < g.n_big) {
+        const int4 r = g.kinfo[blockIdx.x];
+        float2 s = make_float2(0.f, 0.f);
 #pragma unroll 4
-    for (int p = r.x + (big ? w : 0), e = r.x + r.y; p < e; p += step) {
-        const int c = g.pin_node[p];
-        if (c < g.nn) add_scaled(s, dm[(size_t)c * 32 + lane], inv_pins[c]);
-    }
-    if (big) {
+        for (int p = r.x + w, e = r.x + r.y; p < e; p += kBigWarps) {
+            const int c = g.pin_node[p];
+            if (c < g.nn) add_scaled(s, dm[(size_t)c * 32 + lane], inv_pins[c]);
+        }
         __shared__ float2 part[kBigWarps][32];
         part[w][lane] = s;
         __syncthreads();
@@ -539,33 +567,28 @@ __global__ void __launch_bounds__(kT) k_node_mean_t(Net g, const float *__restri
             s.x += part[j][lane].x;
             s.y += part[j][lane].y;
         }
+        da[(size_t)r.w * 32 + lane] = s;
+        return;
     }
-    da[(size_t)r.w * 32 + lane] = s;
+    const int k = g.n_big + ((int)blockIdx.x - g.n_big) * (kT / kHalf) + (int)threadIdx.x / kHalf;
+    if (k >= g.nnet) return;
+    const int4 r = g.kinfo[k];
+    const int l = threadIdx.x & (kHalf - 1);
+    ((float4 *)da)[(size_t)r.w * kHalf + l] = sum_rows<true>(g.pin_node, r.x, r.x + r.y, g.nn, (const float4 *)dm, l,
+                                                                    inv_pins);
 }
 
 // transpose of net_mean, added: dh[c] += sum over the pins of node c of da[net] / deg(net)
-__global__ void k_net_mean_t_add(Net g, const float *__restrict__ inv_deg, const float2 *__restrict__ da,
-                                 float2 *__restrict__ dh) {
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+__global__ void k_net_mean_t_add(Net g, const float *__restrict__ inv_deg, const float4 *__restrict__ da,
+                                 float4 *__restrict__ dh) {
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) / kHalf, l = threadIdx.x & (kHalf - 1);
     if (c >= g.N) return;
-    float2 s = make_float2(0.f, 0.f);
-    if (c < g.nn) {
-#pragma unroll 4
-        for (int q = g.obj_pin_start[c], e = g.obj_pin_start[c + 1]; q < e; q++) {
-            const int n = g.q_net[q];
-            add_scaled(s, da[(size_t)n * 32 + lane], inv_deg[n]);
-        }
-    } else {
-        const int t0 = c - g.nn;
-#pragma unroll 4
-        for (int q = g.pad_start[t0], e = g.pad_start[t0 + 1]; q < e; q++) {
-            const int n = g.pad_net[q];
-            add_scaled(s, da[(size_t)n * 32 + lane], inv_deg[n]);
-        }
-    }
-    float2 &o = dh[(size_t)c * 32 + lane];
-    o.x += s.x;
-    o.y += s.y;
+    const bool node = c < g.nn;
+    const int32_t *start = node ? g.obj_pin_start + c : g.pad_start + (c - g.nn);
+    const float4 s = sum_rows<true>(node ? g.q_net : g.pad_net, start[0], start[1], g.nnet, da, l, inv_deg);
+    float4 &o = dh[(size_t)c * kHalf + l];
+    float4 v = o;
+    o = make_float4(v.x + s.x, v.y + s.y, v.z + s.z, v.w + s.w);
 }
 
 // ------------------------------------------------------------ dense -------
@@ -1465,9 +1488,9 @@ ep_status forward(ep_gnn *g) {
     k_dense<kF, 0><<<nblk(N, kDenseRows), kT, smem_dense(kF), st>>>(N, g->X, nullptr, g->wt, w + kOffB0,
                                                                     g->h[0]);
     for (int l = 1; l <= kLayers; l++) {
-        k_net_mean<<<n.n_big + nblk(n.nnet - n.n_big, kBigWarps), kT, 0, st>>>(n, (const float2 *)g->h[l - 1],
-                                                                (float2 *)g->a);
-        k_node_mean<<<nblk((long long)N * 32), kT, 0, st>>>(n, g->inv_pins, (const float2 *)g->a, (float2 *)g->m[l]);
+        k_net_mean<<<n.n_big + nblk(n.nnet - n.n_big, kT / kHalf), kT, 0, st>>>(n, (const float2 *)g->h[l - 1],
+                                                                                (float2 *)g->a);
+        k_node_mean<<<nblk((long long)N * kHalf), kT, 0, st>>>(n, g->inv_pins, (const float4 *)g->a, (float4 *)g->m[l]);
         launch_dense_tc(tc_grid, st, N, g->h[l - 1], g->m[l], wb + off_w(l), w + off_b(l), g->h[l], g->tc_flag_d,
                         g->eg.d_status, g->tc_wait_limit);
     }
@@ -1500,10 +1523,9 @@ ep_status backward(ep_gnn *g) {
         reduce(kH * 2 * kH, kH, off_w(l), off_b(l));
         // d h_{l-1} (direct part) into dx, d m_l into g->dm
         k_dense_dx<<<std::min(nblk(N, kDxRows), 148 * 2), kT, kDxSmem, st>>>(N, dh, g->h[l], wb + off_w(l), dx, g->dm);
-        k_node_mean_t<<<n.n_big + nblk(n.nnet - n.n_big, kBigWarps), kT, 0, st>>>(n, g->inv_pins, (const float2 *)g->dm,
-                                                                                 (float2 *)g->da);
-        k_net_mean_t_add<<<nblk((long long)N * 32), kT, 0, st>>>(n, g->inv_deg, (const float2 *)g->da,
-                                                                 (float2 *)dx);
+        k_node_mean_t<<<n.n_big + nblk(n.nnet - n.n_big, kT / kHalf), kT, 0, st>>>(
+            n, g->inv_pins, (const float2 *)g->dm, (float2 *)g->da);
+        k_net_mean_t_add<<<nblk((long long)N * kHalf), kT, 0, st>>>(n, g->inv_deg, (const float4 *)g->da, (float4 *)dx);
         std::swap(dh, dx);
     }
     // input layer
