@@ -53,10 +53,10 @@ REF_RUNS = os.path.join(ROOT, "tests", "golden", "reference_runs.json")
 SAMPLE_ITERS = 8  # reference optimizer steps of the cpu_baseline sample
 # kernels one ep_gnn_propose launches on a netlist it has not bound: the
 # features (initial values, terminal pin counts and feature, 1/degree, the
-# aggregation indices, 128 diffusion steps of 2 kernels, 3 feature stores),
+# aggregation indices, one cooperative launch for the 128 diffusion steps),
 # the forward pass (input layer, 3 x (net mean, node mean, dense), output),
 # the proposal and the position store
-GNN_LAUNCHES = 5 + 2 * 128 + 3 + 1 + 3 * 3 + 1 + 2
+GNN_LAUNCHES = 5 + 1 + 1 + 3 * 3 + 1 + 2
 
 
 def netlist():
