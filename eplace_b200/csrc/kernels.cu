@@ -159,13 +159,17 @@ k_prep(Grid g, ull *__restrict__ node_q, ull *__restrict__ filler_q, const float
        double *__restrict__ partials, DevScalars *__restrict__ S) {
     pdl_begin();
     __shared__ double sh[32];
-    if (S->done) return;
+    // tested behind the first bin's loads, one round trip for both: a step at 200k
+    // cells 55.6 -> 55.25 us, at 1M the same
+    const int done = S->done;
     int nb = g.nx * g.ny;
     double acc[1] = {0.0};
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nb; k += gridDim.x * blockDim.x) {
-        double node = (double)(long long)node_q[k] * inv_q;
-        double fill = (double)(long long)filler_q[k] * inv_q;
+        const ull nq = node_q[k], fq = filler_q[k];
         float2 st = stat[k];  // (terminal, base)
+        if (done) return;
+        double node = (double)(long long)nq * inv_q;
+        double fill = (double)(long long)fq * inv_q;
         // eDensity = node + base + filler + terminal (EPlace/eplace.cpp:576-577)
         double dens = (node + (double)st.y + fill + (double)st.x) * inv_bin_area;
         R d = (R)dens;
@@ -195,6 +199,7 @@ k_prep(Grid g, ull *__restrict__ node_q, ull *__restrict__ filler_q, const float
             filler_q[k] = 0ull;
         }
     }
+    if (done) return;  // a thread without bins
     if (!grid_arrive<1>(acc, sh, partials, &S->cnt_prep, gridDim.x, blockIdx.x)) return;
     const int status = S->status;
     grid_total<1>(acc, sh, partials, &S->cnt_prep, gridDim.x);
