@@ -1250,6 +1250,7 @@ struct ep_gnn {
     unsigned *barrier = nullptr;  // the diffusion's arrival count
     double *loss = nullptr;
     int64_t step = 0;
+    cudaEvent_t used = nullptr;  // the end of the last call's work on the workspace (Use)
     // bound netlist
     uint64_t uid = 0;         // 0: none
     bool pads_ready = false;  // terminal pin lists uploaded (training)
@@ -1282,6 +1283,34 @@ namespace {
             return EP_ERR_CUDA;                                                   \
         }                                                                         \
     } while (0)
+
+// One call's use of the network's workspace and weights, on its engine's stream.
+// Engines have streams of their own and some calls return with work pending, so
+// a call waits on the device for the one before, and marks its own end whatever
+// it returns.  Not while the stream is being captured, where neither may be.
+class Use {
+  public:
+    explicit Use(ep_gnn *g) : g_(g) {}
+    Use(const Use &) = delete;
+    ep_status begin(cudaStream_t st) {
+        ep_gnn *const g = g_;
+        cudaStreamCaptureStatus capture;
+        GK(cudaStreamIsCapturing(st, &capture));
+        if (capture != cudaStreamCaptureStatusNone) return EP_OK;
+        GK(cudaStreamWaitEvent(st, g->used));
+        st_ = st;
+        begun_ = true;
+        return EP_OK;
+    }
+    ~Use() {
+        if (begun_ && cudaEventRecord(g_->used, st_) != cudaSuccess) cudaStreamSynchronize(st_);
+    }
+
+  private:
+    ep_gnn *g_;
+    cudaStream_t st_ = nullptr;
+    bool begun_ = false;
+};
 
 size_t smem_dense(int K) { return sizeof(float) * ((size_t)K * kH + (size_t)kDenseRows * (K + 1)); }
 
@@ -1380,7 +1409,7 @@ bool diffuse_at_once(ep_gnn *g, ep_status &status) {
 
 // Bind an engine's netlist: its device arrays, the features (computed on the
 // engine's stream) -- skipped when the workspace already holds them.
-ep_status bind(ep_gnn *g, ep_engine *e) {
+ep_status bind(ep_gnn *g, ep_engine *e, Use &use) {
     EngineGraph eg{};
     if (engine_graph(e, &eg)) return EP_ERR_ARG;
     if (eg.nn <= 0 || eg.nnet <= 0) {
@@ -1391,13 +1420,15 @@ ep_status bind(ep_gnn *g, ep_engine *e) {
         g->err = "the engine lives on another device than the network";
         return EP_ERR_ARG;
     }
+    ep_status s = use.begin(eg.st);
+    if (s) return s;
     if (g->uid == eg.uid) {
         g->eg = eg;
         return EP_OK;
     }
     set_smem_attrs();
     const int N = eg.nn + eg.nt;
-    ep_status s = reserve(g, N, eg.nnet, eg.nt, eg.np);
+    s = reserve(g, N, eg.nnet, eg.nt, eg.np);
     if (s) return s;
     g->eg = eg;
     g->pads_ready = false;
@@ -1574,6 +1605,7 @@ ep_status ep_gnn_create(int32_t device, uint64_t seed, ep_gnn **out) try {
         cudaMalloc(&g->wt, sizeof(float) * kWtSize) != cudaSuccess ||
         cudaMalloc(&g->loss, sizeof(double)) != cudaSuccess ||
         cudaMalloc(&g->barrier, sizeof(unsigned)) != cudaSuccess ||
+        cudaEventCreateWithFlags(&g->used, cudaEventDisableTiming) != cudaSuccess ||
         cudaHostAlloc(&g->tc_flag_h, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&g->tc_flag_d, g->tc_flag_h, 0) != cudaSuccess) {
         g->err = "cudaMalloc failed for the network's weights";
@@ -1607,6 +1639,7 @@ void ep_gnn_destroy(ep_gnn *g) {
                     (void *)g->wt, (void *)g->loss, (void *)g->barrier})
         if (p) cudaFree(p);
     if (g->tc_flag_h) cudaFreeHost(g->tc_flag_h);
+    if (g->used) cudaEventDestroy(g->used);
     delete g;
 }
 
@@ -1618,6 +1651,7 @@ ep_status ep_gnn_get_weights(ep_gnn *g, float *w) {
 
 ep_status ep_gnn_set_weights(ep_gnn *g, const float *w) {
     if (!g || !w) return EP_ERR_ARG;
+    GK(cudaEventSynchronize(g->used));  // a pass that still reads the weights
     GK(cudaMemcpy(g->w, w, sizeof(float) * kParams, cudaMemcpyHostToDevice));
     GK(cudaMemset(g->adam_m, 0, sizeof(float) * kParams));
     GK(cudaMemset(g->adam_v, 0, sizeof(float) * kParams));
@@ -1639,7 +1673,8 @@ ep_status ep_gnn_release(ep_gnn *g, ep_engine *e) {
 
 ep_status ep_gnn_features(ep_gnn *g, ep_engine *e, float *X) {
     if (!g || !e || !X) return EP_ERR_ARG;
-    ep_status s = bind(g, e);
+    Use use(g);
+    ep_status s = bind(g, e, use);
     if (s) return s;
     GK(cudaMemcpyAsync(X, g->X, sizeof(float) * (size_t)g->net.N * kF, cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
@@ -1648,7 +1683,8 @@ ep_status ep_gnn_features(ep_gnn *g, ep_engine *e, float *X) {
 
 ep_status ep_gnn_forward(ep_gnn *g, ep_engine *e, float *xy4) try {
     if (!g || !e || !xy4) return EP_ERR_ARG;
-    ep_status s = bind(g, e);
+    Use use(g);
+    ep_status s = bind(g, e, use);
     if (s || (s = forward(g))) return s;
     const int nn = g->net.nn;
     std::vector<float4> p(nn);
@@ -1670,7 +1706,8 @@ ep_status ep_gnn_forward(ep_gnn *g, ep_engine *e, float *xy4) try {
 
 ep_status ep_gnn_loss_grad(ep_gnn *g, ep_engine *e, const float *target4, double *loss, float *grad) try {
     if (!g || !e || !target4) return EP_ERR_ARG;
-    ep_status s = bind(g, e);
+    Use use(g);
+    ep_status s = bind(g, e, use);
     if (s || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) || (s = backward(g)))
         return s;
     if (loss) GK(cudaMemcpyAsync(loss, g->loss, sizeof(double), cudaMemcpyDeviceToHost, g->eg.st));
@@ -1683,7 +1720,8 @@ ep_status ep_gnn_loss_grad(ep_gnn *g, ep_engine *e, const float *target4, double
 
 ep_status ep_gnn_train_step(ep_gnn *g, ep_engine *e, const float *target4, float lr, double *loss) try {
     if (!g || !e || !target4 || !(lr > 0)) return EP_ERR_ARG;
-    ep_status s = bind(g, e);
+    Use use(g);
+    ep_status s = bind(g, e, use);
     if (s || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) || (s = backward(g)))
         return s;
     g->step++;
@@ -1706,7 +1744,8 @@ ep_status ep_gnn_set_wait_limit(ep_gnn *g, int32_t polls) {
 
 ep_status ep_gnn_propose(ep_gnn *g, ep_engine *e, float alpha) {
     if (!g || !e || !(alpha >= 0.f) || alpha > 1.f) return EP_ERR_ARG;
-    ep_status s = bind(g, e);
+    Use use(g);
+    ep_status s = bind(g, e, use);
     if (s || (s = forward(g))) return s;
     const Grid &gr = g->eg.grid;
     k_propose<<<nblk(g->net.nn), kT, 0, g->eg.st>>>(g->net.nn, g->pred, alpha, gr.llx, gr.lly, gr.urx - gr.llx,

@@ -439,7 +439,9 @@ ep_status ep_density_scatter_noalloc(const ep_scatter_grid *grid, int32_t num_ob
  * accumulate); training minimises the mean squared error of both heads
  * (normalised to the core) with Adam.  All work runs on the engine's
  * stream, in a workspace the network keeps (grown to the largest netlist;
- * the features of the last engine used are kept until ep_gnn_release). */
+ * the features of the last engine used are kept until ep_gnn_release).  The
+ * calls of one network follow one another on the device, whatever streams
+ * their engines use (calls made while a stream is captured are not ordered). */
 typedef struct ep_gnn ep_gnn;
 int32_t ep_gnn_num_weights(void);
 ep_status ep_gnn_create(int32_t device, uint64_t seed, ep_gnn **out);
