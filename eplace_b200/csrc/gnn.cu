@@ -275,7 +275,6 @@ __global__ void k_store_feature(int N, const float2 *__restrict__ v, float *__re
 // us: 2k cells 1050 -> 590, 50k 1190 -> 790, 200k 1910 -> 1400.
 constexpr int kDiffThreads = 1024;
 constexpr size_t kDiffSmem = 216 * 1024;
-constexpr unsigned kBarrierPolls = 1u << 22;  // about a second or two
 
 struct DiffShare {  // pins a CTA's share can have (net phase, node phase)
     int net_pins, node_pins;
@@ -302,14 +301,15 @@ __device__ __forceinline__ int first_at_least(int n, int x, Key &&key) {
     return lo;
 }
 
-// All CTAs have written what they wrote before it; false when the wait gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target) {
+// All CTAs have written what they wrote before it; false when the wait gave up
+// (the default limit is a second or two).
+__device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, unsigned limit) {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
         int got = 0;
-        for (unsigned it = 0; it < kBarrierPolls && !got; it++) {
+        for (unsigned it = 0; it < limit && !got; it++) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
             got = v >= target;
@@ -329,7 +329,8 @@ __device__ __forceinline__ void gather_pins(const int32_t *__restrict__ idx, int
 
 __global__ void __launch_bounds__(kDiffThreads, 1)
 k_diffuse(Net g, int np, DiffShare share, const float *__restrict__ inv_pins, float2 *v, float2 *a,
-          float *__restrict__ X, unsigned *__restrict__ count, int *__restrict__ status, int *__restrict__ engine_status) {
+          float *__restrict__ X, unsigned *__restrict__ count, unsigned limit, int *__restrict__ status,
+          int *__restrict__ engine_status) {
     extern __shared__ __align__(16) unsigned char diff_sm[];
     float2 *val = reinterpret_cast<float2 *>(diff_sm);
     int32_t *net_idx = reinterpret_cast<int32_t *>(val + skew(max(share.net_pins, share.node_pins)) + 1);
@@ -407,7 +408,7 @@ k_diffuse(Net g, int np, DiffShare share, const float *__restrict__ inv_pins, fl
         for (int u = 0; u < kKept; u++)
             if (kb + tid + u * kDiffThreads < k1) sum_net(net[u]);
         for (int k = kb + tid + kKept * kDiffThreads; k < k1; k += kDiffThreads) sum_net(g.kinfo[k]);
-        ok = grid_barrier(count, target += G);
+        ok = grid_barrier(count, target += G, limit);
         if (!ok) break;
         gather_pins(node_idx, q1 - q0, a, val);
         const int col = step == kDiff1 ? 3 : step == kDiff2 ? 5 : step == kDiff3 ? 7 : 0;
@@ -437,7 +438,7 @@ k_diffuse(Net g, int np, DiffShare share, const float *__restrict__ inv_pins, fl
         for (int c = c0 + tid + kKept * kDiffThreads; c < c1; c += kDiffThreads)
             sum_node(c, g.obj_pin_start[c] - q0, g.obj_pin_start[c + 1] - q0, inv_pins[c]);
         if (step == kDiff3) break;
-        ok = grid_barrier(count, target += G);
+        ok = grid_barrier(count, target += G, limit);
         if (!ok) break;
     }
     if (!ok && tid == 0) {
@@ -1243,8 +1244,10 @@ struct ep_gnn {
     float *w = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
     __nv_bfloat16 *wb = nullptr;
     float *wt = nullptr;  // the input layer's weights as FP32 [k][o] (k_transpose_w)
-    int *tc_flag_h = nullptr, *tc_flag_d = nullptr;  // mapped: EP_ERR_TIMEOUT bit of the tensor-core layers
-    unsigned tc_wait_limit = tc::kWaitLimit;          // polls of their mbarrier wait (ep_gnn_set_wait_limit)
+    // mapped, raised by a bounded wait that gave up: [0] the tensor-core layers',
+    // whose outputs every pass computes anew, [1] the diffusion's, whose are kept
+    int *gave_up_h = nullptr, *gave_up_d = nullptr;
+    unsigned wait_limit = tc::kWaitLimit;  // polls of those waits (ep_gnn_set_wait_limit)
     int sms = 148;
     int cooperative = 0;         // the device takes cooperative launches
     unsigned *barrier = nullptr;  // the diffusion's arrival count
@@ -1395,7 +1398,7 @@ bool diffuse_at_once(ep_gnn *g, ep_status &status) {
     cudaError_t rc = cudaMemsetAsync(g->barrier, 0, sizeof(unsigned), eg.st);
     if (rc == cudaSuccess)
         rc = cudaLaunchKernelEx(&cfg, k_diffuse, g->net, eg.np, share, (const float *)g->inv_pins, g->v, g->netv, g->X,
-                                g->barrier, g->tc_flag_d, eg.d_status);
+                                g->barrier, g->wait_limit, g->gave_up_d + 1, eg.d_status);
     if (rc == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs than the device's are ours
         cudaGetLastError();
         return false;
@@ -1431,6 +1434,7 @@ ep_status bind(ep_gnn *g, ep_engine *e, Use &use) {
     s = reserve(g, N, eg.nnet, eg.nt, eg.np);
     if (s) return s;
     g->eg = eg;
+    g->uid = 0;  // until the features are on their way
     g->pads_ready = false;
     Net &n = g->net;
     n.nn = eg.nn;
@@ -1498,11 +1502,15 @@ ep_status bind_pads(ep_gnn *g) {
     return EP_OK;
 }
 
-// A give-up of the tensor-core layers' wait since the last check, reported
-// once (the flag is mapped host memory the kernel writes).
-ep_status tc_give_up(ep_gnn *g) {
-    if (!*(volatile int *)g->tc_flag_h) return EP_OK;
-    *(volatile int *)g->tc_flag_h = 0;
+// A wait that gave up since the last check, reported once: the diffusion's, and
+// with all also the tensor-core layers'.  The features that a diffusion left
+// incomplete are not kept.
+ep_status gave_up(ep_gnn *g, bool all) {
+    volatile int *f = g->gave_up_h;
+    if (!f[1] && !(all && f[0])) return EP_OK;
+    if (f[1]) g->uid = 0;
+    f[1] = 0;
+    if (all) f[0] = 0;
     g->err = "a bounded wait of the network's kernels gave up";
     return EP_ERR_TIMEOUT;
 }
@@ -1514,7 +1522,7 @@ ep_status forward(ep_gnn *g) {
     cudaStream_t st = g->eg.st;
     const float *w = g->w;
     const __nv_bfloat16 *wb = g->wb;
-    if (ep_status s = tc_give_up(g)) return s;  // of an earlier (asynchronous) pass
+    if (ep_status s = gave_up(g, true)) return s;  // of an earlier (asynchronous) pass
     const int tc_grid = std::max(1, std::min((N + kTcRows - 1) / kTcRows, 2 * g->sms));
     k_dense<kF, 0><<<nblk(N, kDenseRows), kT, smem_dense(kF), st>>>(N, g->X, nullptr, g->wt, w + kOffB0,
                                                                     g->h[0]);
@@ -1522,8 +1530,8 @@ ep_status forward(ep_gnn *g) {
         k_net_mean<<<n.n_big + nblk(n.nnet - n.n_big, kT / kHalf), kT, 0, st>>>(n, (const float2 *)g->h[l - 1],
                                                                                 (float2 *)g->a);
         k_node_mean<<<nblk((long long)N * kHalf), kT, 0, st>>>(n, g->inv_pins, (const float4 *)g->a, (float4 *)g->m[l]);
-        launch_dense_tc(tc_grid, st, N, g->h[l - 1], g->m[l], wb + off_w(l), w + off_b(l), g->h[l], g->tc_flag_d,
-                        g->eg.d_status, g->tc_wait_limit);
+        launch_dense_tc(tc_grid, st, N, g->h[l - 1], g->m[l], wb + off_w(l), w + off_b(l), g->h[l], g->gave_up_d,
+                        g->eg.d_status, g->wait_limit);
     }
     k_output<<<nblk(N), kT, 0, st>>>(N, g->h[kLayers], wb + kOffW4, w + kOffB4, g->v, g->raw, g->pred);
     GK(cudaGetLastError());
@@ -1606,12 +1614,12 @@ ep_status ep_gnn_create(int32_t device, uint64_t seed, ep_gnn **out) try {
         cudaMalloc(&g->loss, sizeof(double)) != cudaSuccess ||
         cudaMalloc(&g->barrier, sizeof(unsigned)) != cudaSuccess ||
         cudaEventCreateWithFlags(&g->used, cudaEventDisableTiming) != cudaSuccess ||
-        cudaHostAlloc(&g->tc_flag_h, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer(&g->tc_flag_d, g->tc_flag_h, 0) != cudaSuccess) {
+        cudaHostAlloc(&g->gave_up_h, 2 * sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&g->gave_up_d, g->gave_up_h, 0) != cudaSuccess) {
         g->err = "cudaMalloc failed for the network's weights";
         return EP_ERR_NOMEM;
     }
-    *g->tc_flag_h = 0;
+    g->gave_up_h[0] = g->gave_up_h[1] = 0;
     cudaDeviceGetAttribute(&g->sms, cudaDevAttrMultiProcessorCount, device);
     cudaDeviceGetAttribute(&g->cooperative, cudaDevAttrCooperativeLaunch, device);
     // Glorot-uniform weights, zero biases; the output layer starts small so
@@ -1638,7 +1646,7 @@ void ep_gnn_destroy(ep_gnn *g) {
     for (void *p : {(void *)g->w, (void *)g->grad, (void *)g->adam_m, (void *)g->adam_v, (void *)g->wb,
                     (void *)g->wt, (void *)g->loss, (void *)g->barrier})
         if (p) cudaFree(p);
-    if (g->tc_flag_h) cudaFreeHost(g->tc_flag_h);
+    if (g->gave_up_h) cudaFreeHost(g->gave_up_h);
     if (g->used) cudaEventDestroy(g->used);
     delete g;
 }
@@ -1678,7 +1686,7 @@ ep_status ep_gnn_features(ep_gnn *g, ep_engine *e, float *X) {
     if (s) return s;
     GK(cudaMemcpyAsync(X, g->X, sizeof(float) * (size_t)g->net.N * kF, cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
-    return EP_OK;
+    return gave_up(g, false);
 }
 
 ep_status ep_gnn_forward(ep_gnn *g, ep_engine *e, float *xy4) try {
@@ -1690,7 +1698,7 @@ ep_status ep_gnn_forward(ep_gnn *g, ep_engine *e, float *xy4) try {
     std::vector<float4> p(nn);
     GK(cudaMemcpyAsync(p.data(), g->pred, sizeof(float4) * nn, cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
-    if ((s = tc_give_up(g))) return s;
+    if ((s = gave_up(g, true))) return s;
     const Grid &gr = g->eg.grid;
     const float W = gr.urx - gr.llx, H = gr.ury - gr.lly;
     for (int c = 0; c < nn; c++) {
@@ -1713,7 +1721,7 @@ ep_status ep_gnn_loss_grad(ep_gnn *g, ep_engine *e, const float *target4, double
     if (loss) GK(cudaMemcpyAsync(loss, g->loss, sizeof(double), cudaMemcpyDeviceToHost, g->eg.st));
     if (grad) GK(cudaMemcpyAsync(grad, g->grad, sizeof(float) * kParams, cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
-    return tc_give_up(g);
+    return gave_up(g, true);
 } catch (const std::bad_alloc &) {
     return oom(g);
 }
@@ -1731,14 +1739,14 @@ ep_status ep_gnn_train_step(ep_gnn *g, ep_engine *e, const float *target4, float
     GK(cudaGetLastError());
     if (loss) GK(cudaMemcpyAsync(loss, g->loss, sizeof(double), cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
-    return tc_give_up(g);
+    return gave_up(g, true);
 } catch (const std::bad_alloc &) {
     return oom(g);
 }
 
 ep_status ep_gnn_set_wait_limit(ep_gnn *g, int32_t polls) {
     if (!g) return EP_ERR_ARG;
-    g->tc_wait_limit = polls < 0 ? tc::kWaitLimit : (unsigned)polls;
+    g->wait_limit = polls < 0 ? tc::kWaitLimit : (unsigned)polls;
     return EP_OK;
 }
 

@@ -791,8 +791,9 @@ class Gnn:
         self._check(self._L.ep_gnn_propose(self.h, engine.h, float(alpha)))
 
     def set_wait_limit(self, polls=None):
-        """ep_gnn_set_wait_limit: polls of the tensor-core layers' bounded
-        wait before it gives up (None: the default)."""
+        """ep_gnn_set_wait_limit: polls of the bounded waits of the
+        tensor-core layers and of the diffusion before they give up (None:
+        the default)."""
         self._check(self._L.ep_gnn_set_wait_limit(self.h, -1 if polls is None else int(polls)))
 
     def close(self):

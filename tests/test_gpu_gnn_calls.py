@@ -51,3 +51,41 @@ def test_weights_set_behind_a_proposal():
         g.set_weights(w)
     g.close()
     e.close()
+
+
+@pytest.mark.parametrize("cells", [60, 2_000, 40_000])  # one CTA, a few, one per SM
+def test_diffusion_wait_gives_up_and_recovers(cells):
+    """The diffusion's grid barrier, bounded: with no polls allowed the call
+    reports EP_ERR_TIMEOUT, and with the default limit restored the next call
+    computes the features anew instead of keeping what was left."""
+    (e,) = engines((cells,))
+    g = placer.Gnn(seed=3)
+    ref, pred = g.features(e), g.forward(e)
+    target = np.full((e.info.num_nodes, 4), 0.5, np.float32)
+    loss = g.loss_grad(e, target)
+    for call in (g.features, g.forward, lambda e: g.loss_grad(e, target)):
+        g.release(e)
+        g.set_wait_limit(0)
+        with pytest.raises(placer.EPError) as err:
+            call(e)
+        assert err.value.status == placer.EP_ERR_TIMEOUT
+        g.set_wait_limit()
+        assert np.array_equal(g.features(e), ref)
+    # a proposal returns before its pass is over: the next call reports it
+    g.propose(e, 0.5)
+    xy = e.get_positions()
+    g.release(e)
+    g.set_wait_limit(0)
+    g.propose(e, 0.5)
+    e.synchronize()
+    g.set_wait_limit()
+    with pytest.raises(placer.EPError) as err:
+        g.propose(e, 0.5)
+    assert err.value.status == placer.EP_ERR_TIMEOUT
+    g.propose(e, 0.5)
+    assert np.array_equal(e.get_positions(), xy)
+    assert np.array_equal(g.forward(e), pred)
+    again = g.loss_grad(e, target)
+    assert again[0] == loss[0] and np.array_equal(again[1], loss[1])
+    g.close()
+    e.close()
