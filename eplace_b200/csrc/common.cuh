@@ -26,7 +26,9 @@ enum ObjFlag : uint8_t {
 // finalising block of each reduction; every kernel reads `done`.
 struct DevScalars {
     // arrival counters of the grid-wide reductions (reset by their last block)
-    unsigned int cnt_prep, cnt_wl, cnt_comb, cnt_upd, cnt_hp;
+    unsigned int cnt_prep, cnt_wl, cnt_comb;
+    int step_done;  // `done` as the density pass of the step read it: what the update goes by, as it sets `done`
+    unsigned int cnt_hp;
     double hpwl_query;                // result of the standalone HPWL pass
     // results
     double tau;
@@ -269,18 +271,6 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double *sh) {
         }
     }
     __syncthreads();
-}
-
-// "Last block done": returns true in thread 0 of the block that finishes
-// last among `total` blocks (counted on *cnt, which it resets).
-__device__ __forceinline__ unsigned int arrive_acq_rel(unsigned int *cnt);
-
-__device__ __forceinline__ bool last_block(unsigned int *cnt, unsigned int total) {
-    if (arrive_acq_rel(cnt) == total - 1) {
-        *cnt = 0;
-        return true;
-    }
-    return false;
 }
 
 // Arrival count with acquire-release semantics at GPU scope: the partials this

@@ -2010,7 +2010,7 @@ ep_status ep_load_state(ep_engine *e, const void *buf, uint64_t bytes) {
     }
     std::memcpy(e->hS, p + sizeof(h), sizeof(DevScalars));
     DevScalars &S = *e->hS;
-    S.cnt_prep = S.cnt_wl = S.cnt_comb = S.cnt_upd = S.cnt_hp = 0;  // no reduction in flight
+    S.cnt_prep = S.cnt_wl = S.cnt_comb = S.cnt_hp = 0;  // no reduction in flight
     const unsigned char *v = p + sizeof(h) + sizeof(DevScalars);
     void *dst[kStateVecs] = {e->pos, e->x, e->g, e->y_prev, e->g_prev};
     for (int k = 0; k < kStateVecs; k++)

@@ -167,7 +167,7 @@ k_prep(Grid g, ull *__restrict__ node_q, ull *__restrict__ filler_q, const float
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nb; k += gridDim.x * blockDim.x) {
         const ull nq = node_q[k], fq = filler_q[k];
         float2 st = stat[k];  // (terminal, base)
-        if (done) return;
+        if (done) break;
         double node = (double)(long long)nq * inv_q;
         double fill = (double)(long long)fq * inv_q;
         // eDensity = node + base + filler + terminal (EPlace/eplace.cpp:576-577)
@@ -199,7 +199,8 @@ k_prep(Grid g, ull *__restrict__ node_q, ull *__restrict__ filler_q, const float
             filler_q[k] = 0ull;
         }
     }
-    if (done) return;  // a thread without bins
+    if (blockIdx.x == 0 && threadIdx.x == 0) S->step_done = done;
+    if (done) return;
     if (!grid_arrive<1>(acc, sh, partials, &S->cnt_prep, gridDim.x, blockIdx.x)) return;
     const int status = S->status;
     grid_total<1>(acc, sh, partials, &S->cnt_prep, gridDim.x);
@@ -1177,46 +1178,41 @@ __device__ __forceinline__ vec2<R> nesterov_move(const Grid &g, int o, R s, R c,
 }
 
 // The scalars of an update, read by one thread of the block for all of it, and
-// the step's end: iteration, stop flags and progress (host memory, mapped, that
-// the host watches during a run: steps taken, kProgressDone once the stage has
-// ended).  The end may come as soon as every block has read the scalars -- the
-// kernel's completion, not its own writes, is what the next kernel waits for --
-// so a block is counted right after its read, and the last one counted ends the
-// step: no block waits for its atomics to land before it counts itself (the
-// fence that this took held warp 0 and its block's place), and the positions
-// are read beside the scalars.  A step, before and after (us): 16^2 bins 23.2 ->
-// 22.4, 200k cells 56.6 -> 55.5, in FP64 88.0 -> 85.7, 1M 229 -> 218.
+// the step's end, by the first block: iteration, stop flags and progress (host
+// memory, mapped, that the host watches during a run: steps taken, kProgressDone
+// once the stage has ended).  No block reads what the first one writes (`done`
+// is read in the copy that the density pass left), so it need not know that the
+// others have read theirs, and the stores are out while it moves its objects;
+// what follows the update waits for the kernel's end.  A step (us) with the
+// blocks counted and the last one ending it / with every block's count ordered
+// behind its reads by a release / as here: 16^2 bins 21.5 / 22.4 / 21.5, 200k
+// cells 55.2 / 57.3 / 55.0, in FP64 84.0 / 86.7 / 82.6, 1M 219 / 221 / 202.
 template <typename R>
 struct StepScalars {
     R step, coef;
-    int iter, stop_pending, stage, done;
+    int stop_pending, done;
 };
 template <typename R>
-__device__ __forceinline__ unsigned read_step(StepScalars<R> *sh, DevScalars *S) {
+__device__ __forceinline__ void read_step(StepScalars<R> *sh, DevScalars *S, volatile int *progress) {
+    const bool ends = blockIdx.x == 0 && threadIdx.x == 0;
+    int iter = 0, stage = 0;
     if (threadIdx.x == 0) {
-        StepScalars<R> v{(R)S->step, (R)S->coef, S->iter, S->stop_pending, S->stage, S->done};
+        const StepScalars<R> v{(R)S->step, (R)S->coef, S->stop_pending, S->step_done};
+        if (ends) {
+            iter = S->iter;
+            stage = S->stage;
+        }
         *sh = v;
     }
     __syncthreads();
-    // the values are in shared memory, so the loads are over
-    unsigned arrived = 0;  // blocks counted before this one (thread 0)
-    if (threadIdx.x == 0 && !sh->done)
-        asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], 1;" : "=r"(arrived) : "l"(&S->cnt_upd));
-    return arrived;
-}
-template <typename R>
-__device__ __forceinline__ void end_step(const StepScalars<R> &v, unsigned arrived, DevScalars *S,
-                                         volatile int *progress) {
-    if (threadIdx.x != 0 || arrived != gridDim.x - 1) return;
-    const int iter = v.iter + 1;
-    S->cnt_upd = 0;
-    S->iter = iter;
+    if (!ends || sh->done) return;
+    S->iter = ++iter;
     S->lambda_pending = 1;
-    if (v.stop_pending) {
+    if (sh->stop_pending) {
         S->done = 1;
-        if (v.stage == EP_STAGE_MGP) S->mgp_iterations = iter;
+        if (stage == EP_STAGE_MGP) S->mgp_iterations = iter;
     }
-    *progress = iter | (v.stop_pending ? kProgressDone : 0);
+    *progress = iter | (sh->stop_pending ? kProgressDone : 0);
 }
 
 template <typename R>
@@ -1230,10 +1226,9 @@ k_update(Grid g, int n, const uint8_t *__restrict__ flags, const float2 *__restr
     const bool mine = o < n && (flags[o] & kInView);
     MoveInput<R> in;
     if (mine) in = load_move<R>(o, pos, x, gin);
-    const unsigned arrived = read_step<R>(&step, S);
+    read_step<R>(&step, S, progress);
     if (step.done) return;
     if (mine) nesterov_move<R>(g, o, step.step, step.coef, size[o], in, pos, x, y_prev, g_prev);
-    end_step<R>(step, arrived, S, progress);
 }
 
 // The update of the captured loop, with the next evaluation's scatter fused
@@ -1260,7 +1255,7 @@ k_update_scatter(Grid g, DeviceNetlist d, int big_blocks, vec2<R> *__restrict__ 
     MoveInput<R> in;
     const bool mover = valid && (u.count == 1 ? !(f & kBig) : u.rank == 0);
     if (mover) in = load_move<R>(u.o, pos, x, gin);
-    const unsigned arrived = read_step<R>(&step, S);
+    read_step<R>(&step, S, progress);
     if (step.done) return;
     const bool scatter = !step.stop_pending;
     auto move = [&] {
@@ -1275,7 +1270,6 @@ k_update_scatter(Grid g, DeviceNetlist d, int big_blocks, vec2<R> *__restrict__ 
         __syncthreads();  // block-uniform: every unit of this block has several threads
         if (valid && scatter) scatter_big<R>(g, big_pos[slot], sz, sxy, f, qscale, u.rank, u.count, maps);
     }
-    end_step<R>(step, arrived, S, progress);
 }
 
 // Backtracking trial move (opt_step_bktrk, Optimization/nesterov.hpp:337-349):
