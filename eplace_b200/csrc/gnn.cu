@@ -118,8 +118,7 @@ __global__ void k_pad_feature(int nt, int nn, const int *__restrict__ cnt, float
 
 // The terminals' pin lists (the transposed aggregation into terminals reads
 // them; training only): their starts by one block from the counts, the pins in
-// any order, then each list in pin order by counting the smaller ones (a block
-// per terminal; the lists are short).
+// any order, then each list in pin order (a block per terminal, k_pad_sort).
 __global__ void __launch_bounds__(kT) k_pad_start(int nt, const int *__restrict__ cnt, int32_t *__restrict__ start,
                                                   int *__restrict__ cursor) {
     __shared__ int tot[kT / 32];
@@ -151,14 +150,56 @@ __global__ void k_pad_fill(int np, Net g, int *__restrict__ cursor, int32_t *__r
     if (p < np && g.owner[p] >= g.n_obj) pins[atomicAdd(&cursor[g.owner[p] - g.n_obj], 1)] = p;
 }
 
-__global__ void __launch_bounds__(64) k_pad_sort(Net g, const int32_t *__restrict__ start,
+// A list of L of the np pins: by counting the smaller pins of each while L^2 <=
+// kPadScan np, else by walking all pins in order and keeping its own, so that no
+// list costs more than a walk or so (a fixed macro may have 100k pins).  Measured
+// for one list, counting / walking, us: 200k pins, L = 1000 58 / 95, 2000 193 /
+// 104; 788k pins, 2000 193 / 341, 4000 691 / 348, 64000 410000 / 646; the same
+// for 200 lists at once to a third.
+constexpr int kPadScan = 10;
+__global__ void __launch_bounds__(kT) k_pad_sort(Net g, int np, const int32_t *__restrict__ start,
                                                  const int32_t *__restrict__ pins, int32_t *__restrict__ nets) {
     const int b = start[blockIdx.x], e = start[blockIdx.x + 1];
-    for (int i = b + threadIdx.x; i < e; i += blockDim.x) {
-        const int p = pins[i];
-        int rank = 0;
-        for (int j = b; j < e; j++) rank += pins[j] < p;
-        nets[b + rank] = g.pin_net[p];
+    if ((long long)(e - b) * (e - b) <= (long long)kPadScan * np) {
+        for (int i = b + threadIdx.x; i < e; i += kT) {
+            const int p = pins[i];
+            int rank = 0;
+#pragma unroll 8
+            for (int j = b; j < e; j++) rank += pins[j] < p;
+            nets[b + rank] = g.pin_net[p];
+        }
+        return;
+    }
+    constexpr int kU = 8;  // pins of a thread in flight
+    __shared__ int found[2][kU][kT / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, owner = g.n_obj + blockIdx.x;
+    int at = b, buf = 0;
+    for (int p0 = 0; p0 < np && at < e; p0 += kU * kT, buf ^= 1) {  // block-uniform
+        unsigned m[kU];
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            const int p = p0 + u * kT + (int)threadIdx.x;
+            m[u] = p < np && g.owner[p] == owner;
+        }
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            m[u] = __ballot_sync(0xffffffffu, m[u]);
+            if (lane == 0) found[buf][u][w] = __popc(m[u]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kU; u++) {
+            int before = 0, all = 0;
+#pragma unroll
+            for (int k = 0; k < kT / 32; k++) {
+                const int c = found[buf][u][k];
+                if (k < w) before += c;
+                all += c;
+            }
+            if (m[u] >> lane & 1)
+                nets[at + before + __popc(m[u] & ((1u << lane) - 1))] = g.pin_net[p0 + u * kT + (int)threadIdx.x];
+            at += all;
+        }
     }
 }
 
@@ -1495,7 +1536,7 @@ ep_status bind_pads(ep_gnn *g) {
     if (eg.nt > 0) {
         k_pad_start<<<1, kT, 0, st>>>(eg.nt, g->padcnt, g->pad_start, g->pad_cursor);
         k_pad_fill<<<nblk(eg.np), kT, 0, st>>>(eg.np, g->net, g->pad_cursor, g->pad_pins);
-        k_pad_sort<<<eg.nt, 64, 0, st>>>(g->net, g->pad_start, g->pad_pins, g->pad_net);
+        k_pad_sort<<<eg.nt, kT, 0, st>>>(g->net, eg.np, g->pad_start, g->pad_pins, g->pad_net);
         GK(cudaGetLastError());
     }
     g->pads_ready = true;
