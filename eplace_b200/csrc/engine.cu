@@ -116,7 +116,6 @@ struct ep_engine {
     uint64_t uid = 0;  // distinct per engine created in this process
     QpDev qp{};
     bool qp_ready = false;
-    size_t qp_cap_x = 0, qp_cap_y = 0;
     double *qp_out_h = nullptr;  // pinned mirror of qp.out
     QpSolve *qp_state_h = nullptr;  // pinned mirror of the device solver state
     int bk_trials = 64;       // backtracking trials per step before EP_ERR_TIMEOUT (ep_limits)
@@ -2146,9 +2145,7 @@ ep_status qp_setup(ep_engine *e) {
     q.owner = e->pin_owner;
     q.off = e->pin_off;
 
-    // at most 4 entries per pin and axis: every counted pair of a net involves
-    // one of its two bound pins (< 2 d pairs, two entries each)
-    const size_t cap = qp_entry_cap(nn, np);
+    const size_t cap = qp_entry_cap(nn, e->h_net_deg.data(), nnet);
     const size_t n2 = ((size_t)nn + 1) & ~(size_t)1;  // the vector kernels take rows in pairs
     unsigned char *layout = nullptr;
     const int pb = qp_partial_blocks(nn, nnet);
@@ -2173,7 +2170,6 @@ ep_status qp_setup(ep_engine *e) {
     CK(cudaMemset(q.cnt, 0, sizeof(unsigned)));
     CK(cudaMallocHost((void **)&e->qp_out_h, 4 * sizeof(double)));
     CK(cudaMallocHost((void **)&e->qp_state_h, sizeof(QpSolve)));
-    e->qp_cap_x = e->qp_cap_y = cap;
     q.cap_x = q.cap_y = (int)std::min<size_t>(cap, (size_t)INT32_MAX);
     e->qp_ready = true;
     return EP_OK;

@@ -261,7 +261,7 @@ void qp_rows(const QpDev &q, int fill, cudaStream_t st);
 // where the rows' entries of both systems go, from the counts, on the device
 void qp_scan(const QpDev &q, cudaStream_t st);
 size_t qp_layout_bytes(int nn);
-size_t qp_entry_cap(int nn, int np);
+size_t qp_entry_cap(int nn, const int32_t *deg, int nnet);
 // r = b - A x and the solver's initial state (zero right-hand sides give x = 0)
 void qp_init(const QpDev &q, int max_it, cudaStream_t st);
 // enqueue `count` BiCGSTAB iterations (no-ops once both axes have stopped, and

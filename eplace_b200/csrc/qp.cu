@@ -263,7 +263,8 @@ k_qp_scan(int nw, Window *__restrict__ t, int cap_x, int cap_y, QpSolve *__restr
         v[3] += c.long_x;
         v[4] += c.long_y;
     }
-    int run[5], total[5];
+    int run[5];
+    long long total[5];  // past 2^31 they overflow any allocation, and the places are not used
 #pragma unroll
     for (int q = 0; q < 5; q++) {
         int x = v[q];
@@ -286,7 +287,7 @@ k_qp_scan(int nw, Window *__restrict__ t, int cap_x, int cap_y, QpSolve *__restr
     }
     for (int k = s0; k < s1; k++) {
         const Window c = t[k];
-        t[k] = Window{run[0], run[1], run[2], total[0] + run[3], total[1] + run[4], {0, 0, 0}};
+        t[k] = Window{run[0], run[1], run[2], (int)total[0] + run[3], (int)total[1] + run[4], {0, 0, 0}};
         run[0] += c.x;
         run[1] += c.y;
         run[2] += c.n_long;
@@ -294,7 +295,7 @@ k_qp_scan(int nw, Window *__restrict__ t, int cap_x, int cap_y, QpSolve *__restr
         run[4] += c.long_y;
     }
     if (threadIdx.x == 0) {
-        S->n_long = total[2];
+        S->n_long = (int)total[2];
         S->overflow = total[0] + total[3] > cap_x || total[1] + total[4] > cap_y;
     }
 }
@@ -945,8 +946,27 @@ static QpLayout layout(const QpDev &q) {
     l.slice = l.rel + w * kQT;
     return l;
 }
-// Entries an axis can need: every slice kLongRow long, and the long rows' own.
-size_t qp_entry_cap(int nn, int np) { return (size_t)windows(nn) * kQT * kLongRow + 4 * (size_t)np + 16; }
+// Entries an axis can need, the smaller of two bounds.  A net of d pins gives an
+// axis fewer than 4 d entries (its counted pairs involve one of its two bound
+// pins), and no slice is longer than kLongRow.  Or: of a pin's entries on either
+// axis, the more, there are d - 1 for the at most four bound pins of its net and
+// two for the others; m, their sum over a row, is at least the row's sort key and
+// the length of its longer axis.  In a window a slice's length is at most every m
+// of the slice after it (its long rows included, as their places in the order
+// are), and the last one's at most kLongRow.  So the slices take at most the sum
+// of min(m, kLongRow) over the window's rows and a slice of kLongRow; the long
+// rows' own entries count at most 31 of them twice.  200k cells and 788k pins:
+// 63 MB for both axes, 153 by the first bound alone.
+size_t qp_entry_cap(int nn, const int32_t *deg, int nnet) {
+    size_t pins = 0, most = 0;
+    for (int n = 0; n < nnet; n++) {
+        const size_t d = deg[n];
+        pins += d;
+        most += d > 4 ? 4 * (d - 1) + 2 * (d - 4) : d * (d - 1) * (d > 0);
+    }
+    const size_t w = windows(nn);
+    return std::min(w * kQT * kLongRow + 4 * pins, w * 2 * 32 * kLongRow + most) + 16;
+}
 
 void qp_rows(const QpDev &q, int fill, cudaStream_t st) {
     (fill ? k_qp_rows<true> : k_qp_rows<false>)<<<qblocks(q.nn), kQT, 0, st>>>(
