@@ -1545,10 +1545,13 @@ ep_status bind_pads(ep_gnn *g) {
 
 // A wait that gave up since the last check, reported once: the diffusion's, and
 // with all also the tensor-core layers'.  The features that a diffusion left
-// incomplete are not kept.
+// incomplete are not kept.  Every CTA that gives up raises the flag, so it is
+// cleared when the pass is over.  Called before a call enqueues anything (an
+// earlier pass that was not waited for) and after it has waited for its own.
 ep_status gave_up(ep_gnn *g, bool all) {
     volatile int *f = g->gave_up_h;
     if (!f[1] && !(all && f[0])) return EP_OK;
+    GK(cudaEventSynchronize(g->used));
     if (f[1]) g->uid = 0;
     f[1] = 0;
     if (all) f[0] = 0;
@@ -1563,7 +1566,6 @@ ep_status forward(ep_gnn *g) {
     cudaStream_t st = g->eg.st;
     const float *w = g->w;
     const __nv_bfloat16 *wb = g->wb;
-    if (ep_status s = gave_up(g, true)) return s;  // of an earlier (asynchronous) pass
     const int tc_grid = std::max(1, std::min((N + kTcRows - 1) / kTcRows, 2 * g->sms));
     k_dense<kF, 0><<<nblk(N, kDenseRows), kT, smem_dense(kF), st>>>(N, g->X, nullptr, g->wt, w + kOffB0,
                                                                     g->h[0]);
@@ -1723,8 +1725,8 @@ ep_status ep_gnn_release(ep_gnn *g, ep_engine *e) {
 ep_status ep_gnn_features(ep_gnn *g, ep_engine *e, float *X) {
     if (!g || !e || !X) return EP_ERR_ARG;
     Use use(g);
-    ep_status s = bind(g, e, use);
-    if (s) return s;
+    ep_status s = gave_up(g, false);
+    if (s || (s = bind(g, e, use))) return s;
     GK(cudaMemcpyAsync(X, g->X, sizeof(float) * (size_t)g->net.N * kF, cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
     return gave_up(g, false);
@@ -1733,8 +1735,8 @@ ep_status ep_gnn_features(ep_gnn *g, ep_engine *e, float *X) {
 ep_status ep_gnn_forward(ep_gnn *g, ep_engine *e, float *xy4) try {
     if (!g || !e || !xy4) return EP_ERR_ARG;
     Use use(g);
-    ep_status s = bind(g, e, use);
-    if (s || (s = forward(g))) return s;
+    ep_status s = gave_up(g, true);
+    if (s || (s = bind(g, e, use)) || (s = forward(g))) return s;
     const int nn = g->net.nn;
     std::vector<float4> p(nn);
     GK(cudaMemcpyAsync(p.data(), g->pred, sizeof(float4) * nn, cudaMemcpyDeviceToHost, g->eg.st));
@@ -1756,8 +1758,8 @@ ep_status ep_gnn_forward(ep_gnn *g, ep_engine *e, float *xy4) try {
 ep_status ep_gnn_loss_grad(ep_gnn *g, ep_engine *e, const float *target4, double *loss, float *grad) try {
     if (!g || !e || !target4) return EP_ERR_ARG;
     Use use(g);
-    ep_status s = bind(g, e, use);
-    if (s || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) || (s = backward(g)))
+    ep_status s = gave_up(g, true);
+    if (s || (s = bind(g, e, use)) || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) || (s = backward(g)))
         return s;
     if (loss) GK(cudaMemcpyAsync(loss, g->loss, sizeof(double), cudaMemcpyDeviceToHost, g->eg.st));
     if (grad) GK(cudaMemcpyAsync(grad, g->grad, sizeof(float) * kParams, cudaMemcpyDeviceToHost, g->eg.st));
@@ -1770,8 +1772,8 @@ ep_status ep_gnn_loss_grad(ep_gnn *g, ep_engine *e, const float *target4, double
 ep_status ep_gnn_train_step(ep_gnn *g, ep_engine *e, const float *target4, float lr, double *loss) try {
     if (!g || !e || !target4 || !(lr > 0)) return EP_ERR_ARG;
     Use use(g);
-    ep_status s = bind(g, e, use);
-    if (s || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) || (s = backward(g)))
+    ep_status s = gave_up(g, true);
+    if (s || (s = bind(g, e, use)) || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) || (s = backward(g)))
         return s;
     g->step++;
     const float c1 = 1.f / (1.f - std::pow(0.9f, (float)g->step)), c2 = 1.f / (1.f - std::pow(0.999f, (float)g->step));
@@ -1794,8 +1796,8 @@ ep_status ep_gnn_set_wait_limit(ep_gnn *g, int32_t polls) {
 ep_status ep_gnn_propose(ep_gnn *g, ep_engine *e, float alpha) {
     if (!g || !e || !(alpha >= 0.f) || alpha > 1.f) return EP_ERR_ARG;
     Use use(g);
-    ep_status s = bind(g, e, use);
-    if (s || (s = forward(g))) return s;
+    ep_status s = gave_up(g, true);
+    if (s || (s = bind(g, e, use)) || (s = forward(g))) return s;
     const Grid &gr = g->eg.grid;
     k_propose<<<nblk(g->net.nn), kT, 0, g->eg.st>>>(g->net.nn, g->pred, alpha, gr.llx, gr.lly, gr.urx - gr.llx,
                                                     gr.ury - gr.lly, g->xy);

@@ -63,7 +63,8 @@ def test_diffusion_wait_gives_up_and_recovers(cells):
     ref, pred = g.features(e), g.forward(e)
     target = np.full((e.info.num_nodes, 4), 0.5, np.float32)
     loss = g.loss_grad(e, target)
-    for call in (g.features, g.forward, lambda e: g.loss_grad(e, target)):
+    # 20 times: the CTAs give up one after another, the report comes once
+    for call in 20 * (g.features, g.forward, lambda e: g.loss_grad(e, target)):
         g.release(e)
         g.set_wait_limit(0)
         with pytest.raises(placer.EPError) as err:
