@@ -1173,7 +1173,7 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
         rc = dct_plan_init(e->dct, nbx, nby, g.sx, g.sy, P.dct_mode, e->fp64, e->err);
     }
     if (rc) return (ep_status)rc;
-    set_loop_carveout();
+    set_loop_carveout(kc);
     e->stage = EP_STAGE_MGP;
     s = upload_view(e, EP_STAGE_MGP);
     if (s) return s;

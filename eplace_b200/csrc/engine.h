@@ -146,7 +146,7 @@ int prep_blocks(const Grid &g);
 // smallest split that holds them.
 constexpr size_t kLoopSmemBytes = 64 * 1024;
 int carveout_percent(size_t smem_bytes);
-void set_loop_carveout();
+void set_loop_carveout(const KernelCtx &c);
 void set_sgemm_carveout(int carveout);
 // grid sizes of the reductions: 0 = per-net passes (both kernels), 1 = combine
 int reduction_blocks(const DeviceNetlist &d, int which);

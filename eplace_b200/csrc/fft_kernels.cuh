@@ -1,4 +1,4 @@
-// dct_fft.cu -- the electrostatic Poisson solve of FFT_2D::doFFT
+// fft_kernels.cuh -- the electrostatic Poisson solve of FFT_2D::doFFT
 // (FFT/fft.cpp:191-284) by fast transforms: the same sums as dct.cu,
 //   a   = C_nx rho C_ny^T,   P = a .* K,
 //   E_x = S_nx^T diag(wx) P C_ny,   E_y = C_nx^T P diag(wy) S_ny,   phi = C_nx^T P C_ny,
@@ -43,14 +43,15 @@
 // from 54.2 to 29.5 at 1024^2 and from 196 to 112 at 2048^2 in FP32, in FP64
 // from 23.0 to 17.0, 78 to 56 and 282 to 194; up to 256^2 they are launch and
 // latency bound (9 us).
+#pragma once
 #include <algorithm>
 #include <array>
 #include <cmath>
-#include <new>
 #include <utility>
+#include <string>
 #include <vector>
 
-#include "engine.h"
+#include "fft.h"
 
 namespace ep {
 
@@ -73,22 +74,6 @@ template <typename R>
 constexpr int col_count(int ny) {
     return sizeof(R) == 4 && ny / 4 > 148 ? 4 : 2;
 }
-
-struct FftPlan {
-    int lognx = 0, logny = 0;
-    int fp64 = 0;
-    // twiddles, stage-major: stage s (half-size h = 2^s) holds e^{-i pi j / h},
-    // j < h, at [h - 1 + j]; n - 1 entries per axis (vec2<R>)
-    void *twx = nullptr, *twy = nullptr;
-    // (cos, sin)(pi k / 2n), k <= n/2 (vec2<R>)
-    void *qx = nullptr, *qy = nullptr;
-    void *wx = nullptr, *wy = nullptr;  // frequency weights (R)
-    double kscale = 0.0;                // 4 / (nx ny)
-    void *T = nullptr;                  // [nx][ny] after the first pass (R)
-    void *X = nullptr;                  // X1, X2: [2][nx][ny] (R)
-    size_t smem_rows_fwd = 0, smem_cols = 0, smem_rows_inv = 0;
-    int pairs_fwd = 1, rows_inv = 1, cols = 2;
-};
 
 __device__ __forceinline__ int makhoul(int j, int n) { return (j & 1) ? n - 1 - (j >> 1) : (j >> 1); }
 
@@ -482,8 +467,10 @@ k_fft_cols(const R *__restrict__ T, const R *__restrict__ wx, const R *__restric
         };
         if (k0 == 0) {
             entry(std::false_type{}, 0, 0, zk[it], zk[it], true);
-            // (the loop amplifies a last place, so 512 keeps the rounding that
-            // its placements have had)
+            // Both roundings of this one frequency are equally near its value.
+            // One for all lengths would move 512^2 placements: the loop
+            // amplifies a last place to 1.2e-3 (FP32, 200k cells, 16 steps), so
+            // 512 keeps the one its placements have had.
             entry(std::bool_constant<LOGN == 9>{}, n / 2, n / 2, zm[it], zm[it], true);
         } else {
             entry(std::false_type{}, k0, n - k0, zk[it], zm[it], false);
@@ -594,7 +581,6 @@ k_fft_rows_inv(const R *__restrict__ X1, const R *__restrict__ X2, const R *__re
 }
 
 // Kernel instances for log2 n = kMinLog .. kMaxLog, per precision.
-constexpr int kMinLog = 3, kMaxLog = 11;
 constexpr int kLogs = kMaxLog - kMinLog + 1;
 template <typename R>
 struct FftFns {
@@ -611,6 +597,13 @@ struct FftFns {
     static constexpr std::array<ColsFn, sizeof...(L)> cols(std::integer_sequence<int, L...>) {
         return {k_fft_cols<L + kMinLog, COLS, col_threads(L + kMinLog), R>...};
     }
+    // two columns are half a sector in FP64
+    static constexpr std::array<ColsFn, kLogs> cols4() {
+        if constexpr (sizeof(R) == 4)
+            return cols<4>(std::make_integer_sequence<int, kLogs>{});
+        else
+            return {};
+    }
     static ColsFn cols_fn(int logn, int cols) { return cols == 2 ? kCols2[logn - kMinLog] : kCols4[logn - kMinLog]; }
     template <bool PHI, int... L>
     static constexpr std::array<RowsInvFn, sizeof...(L)> rows_inv(std::integer_sequence<int, L...>) {
@@ -625,25 +618,15 @@ template <typename R>
 const std::array<typename FftFns<R>::RowsFwdFn, kLogs> FftFns<R>::kRowsFwd = FftFns<R>::rows_fwd(LogSeq{});
 template <typename R>
 const std::array<typename FftFns<R>::ColsFn, kLogs> FftFns<R>::kCols2 = FftFns<R>::template cols<2>(LogSeq{});
-template <>
-const std::array<FftFns<float>::ColsFn, kLogs> FftFns<float>::kCols4 = FftFns<float>::cols<4>(LogSeq{});
-template <>
-const std::array<FftFns<double>::ColsFn, kLogs> FftFns<double>::kCols4{};  // two columns are half a sector
+template <typename R>
+const std::array<typename FftFns<R>::ColsFn, kLogs> FftFns<R>::kCols4 = FftFns<R>::cols4();
 template <typename R>
 const std::array<typename FftFns<R>::RowsInvFn, kLogs> FftFns<R>::kRowsInv = FftFns<R>::template rows_inv<false>(LogSeq{});
 template <typename R>
 const std::array<typename FftFns<R>::RowsInvFn, kLogs> FftFns<R>::kRowsInvPhi =
     FftFns<R>::template rows_inv<true>(LogSeq{});
-template struct FftFns<float>;
-template struct FftFns<double>;
 
 int seqs_per_block_rt(int logn) { return std::max(1, kRowElems >> logn); }
-
-int ilog2_exact(int n) {
-    int l = 0;
-    while ((1 << l) < n) l++;
-    return (1 << l) == n ? l : -1;
-}
 
 template <typename T>
 int upload_vec(void *&dst, const std::vector<T> &src, std::string &err) {
@@ -668,9 +651,11 @@ void tables(int n, std::vector<vec2<R>> &tw, std::vector<vec2<R>> &q) {
     for (int k = 0; k <= n / 2; k++) q[k] = mk2<R>((R)cos(pi * k / (2.0 * n)), (R)sin(pi * k / (2.0 * n)));
 }
 
+}  // namespace
+
 template <typename R>
-int fft_init_t(FftPlan *f, int nx, int ny, const std::vector<double> &wx, const std::vector<double> &wy,
-               std::string &err) {
+int FftPasses<R>::init(FftPlan *f, int nx, int ny, const std::vector<double> &wx, const std::vector<double> &wy,
+                       std::string &err) {
     const int lx = f->lognx, ly = f->logny;
     std::vector<vec2<R>> tw, q;
     int rc;
@@ -716,8 +701,8 @@ int fft_init_t(FftPlan *f, int nx, int ny, const std::vector<double> &wx, const 
 }
 
 template <typename R>
-void fft_run_t(const FftPlan *f, int nx, int ny, const R *rho, vec2<R> *field, R *phi, const DevScalars *S,
-               cudaStream_t st) {
+void FftPasses<R>::run(const FftPlan *f, int nx, int ny, const R *rho, vec2<R> *field, R *phi, const DevScalars *S,
+                       cudaStream_t st) {
     using F = FftFns<R>;
     R *X1 = (R *)f->X, *X2 = X1 + (size_t)nx * ny;
     const int pr = launch_priority(true);
@@ -730,46 +715,6 @@ void fft_run_t(const FftPlan *f, int nx, int ny, const R *rho, vec2<R> *field, R
     launch_kp(phi ? F::kRowsInvPhi[ly] : F::kRowsInv[ly], nx / f->rows_inv, row_threads(f->logny),
               phi ? f->smem_rows_inv : f->smem_rows_inv - phi_seqs, st, pr, (const R *)X1, (const R *)X2,
               (const R *)f->wy, field, phi, f->rows_inv, (const vec2<R> *)f->twy, (const vec2<R> *)f->qy, S);
-}
-
-}  // namespace
-
-int dct_fft_init(DctPlan &p, const std::vector<double> &wx, const std::vector<double> &wy, int fp64,
-                 std::string &err) {
-    const int nx = p.nx, ny = p.ny;
-    const int lx = ilog2_exact(nx), ly = ilog2_exact(ny);
-    if (lx < kMinLog || ly < kMinLog || lx > kMaxLog || ly > kMaxLog) {
-        err = "the FFT Poisson path needs power-of-two bin counts in [8, 2048]";
-        return EP_ERR_UNSUPPORTED;
-    }
-    FftPlan *f = new (std::nothrow) FftPlan;
-    if (!f) {
-        err = "out of host memory for the FFT plan";
-        return EP_ERR_NOMEM;
-    }
-    p.fft = f;
-    f->lognx = lx;
-    f->logny = ly;
-    f->fp64 = fp64;
-    return fp64 ? fft_init_t<double>(f, nx, ny, wx, wy, err) : fft_init_t<float>(f, nx, ny, wx, wy, err);
-}
-
-void dct_fft_free(DctPlan &p) {
-    FftPlan *f = (FftPlan *)p.fft;
-    if (!f) return;
-    for (void *d : {f->twx, f->twy, f->qx, f->qy, f->wx, f->wy, f->T, f->X})
-        if (d) cudaFree(d);
-    delete f;
-    p.fft = nullptr;
-}
-
-int dct_fft_run(DctPlan &p, const void *rho, void *field, void *phi, const DevScalars *S, cudaStream_t st) {
-    const FftPlan *f = (const FftPlan *)p.fft;
-    if (f->fp64)
-        fft_run_t<double>(f, p.nx, p.ny, (const double *)rho, (double2 *)field, (double *)phi, S, st);
-    else
-        fft_run_t<float>(f, p.nx, p.ny, (const float *)rho, (float2 *)field, (float *)phi, S, st);
-    return EP_OK;
 }
 
 }  // namespace ep

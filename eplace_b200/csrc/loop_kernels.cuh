@@ -1,4 +1,4 @@
-// kernels.cu -- the per-iteration kernels of the ePlace inner loop.
+// loop_kernels.cuh -- the per-iteration kernels of the ePlace inner loop.
 //
 //   scatter   cell/filler -> bin overlap areas as int64 fixed point with
 //             atomics: order-independent, so the maps are bit-exact and
@@ -22,33 +22,20 @@
 // multi-iteration graph stops doing work after the stop condition.  Each is a
 // template on the working precision R (float: the engine's mixed-precision
 // form, whose arithmetic follows the reference's float steps; double: the
-// plain FP64 form); the launchers pick the instance from KernelCtx::fp64.
+// plain FP64 form), instantiated in a file of its own for each (loop.h).
+#pragma once
 #include <algorithm>
 #include <cmath>
-#include <cstdio>
-#include <iterator>
-#include <mutex>
 #include <vector>
 
-#include "engine.h"
+#include "loop.h"
 #include "scatter.cuh"
 
 namespace ep {
 
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kPinChunk = 128;  // pin gradients a warp of the combine kernel stages per round
-
-constexpr int kSms = 148;
-// Grids of the kernels that loop over their work and end in a grid sum: one
-// block for each that an SM holds, so that a block's reduction and the wait for
-// its slowest warp are paid once.  Fixed numbers, so that the sums do not
-// depend on anything else.
-constexpr int kNetBlocks = kSms * 6, kCombineBlocks = kSms * 3;
-inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
-
-using ull = unsigned long long;
 
 __device__ __forceinline__ float exact_exp(float a) { return expf(a); }
 __device__ __forceinline__ double exact_exp(double a) { return exp(a); }
@@ -1296,18 +1283,6 @@ k_bktrk_move(Grid g, int n, const uint8_t *__restrict__ flags, const float2 *__r
     pos[o] = clamp_center<R>(g, yn, size[o]);
 }
 
-// The accepted trial ends the step: the scalar side of k_update.
-__global__ void k_bktrk_commit(DevScalars *__restrict__ S) {
-    pdl_begin();
-    if (S->done) return;
-    S->iter += 1;
-    S->lambda_pending = 1;
-    if (S->stop_pending) {
-        S->done = 1;
-        if (S->stage == EP_STAGE_MGP) S->mgp_iterations = S->iter;
-    }
-}
-
 // EplaceNesterovOpt::init (nesterov.hpp:207-214): x_0 = current positions.
 template <typename R>
 __global__ void k_stage_begin(int n, const uint8_t *__restrict__ flags, const vec2<R> *__restrict__ pos,
@@ -1336,22 +1311,6 @@ __global__ void k_stage_begin(int n, const uint8_t *__restrict__ flags, const ve
     }
 }
 
-// Scalars that a call sets before its kernels, in stream order (a read-back, a
-// change on the host and a copy cost two synchronisations).
-__global__ void k_set_scalars(DevScalars *__restrict__ S, ScalarSet what, double value) {
-    pdl_begin();
-    if (what == ScalarSet::kLambda) {
-        S->lambda = value;
-        return;
-    }
-    S->lambda0_mode = 1;  // the next evaluation is initialization()'s
-    if (what == ScalarSet::kInitialize) {
-        S->lambda = 0.0;
-        S->status = 0;
-        S->done = 0;
-    }
-}
-
 // wrap_up (nesterov.hpp:216-223): positions = main solution, clamped.
 template <typename R>
 __global__ void k_wrap_up(Grid g, int n, const uint8_t *__restrict__ flags, const float2 *__restrict__ size,
@@ -1364,31 +1323,6 @@ __global__ void k_wrap_up(Grid g, int n, const uint8_t *__restrict__ flags, cons
 }  // namespace
 
 // ------------------------------------------------------------- launchers --
-int launch_priority(bool high) {
-    // the range is the same on every device; a function-local static is
-    // initialised once even when engines are created on several threads
-    static const int2 range = [] {
-        int l = 0, h = 0;
-        cudaDeviceGetStreamPriorityRange(&l, &h);
-        return make_int2(l, h);
-    }();
-    return high ? range.y : range.x;
-}
-
-int prep_blocks(const Grid &g) { return std::min(blocks_for(g.nx * g.ny, kThreads), kSms * 8); }
-
-// Blocks of the object kernels that take the kBig objects (object_unit).
-static int big_blocks(const DeviceNetlist &d) {
-    return d.n_huge_objs + blocks_for(d.n_big_objs - d.n_huge_objs, kThreads / 32);
-}
-
-int reduction_blocks(const DeviceNetlist &d, int which) {
-    switch (which) {
-        case 0: return d.n_block_nets + std::min(blocks_for(d.n_net_tasks - d.n_block_nets, kNetWarps), kNetBlocks);
-        default: return big_blocks(d) + std::min(blocks_for(d.n_obj, kThreads), kCombineBlocks);
-    }
-}
-
 namespace {
 template <typename R>
 inline vec2<R> *V(void *p) {
@@ -1398,61 +1332,47 @@ template <typename R>
 inline const vec2<R> *V(const void *p) {
     return static_cast<const vec2<R> *>(p);
 }
-}  // namespace
-
-template <typename R>
-static void scatter_t(const KernelCtx &c, const DeviceNetlist &d, ull *maps, const DevScalars *S, cudaStream_t st) {
-    const int bb = big_blocks(d);
-    launch_k(k_scatter<R>, bb + blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d, bb, c.qscale, maps, S);
-}
-
-void launch_scatter(const KernelCtx &c, const DeviceNetlist &d, ull *maps, const DevScalars *S, cudaStream_t st) {
-    c.fp64 ? scatter_t<double>(c, d, maps, S, st) : scatter_t<float>(c, d, maps, S, st);
-}
-
-template <typename R>
-static void update_scatter_t(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
-                             void *y_prev, void *g_prev, ull *maps, DevScalars *S, int *progress, cudaStream_t st) {
-    const int bb = big_blocks(d);
-    const int blocks = bb + blocks_for(d.n_obj, kThreads);
-    constexpr int kMany = sizeof(R) == 8 ? 5 : 6;
-    launch_k(blocks <= kSms * 4 ? k_update_scatter<1, R> : k_update_scatter<kMany, R>, blocks, kThreads, 0, st, c.grid,
-             d, bb, V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), c.qscale, maps, S, progress);
-}
-
-void launch_update_scatter(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
-                           void *y_prev, void *g_prev, ull *maps, DevScalars *S, int *progress, cudaStream_t st) {
-    c.fp64 ? update_scatter_t<double>(c, d, pos, x, g, y_prev, g_prev, maps, S, progress, st)
-           : update_scatter_t<float>(c, d, pos, x, g, y_prev, g_prev, maps, S, progress, st);
-}
-
-void launch_prep(const KernelCtx &c, ull *node_q, ull *filler_q, const float2 *static_map, void *rho,
-                 void *rho_bf16, float *node_f, float *filler_f, int zero_maps, DevScalars *S, cudaStream_t st) {
-    int nb = c.grid.nx * c.grid.ny;
-    int blocks = prep_blocks(c.grid);
-    uint16_t *hi = (uint16_t *)rho_bf16;
-    uint16_t *lo = hi ? hi + nb : nullptr;
-    if (c.fp64)
-        launch_k(k_prep<double>, blocks, kThreads, 0, st, c.grid, node_q, filler_q, static_map, (double *)rho,
-                 (uint16_t *)nullptr, (uint16_t *)nullptr, node_f, filler_f, zero_maps, c.inv_qscale,
-                 c.inv_bin_area, c.bin_area, c.area_norm, c.part_prep, S);
-    else
-        launch_k(k_prep<float>, blocks, kThreads, 0, st, c.grid, node_q, filler_q, static_map, (float *)rho, hi, lo,
-                 node_f, filler_f, zero_maps, c.inv_qscale, c.inv_bin_area, c.bin_area, c.area_norm, c.part_prep,
-                 S);
-}
 
 template <bool WL, bool EXACT, bool LSE, typename R>
-static void launch_nets(const KernelCtx &c, const DeviceNetlist &d, void *pin_grad, double *partials, int mode,
-                        DevScalars *S, cudaStream_t st) {
+void launch_nets(const KernelCtx &c, const DeviceNetlist &d, void *pin_grad, double *partials, int mode, DevScalars *S,
+                 cudaStream_t st) {
     PinCtx<R> pc{d.pin_owner, d.pin_off, V<R>(d.pos), d.pin_obj_slot};
     if (d.n_net_tasks == 0) return;
     launch_kp(k_wl<WL, EXACT, LSE, R>, reduction_blocks(d, 0), kNetWarps * 32, 0, st, launch_priority(false),
               d.net_tasks, d.n_block_nets, d.n_net_tasks, pc, V<R>(pin_grad), c.want_wl_value, partials, mode, S);
 }
 
+// Blocks an SM that k_update_scatter's registers allow in a large design.
 template <typename R>
-static void wirelength_t(const KernelCtx &c, const DeviceNetlist &d, void *pin_grad, DevScalars *S, cudaStream_t st) {
+constexpr int kUpdateBlocks = sizeof(R) == 8 ? 5 : 6;
+}  // namespace
+
+template <typename R>
+void Loop<R>::scatter(const KernelCtx &c, const DeviceNetlist &d, ull *maps, const DevScalars *S, cudaStream_t st) {
+    const int bb = big_blocks(d);
+    launch_k(k_scatter<R>, bb + blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d, bb, c.qscale, maps, S);
+}
+
+template <typename R>
+void Loop<R>::update_scatter(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g,
+                             void *y_prev, void *g_prev, ull *maps, DevScalars *S, int *progress, cudaStream_t st) {
+    const int bb = big_blocks(d);
+    const int blocks = bb + blocks_for(d.n_obj, kThreads);
+    launch_k(blocks <= kSms * 4 ? k_update_scatter<1, R> : k_update_scatter<kUpdateBlocks<R>, R>, blocks, kThreads, 0,
+             st, c.grid, d, bb, V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), c.qscale, maps, S, progress);
+}
+
+template <typename R>
+void Loop<R>::prep(const KernelCtx &c, ull *node_q, ull *filler_q, const float2 *static_map, void *rho, void *rho_bf16,
+                   float *node_f, float *filler_f, int zero_maps, DevScalars *S, cudaStream_t st) {
+    uint16_t *hi = sizeof(R) == 4 ? (uint16_t *)rho_bf16 : nullptr;
+    uint16_t *lo = hi ? hi + c.grid.nx * c.grid.ny : nullptr;
+    launch_k(k_prep<R>, prep_blocks(c.grid), kThreads, 0, st, c.grid, node_q, filler_q, static_map, (R *)rho, hi, lo,
+             node_f, filler_f, zero_maps, c.inv_qscale, c.inv_bin_area, c.bin_area, c.area_norm, c.part_prep, S);
+}
+
+template <typename R>
+void Loop<R>::wirelength(const KernelCtx &c, const DeviceNetlist &d, void *pin_grad, DevScalars *S, cudaStream_t st) {
     if (c.exact_exp)
         c.lse ? launch_nets<true, true, true, R>(c, d, pin_grad, c.part_wl, 0, S, st)
               : launch_nets<true, true, false, R>(c, d, pin_grad, c.part_wl, 0, S, st);
@@ -1461,131 +1381,54 @@ static void wirelength_t(const KernelCtx &c, const DeviceNetlist &d, void *pin_g
               : launch_nets<true, false, false, R>(c, d, pin_grad, c.part_wl, 0, S, st);
 }
 
-void launch_wirelength(const KernelCtx &c, const DeviceNetlist &d, void *pin_grad, DevScalars *S, cudaStream_t st) {
-    c.fp64 ? wirelength_t<double>(c, d, pin_grad, S, st) : wirelength_t<float>(c, d, pin_grad, S, st);
+template <typename R>
+void Loop<R>::hpwl(const KernelCtx &c, const DeviceNetlist &d, int mode, DevScalars *S, cudaStream_t st) {
+    launch_nets<false, false, false, R>(c, d, nullptr, c.part_hp, mode, S, st);
 }
 
 template <typename R>
-static void combine_t(const KernelCtx &c, const DeviceNetlist &d, const void *field, const void *pin_grad, void *g,
+void Loop<R>::combine(const KernelCtx &c, const DeviceNetlist &d, const void *field, const void *pin_grad, void *g,
                       const void *g_prev, const void *y_prev, void *dump_gd, void *dump_gwl, int stepping,
                       DevScalars *S, cudaStream_t st) {
-    const int bb = big_blocks(d);
-    launch_k(k_combine<R>, reduction_blocks(d, 1), kThreads, 0, st, c.grid, d, V<R>(field),
-             V<R>(pin_grad), V<R>(g), V<R>(g_prev), V<R>(y_prev), V<R>(dump_gd), V<R>(dump_gwl), bb, stepping,
-             c.part_comb, S);
-}
-
-void launch_combine(const KernelCtx &c, const DeviceNetlist &d, const void *field, const void *pin_grad, void *g,
-                    const void *g_prev, const void *y_prev, void *dump_gd, void *dump_gwl, int stepping, DevScalars *S,
-                    cudaStream_t st) {
-    c.fp64 ? combine_t<double>(c, d, field, pin_grad, g, g_prev, y_prev, dump_gd, dump_gwl, stepping, S, st)
-           : combine_t<float>(c, d, field, pin_grad, g, g_prev, y_prev, dump_gd, dump_gwl, stepping, S, st);
+    launch_k(k_combine<R>, reduction_blocks(d, 1), kThreads, 0, st, c.grid, d, V<R>(field), V<R>(pin_grad), V<R>(g),
+             V<R>(g_prev), V<R>(y_prev), V<R>(dump_gd), V<R>(dump_gwl), big_blocks(d), stepping, c.part_comb, S);
 }
 
 template <typename R>
-static void update_t(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g, void *y_prev,
+void Loop<R>::update(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g, void *y_prev,
                      void *g_prev, DevScalars *S, int *progress, cudaStream_t st) {
     launch_k(k_update<R>, blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d.n_obj, d.flags, d.size,
              V<R>(pos), V<R>(x), V<R>(g), V<R>(y_prev), V<R>(g_prev), S, progress);
 }
 
-void launch_update(const KernelCtx &c, const DeviceNetlist &d, void *pos, void *x, const void *g, void *y_prev,
-                   void *g_prev, DevScalars *S, int *progress, cudaStream_t st) {
-    c.fp64 ? update_t<double>(c, d, pos, x, g, y_prev, g_prev, S, progress, st)
-           : update_t<float>(c, d, pos, x, g, y_prev, g_prev, S, progress, st);
-}
-
 template <typename R>
-static void bktrk_move_t(const KernelCtx &c, const DeviceNetlist &d, const void *ysave, const void *g,
-                         const void *x, void *pos, void *xtrial, const DevScalars *S, cudaStream_t st) {
+void Loop<R>::bktrk_move(const KernelCtx &c, const DeviceNetlist &d, const void *ysave, const void *g, const void *x,
+                         void *pos, void *xtrial, const DevScalars *S, cudaStream_t st) {
     launch_k(k_bktrk_move<R>, blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d.n_obj, d.flags, d.size,
              V<R>(ysave), V<R>(g), V<R>(x), V<R>(pos), V<R>(xtrial), S);
 }
 
-void launch_bktrk_move(const KernelCtx &c, const DeviceNetlist &d, const void *ysave, const void *g, const void *x,
-                       void *pos, void *xtrial, const DevScalars *S, cudaStream_t st) {
-    c.fp64 ? bktrk_move_t<double>(c, d, ysave, g, x, pos, xtrial, S, st)
-           : bktrk_move_t<float>(c, d, ysave, g, x, pos, xtrial, S, st);
-}
-
-void launch_bktrk_commit(DevScalars *S, cudaStream_t st) { launch_k(k_bktrk_commit, 1, 1, 0, st, S); }
-
-void launch_stage_begin(const KernelCtx &c, const DeviceNetlist &d, const void *pos, void *x, int step_cap,
-                        DevScalars *S, int *progress, cudaStream_t st) {
-    const int blocks = std::min(blocks_for(d.n_obj, kThreads), kSms * 4);
-    if (c.fp64)
-        launch_k(k_stage_begin<double>, blocks, kThreads, 0, st, d.n_obj, d.flags, V<double>(pos), V<double>(x),
-                 step_cap, S, progress);
-    else
-        launch_k(k_stage_begin<float>, blocks, kThreads, 0, st, d.n_obj, d.flags, V<float>(pos), V<float>(x), step_cap,
-                 S, progress);
-}
-
-void launch_set_scalars(DevScalars *S, ScalarSet what, double value, cudaStream_t st) {
-    launch_k(k_set_scalars, 1, 1, 0, st, S, what, value);
-}
-
-void launch_wrap_up(const KernelCtx &c, const DeviceNetlist &d, void *pos, const void *x, cudaStream_t st) {
-    if (c.fp64)
-        launch_k(k_wrap_up<double>, blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d.n_obj, d.flags, d.size,
-                 V<double>(pos), V<double>(x));
-    else
-        launch_k(k_wrap_up<float>, blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d.n_obj, d.flags, d.size,
-                 V<float>(pos), V<float>(x));
-}
-
-void launch_hpwl(const KernelCtx &c, const DeviceNetlist &d, int mode, DevScalars *S, cudaStream_t st) {
-    c.fp64 ? launch_nets<false, false, false, double>(c, d, nullptr, c.part_hp, mode, S, st)
-           : launch_nets<false, false, false, float>(c, d, nullptr, c.part_hp, mode, S, st);
-}
-
-int carveout_percent(size_t smem_bytes) {
-    // shared-memory capacities of an sm_100 SM, KB; the driver maps a
-    // preferred percentage of the largest to one of them, so ask for the
-    // middle of the interval that rounds to the capacity wanted
-    static const int kConfigs[] = {0, 8, 16, 32, 64, 100, 132, 164, 196, 228};
-    const double kb = (double)smem_bytes / 1024.0;
-    for (int i = 1; i < 10; i++)
-        if (kConfigs[i] >= kb) return (int)std::ceil(50.0 * (kConfigs[i - 1] + kConfigs[i]) / 228.0);
-    return 100;
+template <typename R>
+void Loop<R>::stage_begin(const DeviceNetlist &d, const void *pos, void *x, int step_cap, DevScalars *S,
+                          int *progress, cudaStream_t st) {
+    launch_k(k_stage_begin<R>, std::min(blocks_for(d.n_obj, kThreads), kSms * 4), kThreads, 0, st, d.n_obj, d.flags,
+             V<R>(pos), V<R>(x), step_cap, S, progress);
 }
 
 template <typename R>
-static void loop_kernels(std::vector<const void *> &fns) {
-    const void *f[] = {(const void *)k_scatter<R>, (const void *)k_prep<R>, (const void *)k_wl<true, false, false, R>,
-                       (const void *)k_wl<true, true, false, R>, (const void *)k_wl<true, false, true, R>,
-                       (const void *)k_wl<true, true, true, R>, (const void *)k_wl<false, false, false, R>,
-                       (const void *)k_combine<R>, (const void *)k_update<R>,
-                       (const void *)k_update_scatter<1, R>,
-                       (const void *)k_update_scatter<sizeof(R) == 8 ? 5 : 6, R>, (const void *)k_bktrk_move<R>,
-                       (const void *)k_stage_begin<R>, (const void *)k_wrap_up<R>};
-    fns.insert(fns.end(), std::begin(f), std::end(f));
+void Loop<R>::wrap_up(const KernelCtx &c, const DeviceNetlist &d, void *pos, const void *x, cudaStream_t st) {
+    launch_k(k_wrap_up<R>, blocks_for(d.n_obj, kThreads), kThreads, 0, st, c.grid, d.n_obj, d.flags, d.size,
+             V<R>(pos), V<R>(x));
 }
 
-// One L1/shared split, kLoopSmemBytes of shared memory, for every kernel of
-// the loop: an SM whose split has to change between consecutive kernels must
-// drain first, which costs the programmatic overlap of the launches (on the
-// 200k-cell solve with the FFT Poisson path: 14.5 ms per solve with one split
-// against 18.3 ms with the driver's choice per kernel).  64 KB holds the
-// per-net and combine kernels' staging at full occupancy and leaves 192 KB of
-// L1; smaller splits cost them occupancy, larger ones L1.
-// Function attributes belong to the current device: set once per device.
-void set_loop_carveout() {
-    static std::mutex mu;
-    static std::vector<int> done_devices;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (std::find(done_devices.begin(), done_devices.end(), dev) != done_devices.end()) return;
-        done_devices.push_back(dev);
-    }
-    const int carveout = carveout_percent(kLoopSmemBytes);
-    std::vector<const void *> fns = {(const void *)k_bktrk_commit, (const void *)k_set_scalars};
-    loop_kernels<float>(fns);
-    loop_kernels<double>(fns);
-    for (const void *f : fns) cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
-    set_sgemm_carveout(carveout);
+template <typename R>
+std::vector<const void *> Loop<R>::kernels(bool exact_exp, bool lse) {
+    const void *wl = exact_exp ? (lse ? (const void *)k_wl<true, true, true, R> : (const void *)k_wl<true, true, false, R>)
+                               : (lse ? (const void *)k_wl<true, false, true, R> : (const void *)k_wl<true, false, false, R>);
+    return {(const void *)k_scatter<R>, (const void *)k_prep<R>, wl, (const void *)k_wl<false, false, false, R>,
+            (const void *)k_combine<R>, (const void *)k_update<R>, (const void *)k_update_scatter<1, R>,
+            (const void *)k_update_scatter<kUpdateBlocks<R>, R>, (const void *)k_bktrk_move<R>,
+            (const void *)k_stage_begin<R>, (const void *)k_wrap_up<R>};
 }
 
 }  // namespace ep
