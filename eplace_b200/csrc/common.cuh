@@ -16,14 +16,15 @@ enum ObjFlag : uint8_t {
     kMacro = 1,     // Module::isMacro
     kFiller = 2,    // Module::isFiller
     kInView = 4,    // member of the current stage view
-    kBig = 8,       // spans more bins than a thread handles: block-per-object path
+    kBig = 8,       // spans more bins than a thread handles: a warp or a block takes it
     kSmoothX = 16,  // narrower than a bin: widened to one bin (local smoothing)
     kSmoothY = 32,  // lower than a bin
 };
 
 // Device-resident scalars of one engine (EPlacer_2D + EplaceNesterovOpt state
-// and the accumulators of the fused reductions).  Written only by the
-// finalising block of each reduction; every kernel reads `done`.
+// and the accumulators of the fused reductions).  Written by one thread of a
+// kernel (the finalising block of a reduction, the update's first block); every
+// kernel of the loop goes by `done`, the update by its copy.
 struct DevScalars {
     // arrival counters of the grid-wide reductions (reset by their last block)
     unsigned int cnt_prep, cnt_wl, cnt_comb;

@@ -8,7 +8,7 @@
 // with the same float arithmetic, so filler counts, bin geometry and the
 // static terminal / base density maps equal the reference's.  The netlist is
 // then laid out on the device as SoA arrays plus two CSRs (net -> pins,
-// object -> pins) and the loop of kernels.cu / dct.cu runs there.
+// object -> pins) and the loop of loop_kernels.cuh / dct.cu runs there.
 #include <algorithm>
 #include <future>
 #include <thread>
@@ -94,7 +94,7 @@ struct ep_engine {
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaEvent_t ev_poll = nullptr;  // the run's read-back of `done` has landed
+    cudaEvent_t ev_poll = nullptr;  // a quadratic solve's read-back of its state has landed
     std::mt19937_64 rng;
     void *snap = nullptr;     // ep_save_positions
     bool has_snap = false;
@@ -925,10 +925,11 @@ static ep_status create_engine(ep_engine *e, const ep_netlist *nl, const ep_para
                 if (owner[p] < no) pin_slot[p] = ops[owner[p]] + cnt[t][owner[p]]++;
         });
     }
-    // Device pin order for the per-net pass (kernels.cu): nets above
+    // Device pin order for the per-net pass (loop_kernels.cuh): nets above
     // kWarpPins pins first, largest first (a block or a warp each), then
-    // degree kWarpPins down to 1, floor(kWarpPins / degree) nets per warp, 32
-    // Nets without pins take no task.
+    // degree kWarpPins down to 1: floor(kWarpPins / degree) nets to a warp's
+    // task, from kThreadPins pins down 32 (degree 1 too).  Nets without pins
+    // take no task.
     std::vector<int4> net_tasks;
     int n_block_nets = 0;
     std::vector<int32_t> dev_owner(np), dev_of_pin(np);
@@ -2084,7 +2085,7 @@ ep_status ep_time_kernels(ep_engine *e, int32_t reps, ep_kernel_times *out) try 
     const double q = (double)e->v2 / sizeof(float2);  // 2 for the FP64 form's vectors
     const double nx = e->grid.nx, ny = e->grid.ny;
     // algorithmic bytes: compulsory reads + writes of each group, per launch
-    s = timed("scatter", 1 + (d.n_big_objs > 0), (9.0 + 8.0 * q) * nobj + 16.0 * nbin, 0.0,
+    s = timed("scatter", 1, (9.0 + 8.0 * q) * nobj + 16.0 * nbin, 0.0,
               [&] { launch_scatter(e->kc, d, e->node_q, e->S, e->st); }, zero_maps);
     if (s) return s;
     s = timed("prep", 1, 24.0 * nbin + 4.0 * q * nbin + (keep_maps ? 0.0 : 16.0 * nbin), 0.0,

@@ -55,7 +55,7 @@ inline void launch_kp(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// Per-net pass: a unit of work per task, by the nets' degree (kernels.cu): a
+// Per-net pass: a unit of work per task, by the nets' degree (loop_kernels.cuh): a
 // thread per net of 2 to kThreadPins pins, a lane per pin up to kWarpPins, a
 // warp per net up to kBlockPins, a block per net above.  Measured (1M cells,
 // FP32 / 200k cells, FP64, us): kThreadPins 1 118 / 38, 3 106 / 30 and 4 97 /
@@ -85,7 +85,7 @@ struct DctPlan {
     float *Tt = nullptr, *P = nullptr, *T3 = nullptr;
     // tensor-core path (bf16 hi/lo planes + TMA descriptors), dct_tc.cu
     void *tc = nullptr;
-    // fast-transform path (twiddle tables, intermediates), dct_fft.cu
+    // fast-transform path (twiddle tables, intermediates), fft.h
     void *fft = nullptr;
 };
 
@@ -101,7 +101,7 @@ inline int dct_launches(const DctPlan &p) { return p.mode == EP_DCT_FFT ? 3 : 4;
 // The tensor-core path reads rho as bf16 hi/lo planes written by the prep kernel.
 void *dct_tc_rho_planes(DctPlan &p);
 
-// ---- kernels (kernels.cu) ---------------------------------------------------
+// ---- kernels (kernels.cu, loop_kernels.cuh) -----------------------------------
 struct DeviceNetlist {
     int n_obj, n_nodes, n_terms;
     int n_nets, n_pins;
@@ -112,7 +112,7 @@ struct DeviceNetlist {
     const float *area;       // [n_obj] Module::area
     const float *sxy;        // [n_obj] local-smoothing scale sx*sy (EPlace/eplace.cpp:1061-1072)
     // pins in DEVICE order: nets grouped by degree (see the per-net pass in
-    // kernels.cu); obj_pin_dev maps each object's pins to their positions
+    // loop_kernels.cuh); obj_pin_dev maps each object's pins to their positions
     const int32_t *pin_owner;
     const float2 *pin_off;
     const int32_t *obj_pin_start;  // [n_obj + 1] object -> its pins (reference pin order)

@@ -903,7 +903,7 @@ void launch_dense_tc(int grid, cudaStream_t st, int N, const float *XA, const fl
 }
 
 // ------------------------------------------------- dense, backward --------
-// FP32 on the CUDA cores, as before: gradients stay in 32 bits, and the hidden
+// FP32 on the CUDA cores: gradients stay in 32 bits, and the hidden
 // layers' two products (0.82 GFLOP each at 50k nodes) are 14 us of FP32 FMAs.
 // One output per thread and two shared-memory reads per FMA made them 258 and
 // 323 us; a thread now holds 4 x 8 outputs and reads 3 (or 5) 16-byte vectors
@@ -1759,7 +1759,8 @@ ep_status ep_gnn_loss_grad(ep_gnn *g, ep_engine *e, const float *target4, double
     if (!g || !e || !target4) return EP_ERR_ARG;
     Use use(g);
     ep_status s = gave_up(g, true);
-    if (s || (s = bind(g, e, use)) || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) || (s = backward(g)))
+    if (s || (s = bind(g, e, use)) || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) ||
+        (s = backward(g)))
         return s;
     if (loss) GK(cudaMemcpyAsync(loss, g->loss, sizeof(double), cudaMemcpyDeviceToHost, g->eg.st));
     if (grad) GK(cudaMemcpyAsync(grad, g->grad, sizeof(float) * kParams, cudaMemcpyDeviceToHost, g->eg.st));
@@ -1773,7 +1774,8 @@ ep_status ep_gnn_train_step(ep_gnn *g, ep_engine *e, const float *target4, float
     if (!g || !e || !target4 || !(lr > 0)) return EP_ERR_ARG;
     Use use(g);
     ep_status s = gave_up(g, true);
-    if (s || (s = bind(g, e, use)) || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) || (s = backward(g)))
+    if (s || (s = bind(g, e, use)) || (s = bind_pads(g)) || (s = upload_target(g, target4)) || (s = forward(g)) ||
+        (s = backward(g)))
         return s;
     g->step++;
     const float c1 = 1.f / (1.f - std::pow(0.9f, (float)g->step)), c2 = 1.f / (1.f - std::pow(0.999f, (float)g->step));

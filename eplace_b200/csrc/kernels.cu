@@ -142,8 +142,9 @@ int carveout_percent(size_t smem_bytes) {
 // L1; smaller splits cost them occupancy, larger ones L1.
 // Function attributes belong to the current device, and setting one loads the
 // kernel: once per device for the kernels that every loop has, and for each
-// precision and wirelength form once an engine has it.  (All forms at once made
-// the first engine of a process LOAD_FIGURES.)
+// precision and wirelength form once an engine has it.  (All forms of both
+// precisions at once, in one file: 17.4 ms for the first engine of a process at
+// 100 cells, 13.5 so.)
 void set_loop_carveout(const KernelCtx &c) {
     static std::mutex mu;
     static std::vector<std::pair<int, int>> done;  // device, form (-1: the common kernels)

@@ -15,9 +15,9 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kSms = 148;
 // Grids of the kernels that loop over their work and end in a grid sum: one
-// block for each that an SM holds, so that a block's reduction and the wait for
-// its slowest warp are paid once.  Fixed numbers, so that the sums do not
-// depend on anything else.
+// block for each that an SM holds in FP32, so that a block's reduction and the
+// wait for its slowest warp are paid once.  Fixed numbers, the same in FP64, so
+// that the sums do not depend on anything else.
 constexpr int kNetBlocks = kSms * 6, kCombineBlocks = kSms * 3;
 inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
 

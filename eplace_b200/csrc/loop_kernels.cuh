@@ -367,8 +367,9 @@ __device__ __forceinline__ void finish_hpwl(DevScalars *S, const HpwlScalars &h,
 // centres and slots share sectors (1M cells: 84 -> 79 us).  The split of the
 // work and six blocks an SM (40 registers; four in FP64) took the pass from
 // 26.1 to 17.7 us at 200k cells, 112 to 75 at 1M, 17.4 to 8.6 at 30k (FP32),
-// 36.9 to 26.2 at 200k (FP64), with bitwise the same gradients.  WL = false computes only the HPWL with the same layout and reduction
-// tree, so both passes give bitwise the same HPWL.
+// 36.9 to 26.2 at 200k (FP64), with bitwise the same gradients.  WL = false
+// computes only the HPWL with the same layout and reduction tree, so both
+// passes give bitwise the same HPWL.
 struct NetOut {
     double hpwl, value;
 };
@@ -583,10 +584,11 @@ __device__ __forceinline__ NetOut net_in_warp(const int4 t, int lane, const PinC
 // kChunkPins at a time: every thread computes its pins' exponentials into
 // shared memory, then warp i adds the i-th of the eight sums, lane l the pins
 // l, l + 32, ... in order across the chunks, and an xor tree adds the lanes --
-// net_in_warp's order.  kChunkPins keeps the staging at 6 KB in both
-// precisions: at 12 KB four blocks an SM were left under the loop's 64 KB split
-// and the whole pass slowed by a fifth.  A net of more pins gathers its
-// positions anew in each sweep.
+// net_in_warp's order.  kChunkPins keeps the FP32 pass's staging at 6 KB: at 12
+// KB four blocks an SM were left under the loop's 64 KB split and the whole pass
+// slowed by a fifth.  (In FP64 the warp form's positions take 12 KB anyway, for
+// four blocks an SM.)  A net of more pins gathers its positions anew in each
+// sweep.
 template <typename R>
 struct BlockStage {
     static constexpr int kChunkPins = 1024 / (int)sizeof(R);
@@ -684,10 +686,13 @@ union NetStage {
 };
 
 // Blocks [0, n_block): one net of more than kBlockPins pins each; the warps of
-// the blocks after them take the other tasks in turn.  As many blocks as the
-// SMs hold at once: a block that ends after one task per warp waits for its
-// slowest warp and its reduction three times as often (1M cells 75 -> 59 us,
-// 200k 20.1 -> 17.4 on the same board, FP64 28.7 -> 25.2).
+// the blocks after them take the other tasks in turn, at most kNetBlocks of
+// them: as many as the SMs hold at once in FP32, where a block that ends after
+// one task per warp waits for its slowest warp and its reduction three times as
+// often (1M cells 75 -> 59 us, 200k 20.1 -> 17.4 on the same board).  In FP64,
+// four blocks an SM, they are a wave and a half (28.7 -> 25.2), and the blocks
+// of the large nets come on top in both.  The registers cost FP32 up to 128
+// bytes of spills a thread, FP64 up to 432.
 template <bool WL, bool EXACT, bool LSE, typename R>
 __global__ void __launch_bounds__(kNetWarps * 32, sizeof(R) == 8 ? 4 : 6)
 k_wl(const int4 *__restrict__ tasks, int n_block, int n_tasks, PinCtx<R> pc, vec2<R> *__restrict__ out,
@@ -1009,8 +1014,9 @@ __device__ __forceinline__ ObjStatic load_static(const DeviceNetlist &d, int o) 
 // static arrays during this one's gather (the first one's before the wait for
 // the previous grid); pin gradients and previous vectors are in flight during
 // the gather; and the registers are left room, as spilling cost more than the
-// warps it bought (1M cells, blocks an SM: 2 69 us, 3 59, 4 64, 5 73; one object
-// a thread at 4 blocks 96).  With the kBig objects' gather, a launch of its own
+// warps it bought in FP32 (1M cells, blocks an SM: 2 69 us, 3 59, 4 64, 5 73; one
+// object a thread at 4 blocks 96; FP64 takes three as well and spills 276 bytes
+// a thread).  With the kBig objects' gather, a launch of its own
 // before, us: 200k cells 18.3 + 3.1 -> 16.8, FP64 29.9 + 3.4 -> 25.5, 1M
 // 88.7 + 9.1 -> 59.5.
 template <typename R>
@@ -1224,8 +1230,8 @@ k_update(Grid g, int n, const uint8_t *__restrict__ flags, const float2 *__restr
 // threads the first moves it.  The step that ends the stage scatters nothing,
 // so the maps stay clear (prep clears them after each read).
 // MINB: blocks an SM that the registers have to allow.  Six hide the latency of
-// a large design's atomics, though they spill a few registers; a design whose
-// blocks are all resident anyway takes the instance without.
+// a large design's atomics (40 registers, no spills); a design whose blocks are
+// all resident anyway takes the instance without.
 template <int MINB, typename R>
 __global__ void __launch_bounds__(kThreads, MINB)
 k_update_scatter(Grid g, DeviceNetlist d, int big_blocks, vec2<R> *__restrict__ pos, vec2<R> *__restrict__ x,

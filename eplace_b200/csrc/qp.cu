@@ -543,7 +543,6 @@ k_qp_rows(int nn, const int32_t *__restrict__ obj_pin_start, const int32_t *__re
 struct QpMat {
     const int2 *ent_x, *ent_y;
     QpLayout lay;
-    const int32_t *count;  // [2 nn] entries of each row
     const float2 *diag;
     int nn;
 };
@@ -978,7 +977,7 @@ void qp_scan(const QpDev &q, cudaStream_t st) {
     k_qp_scan<<<1, kScanThreads, 0, st>>>(windows(q.nn), layout(q).win, q.cap_x, q.cap_y, q.solve);
 }
 
-static QpMat mat(const QpDev &q) { return QpMat{q.ent_x, q.ent_y, layout(q), q.count, q.diag, q.nn}; }
+static QpMat mat(const QpDev &q) { return QpMat{q.ent_x, q.ent_y, layout(q), q.diag, q.nn}; }
 
 // Grids that depend on the sizes alone, so that the dot products group alike on
 // every run: the SpMV kernels' with warps to spare for the long rows of a small
