@@ -349,13 +349,13 @@ __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, u
     __syncthreads();
     if (threadIdx.x == 0) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-        int got = 0;
-        for (unsigned it = 0; it < limit && !got; it++) {
-            unsigned v;
+        unsigned left = limit, v = 0;
+        while (left > 0) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-            got = v >= target;
+            if (v >= target) break;
+            left--;
         }
-        ok = got;
+        ok = left > 0;
     }
     __syncthreads();
     return ok != 0;
@@ -1294,7 +1294,8 @@ struct ep_gnn {
     unsigned *barrier = nullptr;  // the diffusion's arrival count
     double *loss = nullptr;
     int64_t step = 0;
-    cudaEvent_t used = nullptr;  // the end of the last call's work on the workspace (Use)
+    cudaEvent_t used = nullptr;  // the end of the last call's work, where it returned with work
+    bool pending = false;        // pending (Use)
     // bound netlist
     uint64_t uid = 0;         // 0: none
     bool pads_ready = false;  // terminal pin lists uploaded (training)
@@ -1330,30 +1331,40 @@ namespace {
 
 // One call's use of the network's workspace and weights, on its engine's stream.
 // Engines have streams of their own and some calls return with work pending, so
-// a call waits on the device for the one before, and marks its own end whatever
-// it returns.  Not while the stream is being captured, where neither may be.
+// a call waits on the device for one that did, and marks its own end unless it
+// has waited for its stream (synced).  Neither while the stream is being
+// captured, where they may not be.
 class Use {
   public:
     explicit Use(ep_gnn *g) : g_(g) {}
     Use(const Use &) = delete;
     ep_status begin(cudaStream_t st) {
         ep_gnn *const g = g_;
-        cudaStreamCaptureStatus capture;
-        GK(cudaStreamIsCapturing(st, &capture));
-        if (capture != cudaStreamCaptureStatusNone) return EP_OK;
-        GK(cudaStreamWaitEvent(st, g->used));
+        if (g->pending && !capturing(st)) GK(cudaStreamWaitEvent(st, g->used));
         st_ = st;
-        begun_ = true;
+        open_ = true;
         return EP_OK;
     }
+    void synced() {
+        open_ = false;
+        g_->pending = false;  // what was pending came before on this stream
+    }
     ~Use() {
-        if (begun_ && cudaEventRecord(g_->used, st_) != cudaSuccess) cudaStreamSynchronize(st_);
+        if (!open_ || capturing(st_)) return;
+        if (cudaEventRecord(g_->used, st_) == cudaSuccess)
+            g_->pending = true;
+        else
+            cudaStreamSynchronize(st_);
     }
 
   private:
+    static bool capturing(cudaStream_t st) {
+        cudaStreamCaptureStatus c;
+        return cudaStreamIsCapturing(st, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone;
+    }
     ep_gnn *g_;
     cudaStream_t st_ = nullptr;
-    bool begun_ = false;
+    bool open_ = false;
 };
 
 size_t smem_dense(int K) { return sizeof(float) * ((size_t)K * kH + (size_t)kDenseRows * (K + 1)); }
@@ -1702,7 +1713,7 @@ ep_status ep_gnn_get_weights(ep_gnn *g, float *w) {
 
 ep_status ep_gnn_set_weights(ep_gnn *g, const float *w) {
     if (!g || !w) return EP_ERR_ARG;
-    GK(cudaEventSynchronize(g->used));  // a pass that still reads the weights
+    if (g->pending) GK(cudaEventSynchronize(g->used));  // a pass that still reads the weights
     GK(cudaMemcpy(g->w, w, sizeof(float) * kParams, cudaMemcpyHostToDevice));
     GK(cudaMemset(g->adam_m, 0, sizeof(float) * kParams));
     GK(cudaMemset(g->adam_v, 0, sizeof(float) * kParams));
@@ -1729,6 +1740,7 @@ ep_status ep_gnn_features(ep_gnn *g, ep_engine *e, float *X) {
     if (s || (s = bind(g, e, use))) return s;
     GK(cudaMemcpyAsync(X, g->X, sizeof(float) * (size_t)g->net.N * kF, cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
+    use.synced();
     return gave_up(g, false);
 }
 
@@ -1741,6 +1753,7 @@ ep_status ep_gnn_forward(ep_gnn *g, ep_engine *e, float *xy4) try {
     std::vector<float4> p(nn);
     GK(cudaMemcpyAsync(p.data(), g->pred, sizeof(float4) * nn, cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
+    use.synced();
     if ((s = gave_up(g, true))) return s;
     const Grid &gr = g->eg.grid;
     const float W = gr.urx - gr.llx, H = gr.ury - gr.lly;
@@ -1765,6 +1778,7 @@ ep_status ep_gnn_loss_grad(ep_gnn *g, ep_engine *e, const float *target4, double
     if (loss) GK(cudaMemcpyAsync(loss, g->loss, sizeof(double), cudaMemcpyDeviceToHost, g->eg.st));
     if (grad) GK(cudaMemcpyAsync(grad, g->grad, sizeof(float) * kParams, cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
+    use.synced();
     return gave_up(g, true);
 } catch (const std::bad_alloc &) {
     return oom(g);
@@ -1784,6 +1798,7 @@ ep_status ep_gnn_train_step(ep_gnn *g, ep_engine *e, const float *target4, float
     GK(cudaGetLastError());
     if (loss) GK(cudaMemcpyAsync(loss, g->loss, sizeof(double), cudaMemcpyDeviceToHost, g->eg.st));
     GK(cudaStreamSynchronize(g->eg.st));
+    use.synced();
     return gave_up(g, true);
 } catch (const std::bad_alloc &) {
     return oom(g);
