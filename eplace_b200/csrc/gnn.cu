@@ -174,12 +174,12 @@ __global__ void __launch_bounds__(kT) k_pad_sort(Net g, int np, const int32_t *_
     __shared__ int found[2][kU][kT / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, owner = g.n_obj + blockIdx.x;
     int at = b, buf = 0;
-    for (int p0 = 0; p0 < np && at < e; p0 += kU * kT, buf ^= 1) {  // block-uniform
+    for (unsigned p0 = 0; p0 < (unsigned)np && at < e; p0 += kU * kT, buf ^= 1) {  // block-uniform
         unsigned m[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-            const int p = p0 + u * kT + (int)threadIdx.x;
-            m[u] = p < np && g.owner[p] == owner;
+            const unsigned p = p0 + u * kT + threadIdx.x;
+            m[u] = p < (unsigned)np && g.owner[p] == owner;
         }
 #pragma unroll
         for (int u = 0; u < kU; u++) {
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kT) k_pad_sort(Net g, int np, const int32_t *_
                 all += c;
             }
             if (m[u] >> lane & 1)
-                nets[at + before + __popc(m[u] & ((1u << lane) - 1))] = g.pin_net[p0 + u * kT + (int)threadIdx.x];
+                nets[at + before + __popc(m[u] & ((1u << lane) - 1))] = g.pin_net[p0 + u * kT + threadIdx.x];
             at += all;
         }
     }
